@@ -3,10 +3,10 @@
 // This layer validates arguments the way the reference's binding does
 // (PyOptix/PhotonDifferentialSplattig.cpp:14-22: matching photon counts, 2-row positions,
 // 2x3 matrices, one channel row), lays the workspace out, and enqueues
-//   plan:     counter and bucket-count reset, plan count pass, bucket scan, plan place pass,
-//             chunk_tile_kernel
-//   forward:  output reset, fwd_tiles_kernel, tail_fwd_kernel
-//   backward: bwd_tiles_kernel, tail_bwd_kernel, grad_scatter_kernel
+//   plan:     one reset of the counters and bucket counts, plan count pass, (past
+//             kFusedBuckets buckets: the bucket scan,) plan place pass
+//   forward:  output reset, fwd_tiles_kernel
+//   backward: bwd_tiles_kernel, grad_scatter_kernel
 // on the caller's stream. It allocates nothing and never synchronises. Failures return a
 // PDS_ERR_* code and leave a message for pds_last_error() (the reference raises through
 // TORCH_CHECK and does not check its launches, photon_differentials.cu:125, :234).
@@ -75,10 +75,7 @@ int resolve_cfg(const pds_config* in, pds_config& out) {
 // so that every resident CTA of the tile kernels (3 per SM) gets about four chunks; at least
 // 256 photons (one CTA-wide batch).
 int32_t effective_chunk(int32_t chunk, int64_t n) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        sms = 148;
+    const int sms = pds::num_sms();
     const int64_t target = (n + int64_t(sms) * 12 - 1) / (int64_t(sms) * 12);
     const int64_t c = (target + 255) / 256 * 256;
     return int32_t(c < 256 ? 256 : (c < chunk ? c : chunk));
@@ -114,35 +111,35 @@ int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resol
     return PDS_OK;
 }
 
-// The plan's workspace: the inverse map, the wide list, the records in sorted order, the
-// bucket counts, starts and cursors, each plan CTA's window histogram (kept from the count pass
-// for the place pass), the chunks' tiles, each tile's largest box radius (sized by the bucket
-// count, which bounds the tile count), and the backward's gradient records (stage, 32 bytes a
-// photon).
+// The plan's workspace: the counters, each tile's largest box radius, the bucket counts and
+// cursors (these four side by side, reset together), the bucket starts, the inverse map, the
+// wide list, the records in sorted order, each plan CTA's window histogram (kept from the count
+// pass for the place pass), the chunks' tiles, and the backward's gradient records (stage, 32
+// bytes a photon).
 struct Layout {
     size_t counters, inv, wide, stage, srecs, counts, start, cursor, part, cta_hist, chunk_tile,
         tile_r, total;
 };
 
-// Photon count n, bucket count nb (tiles << class bits).
-Layout make_layout(int64_t n, int64_t nb) {
+// Photon count n, tile count nt, bucket count nb (tiles << class bits).
+Layout make_layout(int64_t n, int64_t nt, int64_t nb) {
     Layout L;
     const size_t nn = size_t(n > 0 ? n : 1);
     const size_t nbb = size_t(nb > 0 ? nb : 1);
     size_t off = 0;
     L.counters = off; off += 256;
+    L.tile_r = off; off += pds::align_up(size_t(nt > 0 ? nt : 1) * 4, 256);
+    L.counts = off; off += pds::align_up(nbb * 4, 256);
+    L.cursor = off; off += pds::align_up(nbb * 4, 256);
+    L.start = off; off += pds::align_up((nbb + 1) * 4, 256);
     L.inv = off; off += pds::align_up(nn * 4, 256);
     L.wide = off; off += pds::align_up(nn * 4, 256);
     L.stage = off; off += pds::align_up(nn * sizeof(pds::GradRec), 256);
     L.srecs = off; off += pds::align_up(nn * sizeof(pds::Rec), 256);
-    L.counts = off; off += pds::align_up(nbb * 4, 256);
-    L.start = off; off += pds::align_up((nbb + 1) * 4, 256);
-    L.cursor = off; off += pds::align_up(nbb * 4, 256);
     L.part = off; off += pds::align_up(size_t(pds::bucket_scan_parts(int64_t(nbb))) * 4, 256);
     L.cta_hist = off;
     off += pds::align_up(size_t(pds::plan_hist_entries(int64_t(nn), int64_t(nbb))) * 4, 256);
     L.chunk_tile = off; off += pds::align_up((nn / 256 + 2) * 4, 256);  // chunks >= 256
-    L.tile_r = off; off += pds::align_up(nbb * 4, 256);
     L.total = off;
     return L;
 }
@@ -247,13 +244,15 @@ int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     Resolved r;
     int rc = resolve(cfg, mpr, n_tiles, ph.n, r);
     if (rc) return rc;
-    const Layout L = make_layout(ph.n, r.n_buckets);
+    const Layout L = make_layout(ph.n, n_tiles, r.n_buckets);
     rc = check_ws(ws, ws_bytes, L.total);
     if (rc) return rc;
     const Bufs b = bufs(ws, L);
-    cudaError_t e = cudaMemsetAsync(b.counters, 0, 16, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.counts, 0, size_t(r.n_buckets) * 4, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.tile_r, 0, size_t(n_tiles) * 4, s);
+    // the counters, tile radii and bucket counts, and where the place pass scans them itself its
+    // cursors, in one reset
+    const bool fused = pds::plan_fused(r.n_buckets);
+    cudaError_t e = cudaMemsetAsync(b.counters, 0,
+                                    (fused ? L.cursor : L.counts) + size_t(r.n_buckets) * 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "plan: counter reset");
     pds::PlanArgs a;
     a.ph = ph;
@@ -270,27 +269,24 @@ int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     a.cursor = b.cursor;
     a.srecs = b.srecs;
     a.tile_r = b.tile_r;
+    a.start = b.start;
+    a.chunk_tile = b.chunk_tile;
+    a.fused = fused ? 1 : 0;
     pds::plan_shape(ph.n, r.n_buckets, &a.window, &a.range);
     e = pds::launch_plan_count(a, s);
     if (e != cudaSuccess) return cuda_fail(e, "plan count pass");
-    pds::ScanArgs sa;
-    sa.counts = b.counts;
-    sa.counters = b.counters;
-    sa.part = b.part;
-    sa.start = b.start;
-    sa.cursor = b.cursor;
-    sa.chunk_tile = b.chunk_tile;
-    sa.n = ph.n;
-    sa.nb = r.n_buckets;
-    sa.n_tiles = n_tiles;
-    sa.chunk = r.cfg.chunk;
-    sa.cb = r.cfg.class_bits;
-    e = pds::launch_bucket_scan(sa, s);
-    if (e != cudaSuccess) return cuda_fail(e, "bucket scan");
+    if (!fused) {
+        pds::ScanArgs sa;
+        sa.counts = b.counts;
+        sa.part = b.part;
+        sa.start = b.start;
+        sa.cursor = b.cursor;
+        sa.nb = r.n_buckets;
+        e = pds::launch_bucket_scan(sa, s);
+        if (e != cudaSuccess) return cuda_fail(e, "bucket scan");
+    }
     e = pds::launch_plan_place(a, s);
     if (e != cudaSuccess) return cuda_fail(e, "plan place pass");
-    e = pds::launch_chunk_tiles(sa, s);
-    if (e != cudaSuccess) return cuda_fail(e, "chunk_tile_kernel");
     return PDS_OK;
 }
 
@@ -299,7 +295,7 @@ int tile_args(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     Resolved r;
     int rc = resolve(cfg, mpr, n_tiles, ph.n, r);
     if (rc) return rc;
-    const Layout L = make_layout(ph.n, r.n_buckets);
+    const Layout L = make_layout(ph.n, n_tiles, r.n_buckets);
     rc = check_ws(ws, ws_bytes, L.total);
     if (rc) return rc;
     const Bufs b = bufs(ws, L);
@@ -317,7 +313,6 @@ int tile_args(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     a.tile_r = b.tile_r;
     a.stage = b.stage;
     a.counters = b.counters;
-    a.queue = b.counters + 4;  // [0..3) plan counters; [4] the tile kernels' work counter
     return PDS_OK;
 }
 
@@ -330,8 +325,8 @@ int forward_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tile
     if (rc) return rc;
     a.out = out;
     a.image_elems = image_elems;
+    a.queue = const_cast<uint32_t*>(a.counters) + 4;  // [0..3) plan counters; [4], [5]
     cudaError_t e = cudaMemsetAsync(out, 0, size_t(image_elems) * sizeof(float), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return cuda_fail(e, "forward: output reset");
     if (ph.n == 0) return PDS_OK;
     e = pds::launch_forward(a, s);
@@ -355,9 +350,8 @@ int backward_impl(const float* grad, const pds::Photons& ph, const pds::SimTable
     a.gE = gE;
     a.gX = gX;
     a.gM = gM;
-    cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return cuda_fail(e, "backward: work counter reset");
-    e = pds::launch_backward(a, s);
+    a.queue = const_cast<uint32_t*>(a.counters) + 6;
+    const cudaError_t e = pds::launch_backward(a, s);
     if (e != cudaSuccess) return cuda_fail(e, "bwd_tiles_kernel");
     return PDS_OK;
 }
@@ -391,13 +385,13 @@ const char* pds_version(void) { return "pds_b200 1.0 (sm_100a)"; }
 
 size_t pds_workspace_bytes(int64_t n, int64_t C, int64_t H, int64_t W, const pds_config* cfg) {
     pds_config c;
-    if (resolve_cfg(cfg, c) != PDS_OK || C < 1 || H < 1 || W < 1) return make_layout(n, 1).total;
+    if (resolve_cfg(cfg, c) != PDS_OK || C < 1 || H < 1 || W < 1) return make_layout(n, 1, 1).total;
     const int64_t tiles = C * ((H + c.tile - 1) / c.tile) * ((W + c.tile - 1) / c.tile);
-    return make_layout(n, bucket_count(cfg, tiles)).total;
+    return make_layout(n, tiles, bucket_count(cfg, tiles)).total;
 }
 
 size_t pds_batch_workspace_bytes(int64_t n_total, int64_t n_tiles_total, const pds_config* cfg) {
-    return make_layout(n_total, bucket_count(cfg, n_tiles_total)).total;
+    return make_layout(n_total, n_tiles_total, bucket_count(cfg, n_tiles_total)).total;
 }
 
 int pds_plan_f32(const float* E, const float* X, const float* M, const int64_t* cp,
@@ -664,7 +658,7 @@ static int plan_records(const void* ws, size_t ws_bytes, int64_t n, int64_t n_ti
         int rc = resolve_cfg(cfg, c);
         return rc ? rc : fail(PDS_ERR_UNSUPPORTED, "tile count outside [1, 2^30)");
     }
-    const Layout L = make_layout(n, nb);
+    const Layout L = make_layout(n, n_tiles, nb);
     int rc = check_ws(const_cast<void*>(ws), ws_bytes, L.total);
     if (rc) return rc;
     const Bufs b = bufs(const_cast<void*>(ws), L);
@@ -864,7 +858,7 @@ int pds_plan_export(const void* ws, size_t ws_bytes, int64_t n, int64_t n_tiles,
     Resolved r;
     int rc = resolve(cfg, mpr, n_tiles, n, r);
     if (rc) return rc;
-    const Layout L = make_layout(n, r.n_buckets);
+    const Layout L = make_layout(n, n_tiles, r.n_buckets);
     rc = check_ws(const_cast<void*>(ws), ws_bytes, L.total);
     if (rc) return rc;
     const Bufs b = bufs(const_cast<void*>(ws), L);

@@ -1,6 +1,7 @@
 // Internal (non-ABI) declarations shared by the library's translation units.
 #pragma once
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -10,6 +11,70 @@
 namespace pds {
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+// The current device (0 where there is none).
+inline int current_device() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
+
+// Multiprocessors of the current device (148 where there is none), asked of the driver once per
+// device: a fact of the hardware that every launch's grid needs.
+inline int num_sms() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
+    const int dev = current_device();
+    if (dev >= 0 && dev < kDevices) {
+        const int k = known[dev].load(std::memory_order_relaxed);
+        if (k > 0) return k;
+    }
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return 148;
+    if (dev >= 0 && dev < kDevices) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
+}
+
+// Lets a kernel use up to kMaxDynamicSmem bytes of dynamic shared memory (always the same
+// limit, so that threads raising it for different launches cannot undo one another), once per
+// device. A larger request fails here as its launch would.
+constexpr size_t kMaxDynamicSmem = 226 * 1024;  // 227 KB less what the kernels hold statically
+template <auto Kernel>
+cudaError_t allow_smem(size_t smem) {
+    constexpr int kDevices = 64;
+    static std::atomic<bool> done[kDevices];
+    if (smem <= 48 * 1024) return cudaSuccess;
+    if (smem > kMaxDynamicSmem) return cudaErrorInvalidValue;
+    const int dev = current_device();
+    const bool cached = dev >= 0 && dev < kDevices;
+    if (cached && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(kMaxDynamicSmem));
+    if (e == cudaSuccess && cached) done[dev].store(true, std::memory_order_release);
+    return e;
+}
+
+// Resident CTAs of a kernel on one SM (at least 1) for a block size and dynamic shared memory:
+// a function of the kernel and the device; the last answer per device is kept.
+template <auto Kernel>
+int resident_ctas(int threads, size_t smem) {
+    constexpr int kDevices = 64;
+    static std::atomic<uint64_t> last[kDevices];  // smem << 16 | threads' warps << 8 | CTAs
+    const int dev = current_device();
+    const bool cached = dev >= 0 && dev < kDevices;
+    const uint64_t key = uint64_t(smem) << 16 | uint64_t(threads / 32) << 8;
+    if (cached) {
+        const uint64_t v = last[dev].load(std::memory_order_relaxed);
+        if ((v & ~uint64_t(0xFF)) == key && (v & 0xFF)) return int(v & 0xFF);
+    }
+    int per_sm = 0;
+    if (allow_smem<Kernel>(smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kernel, threads, smem) != cudaSuccess ||
+        per_sm < 1)
+        return 1;
+    if (cached) last[dev].store(key | uint64_t(per_sm), std::memory_order_relaxed);
+    return per_sm;
+}
 
 // refraction to the receiver (pds_refract.cu)
 // A splat plan's per-photon gradient records (the backward's output before the spread into

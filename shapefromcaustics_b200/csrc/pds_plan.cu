@@ -11,15 +11,16 @@
 //                    buckets (up to 32768) that starts at its first photon's simulation; the
 //                    histogram is added into the global counts and kept per CTA. Photons wider
 //                    than the apron go to the wide list.
-//   bucket scan      exclusive scan of the bucket counts (three parallel kernels), giving each
-//                    bucket its first sorted position; a copy serves as the place pass's
-//                    cursors.
+//   bucket scan      exclusive scan of the bucket counts, giving each bucket its first sorted
+//                    position; a copy serves as the place pass's cursors. Up to kFusedBuckets
+//                    buckets every place CTA scans the counts itself (no kernel of its own), up
+//                    to kOneScanBuckets one kernel does it, beyond that three.
 //   place pass       the same CTA ranges: each CTA reserves its share of every bucket with one
 //                    atomic on the bucket's cursor, hands positions out from shared memory,
 //                    re-bins its photons and writes each one's 32-byte record at its position
 //                    (one whole sector), keeping the position per photon (coalesced) for the
-//                    backward's gradient spread.
-//   chunk_tile       the tile holding the first photon of every tile-kernel work chunk.
+//                    backward's gradient spread. The photon placed first in a tile-kernel work
+//                    chunk also writes down the chunk's tile.
 //
 // Nothing per photon is kept between the passes but the inverse map of wide and untouched
 // photons: the place pass recomputes the keys from the inputs (40 bytes a photon read twice)
@@ -55,10 +56,31 @@ constexpr int64_t kPlanMaxCtas = 512;
 // buckets of a CTA's shared histogram (128 KB: a 2048^2 image's buckets at 5 class bits; the
 // SM keeps about 100 KB of L1 cache for the streamed loads)
 constexpr int kMaxWindow = 32768;
+// Buckets up to which every place CTA scans the counts itself (six a thread): a 512^2 image has
+// 2048 at 5 class bits, two of them 4096. The scan's re-reads (16 KB a CTA from the L2) cost
+// about a microsecond; the kernels they replace took 11 us a plan with their launches.
+constexpr int kFusedPer = 6;
+constexpr int64_t kFusedBuckets = int64_t(kFusedPer) * kPlanKernelThreads;
+// Buckets up to which one kernel scans them, each CTA summing the counts before its own (at
+// most 512 KB from the L2); beyond, the sums are formed once, by a kernel of their own.
+constexpr int64_t kOneScanBuckets = 131072;
 
-// First bucket of the simulation owning photon i.
-__device__ __forceinline__ uint32_t window_base(const SimTable& st, int64_t i, int cb) {
-    return uint32_t(load_sim(st, find_sim_of_photon(st, i)).tile_base) << cb;
+// Photons of a plan CTA at least: one per thread, and a quarter of its window's buckets, so that
+// the window's clear and flush stay in proportion. (A fixed 8192 left small calls on a handful
+// of CTAs, each running 11 photons a thread in a row: count and place together took 37 us for
+// 2^14 photons and 46 us for 3 10^5.)
+__host__ __device__ constexpr int64_t min_range(int64_t window) {
+    const int64_t q = window / 4;
+    return q <= kPlanKernelThreads
+               ? kPlanKernelThreads
+               : (q + kPlanKernelThreads - 1) / kPlanKernelThreads * kPlanKernelThreads;
+}
+
+// First bucket of a CTA's window: the first of the simulation owning its first photon i, or the
+// first of all where the window holds every bucket.
+__device__ __forceinline__ uint32_t window_base(const PlanArgs& a, int64_t i) {
+    if (uint32_t(a.window) >= a.key_big) return 0u;
+    return uint32_t(load_sim(a.sims, find_sim_of_photon(a.sims, i)).tile_base) << a.cfg.class_bits;
 }
 
 __device__ __forceinline__ void zero_window(uint32_t* hist, int window) {
@@ -127,6 +149,45 @@ __device__ __forceinline__ uint32_t bin_photon(const PlanArgs& a, const pds_sim&
     return (tile << cb) | cls;
 }
 
+// Exclusive scan of the counts of all buckets (at most kFusedPer a thread, the window holds
+// them all) by one place CTA, then the reservation of the CTA's share: hist[j] = bucket j's
+// first position + what other CTAs have taken before. CTA 0 writes the starts down for the
+// tile kernels.
+__device__ __forceinline__ void fused_scan(const PlanArgs& a, uint32_t* hist,
+                                           const uint32_t* mine) {
+    constexpr int kWarps = kPlanKernelThreads / 32;
+    __shared__ uint32_t wsum[kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b0 = int(threadIdx.x) * kFusedPer, nb = int(a.key_big);
+    uint32_t v[kFusedPer], s = 0;
+#pragma unroll
+    for (int k = 0; k < kFusedPer; ++k) {
+        v[k] = b0 + k < nb ? __ldcg(a.counts + b0 + k) : 0u;
+        s += v[k];
+    }
+    uint32_t x = s;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t run = x - s;
+    for (int w = 0; w < warp; ++w) run += wsum[w];
+#pragma unroll
+    for (int k = 0; k < kFusedPer; ++k) {
+        const int j = b0 + k;
+        if (j < nb) {
+            const uint32_t c = mine[j];
+            hist[j] = c ? run + atomicAdd(a.cursor + j, c) : run;
+            if (blockIdx.x == 0) a.start[j] = run;
+        }
+        run += v[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == kPlanKernelThreads - 1) a.start[nb] = run;
+}
+
 // One pass of the plan over a CTA's contiguous photon range (coalesced SoA reads; each thread
 // loads its next photon's inputs while it bins the current one).
 //   count (PLACE = false): every photon's bucket into the CTA's shared histogram window (global
@@ -136,21 +197,27 @@ __device__ __forceinline__ uint32_t bin_photon(const PlanArgs& a, const pds_sim&
 //   place (PLACE = true, after the scan): the CTA reserves its share of every window bucket
 //       with one atomic on the bucket's cursor (from its kept histogram), re-bins its photons,
 //       builds each tile-path photon's record and writes it at its sorted position (one whole
-//       32-byte sector), keeping the position in the inverse map.
+//       32-byte sector), keeping the position in the inverse map. With few buckets (a.fused) it
+//       first scans the counts itself; a.cursor then starts at zero and holds what the CTAs
+//       have taken.
 template <bool PLACE>
 __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs a) {
     extern __shared__ uint32_t hist[];  // a.window buckets
     const int64_t n = a.ph.n;
     const int lane = threadIdx.x & 31;
     const int64_t r0 = int64_t(blockIdx.x) * a.range, r1 = min(r0 + a.range, n);
-    const uint32_t kb0 = window_base(a.sims, r0, a.cfg.class_bits);
+    const uint32_t kb0 = window_base(a, r0);
     const int64_t wend = min(int64_t(a.window), int64_t(a.key_big) - int64_t(kb0));
     uint32_t* mine = a.cta_hist + int64_t(blockIdx.x) * a.window;
     if (PLACE) {
         // hist[j] becomes the CTA's first position in window bucket j
-        for (int j = threadIdx.x; j < a.window; j += blockDim.x) {
-            const uint32_t c = j < wend ? mine[j] : 0u;
-            hist[j] = c ? atomicAdd(a.cursor + kb0 + j, c) : 0u;
+        if (a.fused) {
+            fused_scan(a, hist, mine);
+        } else {
+            for (int j = threadIdx.x; j < a.window; j += blockDim.x) {
+                const uint32_t c = j < wend ? mine[j] : 0u;
+                hist[j] = c ? atomicAdd(a.cursor + kb0 + j, c) : 0u;
+            }
         }
     } else {
         zero_window(hist, a.window);
@@ -230,6 +297,9 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
                 if (pos < uint32_t(n)) {
                     a.srecs[pos] = r;
                     a.inv[i] = pos;
+                    // the first photon of a work chunk (a multiple of 256 positions)
+                    if ((pos & 255u) == 0u && pos % uint32_t(a.cfg.chunk) == 0u)
+                        a.chunk_tile[pos / uint32_t(a.cfg.chunk)] = key >> a.cfg.class_bits;
                 }
             }
             continue;
@@ -284,11 +354,12 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
 }
 
 // ------------------------------------------------------------------ bucket scan --------
-// Exclusive scan of counts[0, nb) into start[0, nb] (start[nb] = the total) and cursor[0, nb):
-// per-CTA sums of kScanItems buckets, one CTA scanning those sums, then each CTA's rescan.
+// Exclusive scan of counts[0, nb) into start[0, nb] (start[nb] = the total) and cursor[0, nb).
+// Up to kOneScanBuckets: bucket_down alone, whose CTAs each sum the counts before theirs.
+// Beyond: per-CTA sums of kScanItems buckets, one CTA scanning those sums, then bucket_down.
 
-constexpr int kScanThreads = 256;
-constexpr int kScanPer = 16;
+constexpr int kScanThreads = 1024;
+constexpr int kScanPer = 4;
 constexpr int kScanItems = kScanThreads * kScanPer;
 
 // Exclusive scan of one value per thread over the CTA; *total gets the CTA's sum.
@@ -304,13 +375,13 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
     if (lane == 31) wsum[warp] = x;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = lane < kScanThreads / 32 ? wsum[lane] : 0u;
+        uint32_t w = wsum[lane];
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, off);
             if (lane >= off) w += y;
         }
-        if (lane < kScanThreads / 32) wsum[lane] = w;
+        wsum[lane] = w;
     }
     __syncthreads();
     const uint32_t before = warp > 0 ? wsum[warp - 1] : 0u;
@@ -318,24 +389,33 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
     __syncthreads();
     return before + x - v;
 }
+static_assert(kScanThreads == 1024, "one warp scans the warps' sums");
+
+// Sum of the counts of one CTA's buckets; four a thread (the counts start 256-byte aligned and
+// are padded to a multiple of 256 bytes, so a group of four that begins before nb is inside).
+__device__ __forceinline__ uint4 count_group(const uint32_t* counts, int64_t j, int64_t nb) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (j < nb) {
+        v = __ldg(reinterpret_cast<const uint4*>(counts + j));
+        if (j + 1 >= nb) v.y = 0u;
+        if (j + 2 >= nb) v.z = 0u;
+        if (j + 3 >= nb) v.w = 0u;
+    }
+    return v;
+}
 
 __global__ __launch_bounds__(kScanThreads) void bucket_reduce(const uint32_t* __restrict__ counts,
                                                               int64_t nb,
                                                               uint32_t* __restrict__ part) {
-    const int64_t b0 = int64_t(blockIdx.x) * kScanItems;
-    uint32_t s = 0;
-    for (int k = threadIdx.x; k < kScanItems; k += kScanThreads) {
-        const int64_t j = b0 + k;
-        if (j < nb) s += __ldg(counts + j);
-    }
+    const uint4 v = count_group(counts, int64_t(blockIdx.x) * kScanItems + threadIdx.x * kScanPer,
+                                nb);
     uint32_t total;
-    block_exclusive_scan(s, &total);
+    block_exclusive_scan(v.x + v.y + v.z + v.w, &total);
     if (threadIdx.x == 0) part[blockIdx.x] = total;
 }
 
 __global__ __launch_bounds__(kScanThreads) void bucket_top(uint32_t* __restrict__ part,
-                                                           int64_t np, uint32_t* __restrict__ start,
-                                                           int64_t nb) {
+                                                           int64_t np) {
     uint32_t carry = 0;
     for (int64_t b = 0; b < np; b += kScanThreads) {
         const int64_t j = b + threadIdx.x;
@@ -345,50 +425,41 @@ __global__ __launch_bounds__(kScanThreads) void bucket_top(uint32_t* __restrict_
         if (j < np) part[j] = carry + ex;
         carry += total;
     }
-    if (threadIdx.x == 0) start[nb] = carry;
 }
 
+// part: the scanned sums of the CTAs' buckets, or null to sum the counts before this CTA's here.
 __global__ __launch_bounds__(kScanThreads) void bucket_down(const uint32_t* __restrict__ counts,
                                                             int64_t nb,
                                                             const uint32_t* __restrict__ part,
                                                             uint32_t* __restrict__ start,
                                                             uint32_t* __restrict__ cursor) {
     // thread t owns buckets [b0 + t * kScanPer, + kScanPer)
-    const int64_t b0 = int64_t(blockIdx.x) * kScanItems + int64_t(threadIdx.x) * kScanPer;
-    uint32_t v[kScanPer];
-    uint32_t s = 0;
+    const int64_t b0 = int64_t(blockIdx.x) * kScanItems;
+    uint32_t base, total;
+    if (part) {
+        base = part[blockIdx.x];
+    } else {
+        uint32_t s = 0;
+        for (int64_t j = int64_t(threadIdx.x) * kScanPer; j < b0; j += kScanItems) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(counts + j));
+            s += v.x + v.y + v.z + v.w;
+        }
+        block_exclusive_scan(s, &base);
+    }
+    const int64_t j = b0 + int64_t(threadIdx.x) * kScanPer;
+    const uint4 v = count_group(counts, j, nb);
+    const uint32_t sum = v.x + v.y + v.z + v.w;
+    uint32_t run = base + block_exclusive_scan(sum, &total);
+    const uint32_t c[kScanPer] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
-        v[k] = b0 + k < nb ? __ldg(counts + b0 + k) : 0u;
-        s += v[k];
-    }
-    uint32_t total;
-    uint32_t run = part[blockIdx.x] + block_exclusive_scan(s, &total);
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        if (b0 + k < nb) {
-            start[b0 + k] = run;
-            cursor[b0 + k] = run;
+        if (j + k < nb) {
+            start[j + k] = run;
+            cursor[j + k] = run;
         }
-        run += v[k];
+        run += c[k];
     }
-}
-
-// Tile of the first photon of every work chunk: the last tile whose bucket range starts at or
-// before the chunk's first position (empty tiles start where their successor does).
-__global__ __launch_bounds__(256) void chunk_tile_kernel(ScanArgs a) {
-    const int64_t n_tile = min(int64_t(a.counters[0]), a.n);
-    const int64_t nchunks = (n_tile + a.chunk - 1) / a.chunk;
-    for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nchunks;
-         c += int64_t(gridDim.x) * blockDim.x) {
-        const uint32_t p = uint32_t(c * a.chunk);
-        int64_t lo = 0, hi = a.n_tiles - 1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (__ldg(a.start + (mid << a.cb)) <= p) lo = mid; else hi = mid - 1;
-        }
-        a.chunk_tile[c] = uint32_t(lo);
-    }
+    if (threadIdx.x == 0 && b0 + kScanItems >= nb) start[nb] = base + total;
 }
 
 // The plan's binning per photon: its bucket (from its sorted position and the bucket starts)
@@ -421,13 +492,6 @@ __global__ __launch_bounds__(256) void plan_export_kernel(const uint32_t* __rest
     }
 }
 
-int num_sms() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 unsigned capped_blocks(int64_t items, int per_sm) {
     const int64_t blocks = (items + 255) / 256;
     const int64_t cap = int64_t(num_sms()) * per_sm;
@@ -436,49 +500,36 @@ unsigned capped_blocks(int64_t items, int per_sm) {
 
 }  // namespace
 
+bool plan_fused(int64_t nb) { return nb <= kFusedBuckets; }
+
 int64_t bucket_scan_parts(int64_t nb) { return (nb + kScanItems - 1) / kScanItems; }
 
-template <typename K>
-cudaError_t window_smem(K kernel, int32_t window) {
-    const size_t smem = size_t(window) * 4;
-    if (smem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-}
-
 // Window and photons per CTA of the two plan passes: the window holds a simulation's buckets
-// where it can (at most kMaxWindow); as many CTAs per SM as the window's shared memory allows
-// (the kernels' shared-memory limit is raised first, or the occupancy query would see a kernel
-// that cannot launch), at most kPlanMaxCtas in all (the size of the kept histograms), and the
-// photons are split evenly over one wave of them (at least 8192 a CTA, so the window's clear
-// and flush are amortised).
+// where it can (at most kMaxWindow); as many CTAs per SM as the window's shared memory allows,
+// at most kPlanMaxCtas in all (the size of the kept histograms), and the photons are split
+// evenly over one wave of them (at least min_range a CTA).
 void plan_shape(int64_t n, int64_t nb, int32_t* window, int64_t* range) {
     const int64_t w = nb < kMaxWindow ? nb : kMaxWindow;
     *window = int32_t(w > 0 ? w : 1);
-    const size_t smem = size_t(*window) * 4;
-    int per_sm = 1;
-    if (window_smem(plan_pass_kernel<false>, *window) != cudaSuccess ||
-        window_smem(plan_pass_kernel<true>, *window) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plan_pass_kernel<false>,
-                                                      kPlanKernelThreads, smem) != cudaSuccess)
-        per_sm = 1;
-    if (per_sm < 1) per_sm = 1;
-    int64_t ctas = int64_t(num_sms()) * per_sm;
+    int64_t ctas = int64_t(num_sms()) *
+                   resident_ctas<plan_pass_kernel<false>>(kPlanKernelThreads, size_t(*window) * 4);
     if (ctas > kPlanMaxCtas) ctas = kPlanMaxCtas;
     int64_t r = (n + ctas - 1) / ctas;
     r = (r + kPlanKernelThreads - 1) / kPlanKernelThreads * kPlanKernelThreads;
-    *range = r < 8192 ? 8192 : r;
+    const int64_t least = min_range(*window);
+    *range = r < least ? least : r;
 }
 
 int64_t plan_hist_entries(int64_t n, int64_t nb) {
     const int64_t w = nb < kMaxWindow ? (nb > 0 ? nb : 1) : kMaxWindow;
-    const int64_t by_n = (n + 8191) / 8192;
+    const int64_t by_n = (n + min_range(w) - 1) / min_range(w);
     return (by_n < kPlanMaxCtas ? (by_n > 0 ? by_n : 1) : kPlanMaxCtas) * w;
 }
 
 template <bool PLACE>
 cudaError_t launch_pass(const PlanArgs& a, cudaStream_t st) {
     if (a.ph.n <= 0) return cudaSuccess;
-    cudaError_t e = window_smem(plan_pass_kernel<PLACE>, a.window);
+    const cudaError_t e = allow_smem<plan_pass_kernel<PLACE>>(size_t(a.window) * 4);
     if (e != cudaSuccess) return e;
     plan_pass_kernel<PLACE><<<unsigned((a.ph.n + a.range - 1) / a.range), kPlanKernelThreads,
                               size_t(a.window) * 4, st>>>(a);
@@ -500,16 +551,13 @@ cudaError_t launch_plan_export(const uint32_t* inv, const uint32_t* start, int64
 
 cudaError_t launch_bucket_scan(const ScanArgs& a, cudaStream_t st) {
     const int64_t np = bucket_scan_parts(a.nb);
-    bucket_reduce<<<unsigned(np), kScanThreads, 0, st>>>(a.counts, a.nb, a.part);
-    bucket_top<<<1, kScanThreads, 0, st>>>(a.part, np, a.start, a.nb);
-    bucket_down<<<unsigned(np), kScanThreads, 0, st>>>(a.counts, a.nb, a.part, a.start,
-                                                       a.cursor);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_chunk_tiles(const ScanArgs& a, cudaStream_t st) {
-    if (a.n <= 0) return cudaSuccess;
-    chunk_tile_kernel<<<capped_blocks((a.n + a.chunk - 1) / a.chunk, 4), 256, 0, st>>>(a);
+    uint32_t* part = nullptr;
+    if (a.nb > kOneScanBuckets) {
+        part = a.part;
+        bucket_reduce<<<unsigned(np), kScanThreads, 0, st>>>(a.counts, a.nb, part);
+        bucket_top<<<1, kScanThreads, 0, st>>>(part, np);
+    }
+    bucket_down<<<unsigned(np), kScanThreads, 0, st>>>(a.counts, a.nb, part, a.start, a.cursor);
     return cudaGetLastError();
 }
 

@@ -15,7 +15,8 @@
 //                    and writes one gradient record (no atomics). The per-pixel work is reduced
 //                    to the moments sum(t g), sum(t^2 g), sum(t g d), sum(t g d d^T) of the
 //                    offset d, from which dL/dE, dL/dx and dL/dM follow by 2x2 algebra.
-//   tail kernels     footprints wider than the apron (direct global path, a warp per photon).
+//   tail_*           footprints wider than the apron (direct global path, a warp per photon), by
+//                    the tile kernels' CTAs once no chunk is left.
 //   grad_scatter     gradient records into the reference's SoA outputs, zero for photons that
 //                    touch no pixel.
 #include <climits>
@@ -104,15 +105,33 @@ __device__ __forceinline__ void fwd_row(int n, uint32_t a, float b0, float b1, f
     }
 }
 
+// Clipped box of a record in pixel coordinates.
+__device__ __forceinline__ void rec_box(const Rec& r, const TileInfo& ti, int& pxc, int& pyc,
+                                        int& x0, int& x1, int& y0, int& y1) {
+    const uint32_t p = r.packed;
+    pxc = ti.ox + rec_lx(p);
+    pyc = ti.oy + rec_ly(p);
+    const int rx = rec_rx(p), ry = rec_ry(p);
+    x0 = max(pxc - rx, 0);
+    x1 = min(pxc + rx, ti.W - 1);
+    y0 = max(pyc - ry, 0);
+    y1 = min(pyc + ry, ti.H - 1);
+}
+
 // Forward deposit of one photon over its band (see Band): one flattened loop over
 // rows x bw pixels, so the trip count depends only on the band's area (photons of a warp
 // share an area class), the row changing every bw steps. Pixels outside the reference's
-// clipped box are masked off (their add is predicated away).
-__device__ __forceinline__ void deposit_band(const Rec& r, const Band& bd, const TileInfo& ti,
-                                             int sw, uint32_t acc_base, int pxc, int pyc, int x0,
-                                             int x1, int y0, int y1) {
+// clipped box are masked off (their add is predicated away). False: the photon has no band.
+__device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, int sw,
+                                             uint32_t acc_base) {
+    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
+    int pxc, pyc, x0, x1, y0, y1;
+    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+    const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
+                              float(rec_rx(r.packed)) + 1.f);
+    if (!bd.on) return false;
     const int ky0 = max(bd.ky0, y0 - pyc), ky1 = min(bd.ky1, y1 - pyc);
-    if (ky0 > ky1) return;
+    if (ky0 > ky1) return true;
     const int kxb0 = x0 - pxc;
     const uint32_t kxspan = uint32_t(x1 - x0);
     const float e3 = r.e * kThreeOverPi;
@@ -142,35 +161,25 @@ __device__ __forceinline__ void deposit_band(const Rec& r, const Band& bd, const
             row += 4u * uint32_t(sw);
         }
     }
+    return true;
 }
 
-// Forward deposit of one photon into the shared accumulator (photon_differentials.cu:91-110).
-// With spans on, only the support's rows and row spans are visited; the other box pixels
-// add exactly zero in the reference (value > 0 fails, :106). Photons that fail the
-// reference's image-half-size ellipse test somewhere in their box (tiny images only) take
-// the per-pixel test path.
-__device__ __forceinline__ void deposit(const Rec& r, const TileInfo& ti, int sw, bool spans,
-                                        bool band, float* acc, int& bx0, int& bx1, int& by0,
-                                        int& by1) {
+// Forward deposit of one photon without a band walk (photon_differentials.cu:91-110): the whole
+// box, or with spans on only the support's rows and row spans (the other box pixels add exactly
+// zero in the reference: value > 0 fails, :106). Photons that fail the reference's
+// image-half-size ellipse test somewhere in their box (tiny images only) take the per-pixel test
+// path. Out of line: with the band walk on, hardly any photon comes here, and inlined its
+// registers were spilled around every photon's band walk.
+__device__ __noinline__ void deposit_generic(const Rec* rp, TileInfo ti, int sw, bool spans,
+                                             float* acc) {
+    const Rec r = *rp;
     const uint32_t p = r.packed;
-    const uint32_t fl = rec_flags(p);
-    if (fl & kFlagFwdSkip) return;
     const int pxc = ti.ox + rec_lx(p), pyc = ti.oy + rec_ly(p);
     const int rx = rec_rx(p), ry = rec_ry(p);
     const int x0 = max(pxc - rx, 0), x1 = min(pxc + rx, ti.W - 1);
     const int y0 = max(pyc - ry, 0), y1 = min(pyc + ry, ti.H - 1);
-    bx0 = x0; bx1 = x1; by0 = y0; by1 = y1;
     const float e3 = r.e * kThreeOverPi;
-    const bool all = fl & kFlagEllipseAll;
-    if (band && all) {
-        const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
-                                  float(rx) + 1.f);
-        if (bd.on) {
-            deposit_band(r, bd, ti, sw, static_cast<uint32_t>(__cvta_generic_to_shared(acc)), pxc,
-                         pyc, x0, x1, y0, y1);
-            return;
-        }
-    }
+    const bool all = rec_flags(p) & kFlagEllipseAll;
     const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, spans && all);
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
     const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
@@ -234,20 +243,7 @@ struct RowGeo {
     float A;                // |M (sx, 0)|^2: half the second difference of s along a row
 };
 
-// The clipped box of a record (pixel coordinates) and its centre pixel.
-__device__ __forceinline__ void rec_clip(const Rec& r, const TileInfo& ti, int& pxc, int& pyc,
-                                         int& x0, int& x1, int& y0, int& y1) {
-    const uint32_t p = r.packed;
-    pxc = ti.ox + rec_lx(p);
-    pyc = ti.oy + rec_ly(p);
-    const int rx = rec_rx(p), ry = rec_ry(p);
-    x0 = max(pxc - rx, 0);
-    x1 = min(pxc + rx, ti.W - 1);
-    y0 = max(pyc - ry, 0);
-    y1 = min(pyc + ry, ti.H - 1);
-}
-
-// Row walk of a record inside its clipped box (x0..y1, from rec_clip); false when the photon
+// Row walk of a record inside its clipped box (x0..y1, from rec_box); false when the photon
 // needs the generic walk (the image-half-size ellipse quirk of tiny images, or an M without a
 // band).
 __device__ __forceinline__ bool prep_rows(const Rec& r, const TileInfo& ti, int sw, int pxc,
@@ -451,35 +447,10 @@ __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-__device__ __forceinline__ Rec shfl_rec(const Rec& r, int src) {
-    Rec o;
-    o.dx0 = __shfl_sync(0xFFFFFFFFu, r.dx0, src);
-    o.dy0 = __shfl_sync(0xFFFFFFFFu, r.dy0, src);
-    o.m00 = __shfl_sync(0xFFFFFFFFu, r.m00, src);
-    o.m01 = __shfl_sync(0xFFFFFFFFu, r.m01, src);
-    o.m10 = __shfl_sync(0xFFFFFFFFu, r.m10, src);
-    o.m11 = __shfl_sync(0xFFFFFFFFu, r.m11, src);
-    o.e = __shfl_sync(0xFFFFFFFFu, r.e, src);
-    o.packed = __shfl_sync(0xFFFFFFFFu, r.packed, src);
-    return o;
-}
-
-// Clipped box of a record in pixel coordinates.
-__device__ __forceinline__ void rec_box(const Rec& r, const TileInfo& ti, int& pxc, int& pyc,
-                                        int& x0, int& x1, int& y0, int& y1) {
-    const uint32_t p = r.packed;
-    pxc = ti.ox + rec_lx(p);
-    pyc = ti.oy + rec_ly(p);
-    const int rx = rec_rx(p), ry = rec_ry(p);
-    x0 = max(pxc - rx, 0);
-    x1 = min(pxc + rx, ti.W - 1);
-    y0 = max(pyc - ry, 0);
-    y1 = min(pyc + ry, ti.H - 1);
-}
-
 // Forward deposit of one photon by the whole warp (see use_coop).
-__device__ __forceinline__ void deposit_coop(const Rec& r, const TileInfo& ti, int sw,
-                                             uint32_t acc_base, int lane) {
+__device__ __noinline__ void deposit_coop(const Rec* rp, TileInfo ti, int sw, uint32_t acc_base,
+                                          int lane) {
+    const Rec r = *rp;
     int pxc, pyc, x0, x1, y0, y1;
     rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
     const float e3 = r.e * kThreeOverPi;
@@ -501,96 +472,22 @@ __device__ __forceinline__ void deposit_coop(const Rec& r, const TileInfo& ti, i
     }
 }
 
-__device__ __forceinline__ void bbox_publish(int* sb, int x0, int x1, int y0, int y1) {
-    x0 = __reduce_min_sync(0xFFFFFFFFu, x0);
-    x1 = __reduce_max_sync(0xFFFFFFFFu, x1);
-    y0 = __reduce_min_sync(0xFFFFFFFFu, y0);
-    y1 = __reduce_max_sync(0xFFFFFFFFu, y1);
-    if ((threadIdx.x & 31) == 0 && x0 <= x1) {
-        atomicMin(sb + 0, x0);
-        atomicMax(sb + 1, x1);
-        atomicMin(sb + 2, y0);
-        atomicMax(sb + 3, y1);
-    }
-}
-
-// Adds the touched box of the accumulator into the image and clears it: warps take rows,
-// lanes take consecutive columns. When image rows are 16-byte aligned the adds are 4-wide
-// vector reductions (red.global.add.v4.f32) over 4-aligned column groups; columns of a group
-// outside the touched box add zero. All-zero groups are skipped.
-__device__ __forceinline__ void flush_tile(float* acc, int sw, const TileInfo& ti, float* out,
-                                           int* sb) {
-    __syncthreads();
-    const int x0 = sb[0], x1 = sb[1], y0 = sb[2], y1 = sb[3];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        sb[0] = INT_MAX; sb[1] = INT_MIN; sb[2] = INT_MAX; sb[3] = INT_MIN;
-    }
-    if (x0 <= x1 && !ti.in_image) {
-        // a plane outside the caller's buffer (an inconsistent simulation table): clear only
-        for (int gy = y0 + int(threadIdx.x >> 5); gy <= y1; gy += int(blockDim.x >> 5)) {
-            float* arow = acc + (gy - ti.oy) * sw - ti.ox;
-            for (int gx = x0 + int(threadIdx.x & 31); gx <= x1; gx += 32) arow[gx] = 0.f;
-        }
-    } else if (x0 <= x1) {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int nw = blockDim.x >> 5;
-        float* img = out + ti.img_off;
-        const bool vec = (ti.W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
-        if (vec) {
-            const int g0 = x0 >> 2, g1 = x1 >> 2;
-            for (int gy = y0 + warp; gy <= y1; gy += nw) {
-                float* arow = acc + (gy - ti.oy) * sw - ti.ox;
-                float* grow = img + int64_t(gy) * ti.W;
-                for (int g = g0 + lane; g <= g1; g += 32) {
-                    const int gx = g << 2;
-                    float v[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int c = gx + j;
-                        v[j] = 0.f;
-                        if (c >= x0 && c <= x1) {
-                            v[j] = arow[c];
-                            arow[c] = 0.f;
-                        }
-                    }
-                    if (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f)
-                        atomicAdd(reinterpret_cast<float4*>(grow + gx),
-                                  make_float4(v[0], v[1], v[2], v[3]));
-                }
-            }
-        } else {
-            for (int gy = y0 + warp; gy <= y1; gy += nw) {
-                float* arow = acc + (gy - ti.oy) * sw - ti.ox;
-                float* grow = img + int64_t(gy) * ti.W;
-                for (int gx = x0 + lane; gx <= x1; gx += 32) {
-                    const float v = arow[gx];
-                    if (v != 0.f) {
-                        atomicAdd(grow + gx, v);
-                        arow[gx] = 0.f;
-                    }
-                }
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// A run of sorted positions [begin, end) holding one screen tile's photons.
+// A run of sorted positions [begin, end) holding one screen tile's photons (positions and tiles
+// fit in 31 bits: the entry points reject larger calls).
 struct Segment {
-    uint32_t tile;
-    int64_t begin, end;
+    int tile;
+    uint32_t begin, end;
 };
 
 // End of tile t's photons: the start of its successor's first bucket.
-__device__ __forceinline__ int64_t tile_end(const TileArgs& a, int64_t t) {
-    return int64_t(__ldg(a.start + ((t + 1) << a.cfg.class_bits)));
+__device__ __forceinline__ uint32_t tile_end(const TileArgs& a, int t) {
+    return __ldg(a.start + ((int64_t(t) + 1) << a.cfg.class_bits));
 }
 
-__device__ __forceinline__ Segment first_segment(const TileArgs& a, int64_t chunk, int64_t p0) {
+__device__ __forceinline__ Segment first_segment(const TileArgs& a, uint32_t chunk, uint32_t p0) {
     Segment s;
     // (clamped, like the counters, so that a workspace without a plan stays in its arrays)
-    s.tile = uint32_t(min(int64_t(__ldg(a.chunk_tile + chunk)), a.n_tiles - 1));
+    s.tile = int(min(int64_t(__ldg(a.chunk_tile + chunk)), a.n_tiles - 1));
     s.begin = p0;
     s.end = tile_end(a, s.tile);
     return s;
@@ -598,91 +495,254 @@ __device__ __forceinline__ Segment first_segment(const TileArgs& a, int64_t chun
 
 // The segment after sg (sg.end below the tile path's photon count): the first tile after
 // sg.tile whose range is not empty, found by doubling steps then bisection (empty tiles are
-// usually few, so one probe mostly suffices). Every thread computes it from the same loads.
+// usually few, so one probe mostly suffices).
 __device__ __forceinline__ Segment next_segment(const TileArgs& a, const Segment& sg) {
-    const int64_t p = sg.end, t = sg.tile, last = a.n_tiles - 1;
-    int64_t k = 1;
-    while (t + k < last && tile_end(a, t + k) <= p) k <<= 1;
-    int64_t lo = t + (k >> 1) + 1, hi = min(t + k, last);
+    const uint32_t p = sg.end;
+    const int t = sg.tile, last = int(a.n_tiles) - 1;
+    int k = 1;
+    while (k < last - t && tile_end(a, t + k) <= p) k <<= 1;
+    int lo = t + (k >> 1) + 1, hi = k < last - t ? t + k : last;
     while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
+        const int mid = (lo + hi) >> 1;
         if (tile_end(a, mid) > p) hi = mid; else lo = mid + 1;
     }
     Segment s;
-    s.tile = uint32_t(lo);
+    s.tile = lo;
     s.begin = p;
     s.end = tile_end(a, lo);
     return s;
 }
 
-// Next chunk of sorted photons for this CTA: a shared work counter (reset to zero before the
-// launch) hands chunks out in order as CTAs finish, so CTAs that drew chunks of large
+// The current segment and its tile, held in shared memory: one thread finds and decodes the next
+// one while the others flush the last (two slots), and the photon loops read the fields they
+// need instead of keeping them all in registers across a walk.
+struct TileState {
+    Segment sg;
+    TileInfo ti;
+    int x0, x1, y0, y1;  // pixels its photons can touch: the tile and the plan's largest radius
+                         // around it, inside the image
+};
+
+__device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, TileState* t) {
+    t->sg = sg;
+    const TileInfo ti = decode_tile(a.sims, uint32_t(sg.tile), a.cfg, a.image_elems);
+    t->ti = ti;
+    const int m = a.cfg.apron - int(min(__ldg(a.tile_r + sg.tile), uint32_t(a.cfg.apron)));
+    t->x0 = max(ti.ox + m, 0);
+    t->y0 = max(ti.oy + m, 0);
+    t->x1 = min(ti.ox + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.W - 1);
+    t->y1 = min(ti.oy + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.H - 1);
+}
+
+// Next chunk of sorted photons for this CTA: a shared work counter (zero when the kernel starts)
+// hands chunks out in order as CTAs finish, so CTAs that drew chunks of large
 // footprints do not hold up the others. Nothing waits on it.
-__device__ __forceinline__ int64_t next_chunk(uint32_t* queue, uint32_t* slot) {
+__device__ __forceinline__ uint32_t next_chunk(uint32_t* queue, uint32_t* slot) {
     __syncthreads();
     if (threadIdx.x == 0) *slot = atomicAdd(queue, 1u);
     __syncthreads();
-    return int64_t(*slot);
+    return *slot;
+}
+
+// Called by every CTA after it drew its last chunk: the last CTA to do so leaves the work counter
+// at zero for the next launch on this plan (the count of finished CTAs wraps to zero by itself).
+// Nothing waits.
+__device__ __forceinline__ void finish_queue(uint32_t* queue) {
+    if (threadIdx.x == 0 && atomicInc(queue + 1, gridDim.x - 1u) == gridDim.x - 1u) *queue = 0u;
+}
+
+// ------------------------------------------------------------------ tail ---------------
+// Footprints wider than the apron (the plan's wide list) are splatted straight into global
+// memory, one warp per photon; their gradient records follow the tile path's in the stage. The
+// tile kernels do it after their last chunk: as kernels of their own they cost every call a
+// launch (1.5 us and the gap before it), and hardly any call has such footprints.
+
+struct Direct {
+    int pxc, pyc, x0, x1, y0, y1;
+    bool all;
+    float dx0, dy0, m00, m01, m10, m11, e;
+    float sx, sy;
+    double wd, hd;
+    int64_t img_off;
+    int W;
+};
+
+__device__ __forceinline__ bool direct_setup(const TileArgs& a, uint32_t rid, Direct& d) {
+    const int64_t n = a.ph.n;
+    const int s = find_sim_of_photon(a.sims, rid);
+    const pds_sim sim = load_sim(a.sims, s);
+    const int64_t ch = a.ph.cp[rid];
+    const float x = a.ph.X[rid], y = a.ph.X[n + rid];
+    const Footprint f = make_footprint(x, y, a.ph.R[rid], sim.height, sim.width, a.mpr);
+    if (!clip_box(f, sim.height, sim.width, d.x0, d.x1, d.y0, d.y1)) return false;
+    d.pxc = f.px_c;
+    d.pyc = f.py_c;
+    d.all = f.ellipse_all;
+    d.dx0 = corner_offset(f.px_c, sim.width, x);
+    d.dy0 = corner_offset(f.py_c, sim.height, y);
+    d.m00 = a.ph.M[rid];
+    d.m01 = a.ph.M[n + rid];
+    d.m10 = a.ph.M[3 * n + rid];
+    d.m11 = a.ph.M[4 * n + rid];
+    d.e = a.ph.E[rid];
+    d.sx = float(2.0 / double(sim.width));
+    d.sy = float(2.0 / double(sim.height));
+    d.wd = double(float(sim.width));
+    d.hd = double(float(sim.height));
+    d.img_off = sim.image_offset + ch * sim.height * sim.width;
+    if (d.img_off < 0 || d.img_off + int64_t(sim.height) * sim.width > a.image_elems) return false;
+    d.W = sim.width;
+    return true;
+}
+
+// (Out of line, so that its registers do not burden the walk before it.)
+__device__ __noinline__ void tail_forward(const TileArgs& a) {
+    const int64_t n_big = wide_count(a);
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t w = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_big;
+         w += warps) {
+        const uint32_t rid = __ldg(a.wide + w);
+        Direct d;
+        if (!direct_setup(a, rid, d) || !(d.e > 0.f)) continue;
+        const float e3 = d.e * kThreeOverPi;
+        const int bw = d.x1 - d.x0 + 1;
+        const int64_t total = int64_t(bw) * (d.y1 - d.y0 + 1);
+        float* img = a.out + d.img_off;
+        for (int64_t k = lane; k < total; k += 32) {
+            const int py = d.y0 + int(k / bw), px = d.x0 + int(k % bw);
+            const int kx = px - d.pxc, ky = py - d.pyc;
+            if (!d.all && !ellipse_ok(kx, ky, d.wd, d.hd)) continue;
+            const float dx = fmaf(float(kx), d.sx, d.dx0), dy = fmaf(float(ky), d.sy, d.dy0);
+            const float u0 = fmaf(d.m00, dx, d.m01 * dy), u1 = fmaf(d.m10, dx, d.m11 * dy);
+            const float s = fmaf(u0, u0, u1 * u1);
+            if (s < 1.f) {
+                const float t = 1.f - s;
+                atomicAdd(img + int64_t(py) * d.W + px, t * t * e3);
+            }
+        }
+    }
+}
+
+// Adds the pixels that the segment's photons can touch from the accumulator into the image and
+// clears them: warps take rows, lanes take consecutive columns. When image rows are 16-byte
+// aligned the adds are 4-wide vector reductions (red.global.add.v4.f32) over 4-aligned column
+// groups; columns of a group outside the range add zero. All-zero groups are skipped.
+__device__ __forceinline__ void flush_rows(float* acc, int sw, const TileState& t, float* out) {
+    const int x0 = t.x0, x1 = t.x1, y1 = t.y1;
+    const int ox = t.ti.ox, oy = t.ti.oy, W = t.ti.W;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = blockDim.x >> 5;
+    float* img = out + t.ti.img_off;
+    const bool vec = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
+    if (!t.ti.in_image) {
+        // a plane outside the caller's buffer (an inconsistent simulation table): clear only
+        for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
+            float* arow = acc + (gy - oy) * sw - ox;
+            for (int gx = x0 + lane; gx <= x1; gx += 32) arow[gx] = 0.f;
+        }
+    } else if (vec) {
+        const int g0 = x0 >> 2, g1 = x1 >> 2;
+        for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
+            float* arow = acc + (gy - oy) * sw - ox;
+            float* grow = img + int64_t(gy) * W;
+            for (int g = g0 + lane; g <= g1; g += 32) {
+                const int gx = g << 2;
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c = gx + j;
+                    v[j] = 0.f;
+                    if (c >= x0 && c <= x1) {
+                        v[j] = arow[c];
+                        arow[c] = 0.f;
+                    }
+                }
+                if (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f)
+                    atomicAdd(reinterpret_cast<float4*>(grow + gx),
+                              make_float4(v[0], v[1], v[2], v[3]));
+            }
+        }
+    } else {
+        for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
+            float* arow = acc + (gy - oy) * sw - ox;
+            float* grow = img + int64_t(gy) * W;
+            for (int gx = x0 + lane; gx <= x1; gx += 32) {
+                const float v = arow[gx];
+                if (v != 0.f) {
+                    atomicAdd(grow + gx, v);
+                    arow[gx] = 0.f;
+                }
+            }
+        }
+    }
+}
+
+// Ends a segment of the forward (all threads call it): the accumulator's pixels into the image;
+// with more, one thread of the last warp (which has the fewest rows) finds the next segment
+// meanwhile. Returns the slot of the tile state to use from here on.
+__device__ __forceinline__ int end_segment(const TileArgs& a, float* acc, int sw, TileState* ts,
+                                           int cur, bool more) {
+    __syncthreads();
+    if (more && threadIdx.x == blockDim.x - 1) set_tile(a, next_segment(a, ts[cur].sg), ts + (cur ^ 1));
+    flush_rows(acc, sw, ts[cur], a.out);
+    __syncthreads();
+    return more ? cur ^ 1 : cur;
 }
 
 template <int NT, int MINB>
-__global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(TileArgs a) {
+__global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ float acc[];
-    __shared__ int sb[4];
-    const Cfg cfg = a.cfg;
-    const int sw = cfg.sw;
+    __shared__ TileState ts[2];
+    __shared__ uint32_t chunk_slot;
+    const int sw = a.cfg.sw;
     Rec* stage = reinterpret_cast<Rec*>(acc + stage_offset_floats(sw));
     for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0.f;
-    if (threadIdx.x == 0) {
-        sb[0] = INT_MAX; sb[1] = INT_MIN; sb[2] = INT_MAX; sb[3] = INT_MIN;
-    }
-    __syncthreads();
     const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
-    const int64_t n_tile = tile_count(a);
-    const int64_t nchunks = (n_tile + cfg.chunk - 1) / cfg.chunk;
-    __shared__ uint32_t chunk_slot;
-    for (int64_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
          c = next_chunk(a.queue, &chunk_slot)) {
-        const int64_t p0 = c * cfg.chunk, p1 = min(p0 + cfg.chunk, n_tile);
-        if (p0 + threadIdx.x < p1) stage_rec_async(stage + threadIdx.x, a.srecs + p0 + threadIdx.x);
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        if (p0 + threadIdx.x < p1)
+            stage_rec_async(stage + threadIdx.x, a.srecs + p0 + threadIdx.x);
         cp_async_commit();
-        Segment sg = first_segment(a, c, p0);
-        TileInfo ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-        int buf = 0;
-        for (int64_t base = p0; base < p1; base += NT, buf ^= 1) {
-            const int64_t i = base + threadIdx.x;
-            const bool have = i < p1;
+        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), ts);
+        __syncthreads();
+        int cur = 0, buf = 0;
+        for (uint32_t base = p0; base < p1; base += NT, buf ^= 1) {
+            const uint32_t i = base + threadIdx.x;
             cp_async_wait_all();
-            Rec r = {};
-            if (have) r = stage[buf * NT + threadIdx.x];
+            const Rec* slot = stage + buf * NT + threadIdx.x;
             if (i + NT < p1) stage_rec_async(stage + (buf ^ 1) * NT + threadIdx.x, a.srecs + i + NT);
             cp_async_commit();
-            const int64_t bend = min(base + NT, p1);
             // The batch's segments (runs of one tile) are consecutive thread ranges; each
             // pass handles one and flushes the tile's accumulator when the next one starts.
             // Every pass but the first covers at least one photon, so NT + 1 passes suffice.
             for (int pass = 0; pass <= NT; ++pass) {
-                const bool mine = have && i >= sg.begin && i < sg.end;
-                const bool coop = mine && use_coop(r, cfg.coop_r);
-                int x0 = INT_MAX, x1 = INT_MIN, y0 = INT_MAX, y1 = INT_MIN;
-                if (mine && !coop) deposit(r, ti, sw, cfg.spans, cfg.band, acc, x0, x1, y0, y1);
-                if (coop) {
-                    int pxc, pyc;
-                    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+                const TileState& t = ts[cur];
+                bool coop = false;
+                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
+                    const Rec r = *slot;
+                    coop = use_coop(r, a.cfg.coop_r);
+                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip) &&
+                        !(a.cfg.band && deposit_band(r, t.ti, sw, acc_base)))
+                        deposit_generic(slot, t.ti, sw, a.cfg.spans, acc);
                 }
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                    const Rec rb = shfl_rec(r, __ffs(cm) - 1);
-                    deposit_coop(rb, ti, sw, acc_base, threadIdx.x & 31);
+                if (a.cfg.coop_r > 0) {
+                    __syncwarp();
+                    for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
+                        deposit_coop(stage + buf * NT + (threadIdx.x & ~31u) + (__ffs(cm) - 1),
+                                     t.ti, sw, acc_base, threadIdx.x & 31);
                 }
-                bbox_publish(sb, x0, x1, y0, y1);
-                if (sg.end >= bend) break;
-                flush_tile(acc, sw, ti, a.out, sb);
-                sg = next_segment(a, sg);
-                ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
+                if (t.sg.end >= min(base + NT, p1)) break;
+                cur = end_segment(a, acc, sw, ts, cur, true);
             }
         }
-        flush_tile(acc, sw, ti, a.out, sb);
+        end_segment(a, acc, sw, ts, cur, false);
     }
+    finish_queue(a.queue);
+    tail_forward(a);
 }
 
 // Stages the upstream gradient that a tile's photons read (clipped to the image): the tile and
@@ -691,19 +751,19 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(TileArgs a) {
 // the pixel after an odd row's end; the pitch sw = tile + 2 apron + 1 has room for it). The
 // apron's outer margin, which no photon of the tile reaches, is not loaded. Warps take rows,
 // lanes take consecutive columns.
-__device__ __forceinline__ void load_region(float* tg, int sw, const TileInfo& ti,
-                                            const float* grad, int apron, uint32_t r) {
-    const int m = apron - int(min(r, uint32_t(apron)));
-    const int gx0 = max(ti.ox + m, 0), gx1 = min(ti.ox + sw - m, ti.W);
-    const int gy0 = max(ti.oy + m, 0), gy1 = min(ti.oy + sw - m, ti.H);
+__device__ __forceinline__ void load_region(float* tg, int sw, const TileState& t,
+                                            const float* grad) {
+    const int gx1 = min(t.x1 + 1, t.ti.W - 1), y1 = t.y1;
+    const int ox = t.ti.ox, oy = t.ti.oy, W = t.ti.W;
+    const bool in_image = t.ti.in_image;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nw = blockDim.x >> 5;
-    const float* img = grad + ti.img_off;
-    for (int gy = gy0 + warp; gy < gy1; gy += nw) {
-        float* trow = tg + (gy - ti.oy) * sw - ti.ox;
-        const float* grow = img + int64_t(gy) * ti.W;
-        for (int gx = gx0 + lane; gx < gx1; gx += 32)
-            trow[gx] = ti.in_image ? __ldg(grow + gx) : 0.f;
+    const float* img = grad + t.ti.img_off;
+    for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
+        float* trow = tg + (gy - oy) * sw - ox;
+        const float* grow = img + int64_t(gy) * W;
+        for (int gx = t.x0 + lane; gx <= gx1; gx += 32)
+            trow[gx] = in_image ? __ldg(grow + gx) : 0.f;
     }
 }
 
@@ -877,12 +937,18 @@ __device__ __forceinline__ BandMoments gather_band_rows(const Band& bd, const Ba
     return m;
 }
 
-// Backward gather of one photon over its band rows ky0..ky1 (see BandWalk); with no row
-// inside the box (ky0 > ky1) its gradients are zero.
-__device__ __forceinline__ void gather_band(const Rec& r, const Band& bd, const TileInfo& ti,
-                                            int sw, const float* tg, uint32_t slot, int pxc,
-                                            int pyc, int ky0, int ky1, int kxb0, int kxb1,
-                                            GradRec* stage) {
+// Backward gather of one photon over its band's rows in the box (see BandWalk); with no row
+// inside the box (ky0 > ky1) its gradients are zero. False: the photon has no band.
+__device__ __forceinline__ bool gather_band(const Rec& r, const TileInfo& ti, int sw,
+                                            const float* tg, uint32_t slot, GradRec* stage) {
+    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
+    const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
+                              float(rec_rx(r.packed)) + 1.f);
+    if (!bd.on) return false;
+    int pxc, pyc, x0, x1, y0, y1;
+    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+    const int ky0 = max(bd.ky0, y0 - pyc), ky1 = min(bd.ky1, y1 - pyc);
+    const int kxb0 = x0 - pxc, kxb1 = x1 - pxc;
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
     const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
     const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
@@ -897,31 +963,23 @@ __device__ __forceinline__ void gather_band(const Rec& r, const Band& bd, const 
                            fmaf(2.f * ti.sx * r.dx0, m.B1t, r.dx0 * r.dx0 * m.A0t));
     finish_grad(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, m.sE, Sx, m.Sy, Sxx, m.Sxy,
                 m.Syy);
+    return true;
 }
 
-// Backward gather of one photon (photon_differentials.cu:169-218) from the staged gradient.
-// Pixels outside the support contribute 0 * g in the reference; with spans on they are not
-// visited. The offset d of pixel (kx, ky) is (kx sx + dx0, ky sy + dy0); moments in x are
-// kept in the integer offset kx and converted once per photon.
-__device__ __forceinline__ void gather(const Rec& r, const TileInfo& ti, int sw, bool spans,
-                                       bool band, const float* tg, uint32_t rid,
-                                       GradRec* stage) {
+// Backward gather of one photon without a band walk (photon_differentials.cu:169-218) from the
+// staged gradient. Pixels outside the support contribute 0 * g in the reference; with spans on
+// they are not visited. The offset d of pixel (kx, ky) is (kx sx + dx0, ky sy + dy0); moments in
+// x are kept in the integer offset kx and converted once per photon. Out of line, like
+// deposit_generic.
+__device__ __noinline__ void gather_generic(const Rec* rp, TileInfo ti, int sw, bool spans,
+                                            const float* tg, uint32_t rid, GradRec* stage) {
+    const Rec r = *rp;
     const uint32_t p = r.packed;
-    const uint32_t fl = rec_flags(p);
     const int pxc = ti.ox + rec_lx(p), pyc = ti.oy + rec_ly(p);
     const int rx = rec_rx(p), ry = rec_ry(p);
     const int x0 = max(pxc - rx, 0), x1 = min(pxc + rx, ti.W - 1);
     const int y0 = max(pyc - ry, 0), y1 = min(pyc + ry, ti.H - 1);
-    const bool all = fl & kFlagEllipseAll;
-    if (band && all) {
-        const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
-                                  float(rx) + 1.f);
-        if (bd.on) {
-            const int ky0 = max(bd.ky0, y0 - pyc), ky1 = min(bd.ky1, y1 - pyc);
-            gather_band(r, bd, ti, sw, tg, rid, pxc, pyc, ky0, ky1, x0 - pxc, x1 - pxc, stage);
-            return;
-        }
-    }
+    const bool all = rec_flags(p) & kFlagEllipseAll;
     const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, spans && all);
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
     int ky0 = y0 - pyc, ky1 = y1 - pyc;
@@ -968,9 +1026,9 @@ __device__ __forceinline__ void gather(const Rec& r, const TileInfo& ti, int sw,
 
 // Backward gather of one photon by the whole warp (see use_coop): lanes take rows and walk
 // their support spans, and a warp reduction hands the moments to the owning lane.
-__device__ __forceinline__ void gather_coop(const Rec& r, const TileInfo& ti, int sw,
-                                            const float* tg, uint32_t rid, int owner,
-                                            GradRec* stage) {
+__device__ __noinline__ void gather_coop(const Rec* rp, TileInfo ti, int sw, const float* tg,
+                                         uint32_t rid, int owner, GradRec* stage) {
+    const Rec r = *rp;
     const int lane = threadIdx.x & 31;
     int pxc, pyc, x0, x1, y0, y1;
     rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
@@ -1014,272 +1072,7 @@ __device__ __forceinline__ void gather_coop(const Rec& r, const TileInfo& ti, in
     }
 }
 
-template <int NT, int MINB>
-__global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(TileArgs a) {
-    extern __shared__ float tg[];
-    const Cfg cfg = a.cfg;
-    const int sw = cfg.sw;
-    const int64_t n_tile = tile_count(a);
-    const int64_t nchunks = (n_tile + cfg.chunk - 1) / cfg.chunk;
-    __shared__ uint32_t chunk_slot;
-    for (int64_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
-         c = next_chunk(a.queue, &chunk_slot)) {
-        const int64_t p0 = c * cfg.chunk, p1 = min(p0 + cfg.chunk, n_tile);
-        Segment sg = first_segment(a, c, p0);
-        TileInfo ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-        // next_chunk's barrier ends the previous chunk's reads of the staged tile
-        load_region(tg, sw, ti, a.grad, cfg.apron, __ldg(a.tile_r + sg.tile));
-        __syncthreads();
-        for (int64_t base = p0; base < p1; base += NT) {
-            const int64_t i = base + threadIdx.x;
-            const bool have = i < p1;
-            Rec r = {};
-            if (have) r = a.srecs[i];
-            const int64_t bend = min(base + NT, p1);
-            // consecutive segments of the batch, as in fwd_tiles_kernel; a photon's gradient
-            // record goes to its sorted position
-            for (int pass = 0; pass <= NT; ++pass) {
-                const bool mine = have && i >= sg.begin && i < sg.end;
-                const bool coop = mine && use_coop(r, cfg.coop_r);
-                if (mine && !coop) gather(r, ti, sw, cfg.spans, cfg.band, tg, uint32_t(i), a.stage);
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                    const int src = __ffs(cm) - 1;
-                    const Rec rb = shfl_rec(r, src);
-                    const uint32_t slot = uint32_t(base) + (threadIdx.x & ~31u) + uint32_t(src);
-                    gather_coop(rb, ti, sw, tg, slot, src, a.stage);
-                }
-                if (sg.end >= bend) break;
-                sg = next_segment(a, sg);
-                ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-                __syncthreads();
-                load_region(tg, sw, ti, a.grad, cfg.apron, __ldg(a.tile_r + sg.tile));
-                __syncthreads();
-            }
-        }
-    }
-}
-
-// ---- the padded-row walk's kernels (walk 4) ---------------------------------------------
-// The same persistent chunk and segment loop as fwd_tiles_kernel / bwd_tiles_kernel, with the
-// padded-row walk for the photons that have a band. A lane loads its record in the pass of its
-// segment only, and keeps just the row walk's constants across the walk; the rare paths (no
-// band, warp-cooperative splat) reload the record out of line, so their registers do not
-// burden the walk.
-
-__device__ __noinline__ void deposit_generic(const Rec* rp, TileInfo ti, int sw, bool spans,
-                                             float* acc) {
-    const Rec r = *rp;
-    int x0, x1, y0, y1;
-    deposit(r, ti, sw, spans, false, acc, x0, x1, y0, y1);
-}
-
-__device__ __noinline__ void deposit_coop_at(const Rec* rp, TileInfo ti, int sw, uint32_t acc_base,
-                                             int lane) {
-    deposit_coop(*rp, ti, sw, acc_base, lane);
-}
-
-__device__ __noinline__ void gather_generic(const Rec* rp, TileInfo ti, int sw, bool spans,
-                                            const float* tg, uint32_t rid, GradRec* stage) {
-    gather(*rp, ti, sw, spans, false, tg, rid, stage);
-}
-
-__device__ __noinline__ void gather_coop_at(const Rec* rp, TileInfo ti, int sw, const float* tg,
-                                            uint32_t rid, int owner, GradRec* stage) {
-    gather_coop(*rp, ti, sw, tg, rid, owner, stage);
-}
-
-template <int NT, int MINB>
-__global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(TileArgs a) {
-    extern __shared__ float acc[];
-    __shared__ int sb[4];
-    __shared__ uint32_t chunk_slot;
-    const Cfg cfg = a.cfg;
-    const int sw = cfg.sw;
-    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0.f;
-    if (threadIdx.x == 0) {
-        sb[0] = INT_MAX; sb[1] = INT_MIN; sb[2] = INT_MAX; sb[3] = INT_MIN;
-    }
-    __syncthreads();
-    const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
-    const int lane = threadIdx.x & 31;
-    // photon positions fit in 31 bits (the entry points reject larger calls)
-    const int n_tile = int(tile_count(a));
-    const int nchunks = (n_tile + cfg.chunk - 1) / cfg.chunk;
-    for (int c = int(next_chunk(a.queue, &chunk_slot)); c < nchunks;
-         c = int(next_chunk(a.queue, &chunk_slot))) {
-        const int p0 = c * cfg.chunk, p1 = min(p0 + cfg.chunk, n_tile);
-        Segment sg = first_segment(a, c, p0);
-        TileInfo ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-        for (int base = p0; base < p1; base += NT) {
-            const int i = base + int(threadIdx.x);
-            const int bend = min(base + NT, p1);
-            for (int pass = 0; pass <= NT; ++pass) {
-                const bool mine = i < p1 && i >= sg.begin && i < sg.end;
-                RowGeo g;
-                int rows = 0;
-                float e3 = 0.f;
-                bool generic = false, coop = false;
-                int x0 = INT_MAX, x1 = INT_MIN, y0 = INT_MAX, y1 = INT_MIN;
-                if (mine) {
-                    const Rec r = a.srecs[i];
-                    coop = use_coop(r, cfg.coop_r);
-                    if (coop || !(rec_flags(r.packed) & kFlagFwdSkip)) {
-                        int pxc, pyc;
-                        rec_clip(r, ti, pxc, pyc, x0, x1, y0, y1);
-                        if (!coop) {
-                            generic = !prep_rows(r, ti, sw, pxc, pyc, x0, x1, y0, y1, g);
-                            rows = generic ? 0 : g.rows;
-                            e3 = r.e * kThreeOverPi;
-                        }
-                    }
-                }
-                deposit_rows(g, rows, e3, acc_base, sw);
-                if (generic) deposit_generic(a.srecs + i, ti, sw, cfg.spans, acc);
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                    const int src = __ffs(cm) - 1;
-                    deposit_coop_at(a.srecs + (base + int(threadIdx.x & ~31u) + src), ti, sw,
-                                    acc_base, lane);
-                }
-                bbox_publish(sb, x0, x1, y0, y1);
-                if (sg.end >= bend) break;
-                flush_tile(acc, sw, ti, a.out, sb);
-                sg = next_segment(a, sg);
-                ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-            }
-        }
-        flush_tile(acc, sw, ti, a.out, sb);
-    }
-}
-
-template <int NT, int MINB>
-__global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(TileArgs a) {
-    extern __shared__ float tg[];
-    __shared__ uint32_t chunk_slot;
-    const Cfg cfg = a.cfg;
-    const int sw = cfg.sw;
-    const uint32_t tg_base = static_cast<uint32_t>(__cvta_generic_to_shared(tg));
-    const int n_tile = int(tile_count(a));
-    const int nchunks = (n_tile + cfg.chunk - 1) / cfg.chunk;
-    for (int c = int(next_chunk(a.queue, &chunk_slot)); c < nchunks;
-         c = int(next_chunk(a.queue, &chunk_slot))) {
-        const int p0 = c * cfg.chunk, p1 = min(p0 + cfg.chunk, n_tile);
-        Segment sg = first_segment(a, c, p0);
-        TileInfo ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-        // next_chunk's barrier ends the previous chunk's reads of the staged tile
-        load_region(tg, sw, ti, a.grad, cfg.apron, __ldg(a.tile_r + sg.tile));
-        __syncthreads();
-        for (int base = p0; base < p1; base += NT) {
-            const int i = base + int(threadIdx.x);
-            const int bend = min(base + NT, p1);
-            for (int pass = 0; pass <= NT; ++pass) {
-                const bool mine = i < p1 && i >= sg.begin && i < sg.end;
-                RowGeo g;
-                int rows = 0;
-                float dy0 = 0.f;
-                bool walk = false, generic = false, coop = false;
-                if (mine) {
-                    const Rec r = a.srecs[i];
-                    coop = use_coop(r, cfg.coop_r);
-                    if (!coop) {
-                        int pxc, pyc, x0, x1, y0, y1;
-                        rec_clip(r, ti, pxc, pyc, x0, x1, y0, y1);
-                        walk = prep_rows(r, ti, sw, pxc, pyc, x0, x1, y0, y1, g);
-                        generic = !walk;
-                        rows = walk ? g.rows : 0;
-                        dy0 = r.dy0;
-                    }
-                }
-                const RowMoments m = gather_rows(g, rows, tg_base, sw, ti.sy, dy0);
-                if (walk) finish_rows(a.stage, uint32_t(i), a.srecs[i], ti, m);
-                if (generic)
-                    gather_generic(a.srecs + i, ti, sw, cfg.spans, tg, uint32_t(i), a.stage);
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                    const int src = __ffs(cm) - 1;
-                    const int slot = base + int(threadIdx.x & ~31u) + src;
-                    gather_coop_at(a.srecs + slot, ti, sw, tg, uint32_t(slot), src, a.stage);
-                }
-                if (sg.end >= bend) break;
-                sg = next_segment(a, sg);
-                ti = decode_tile(a.sims, sg.tile, cfg, a.image_elems);
-                __syncthreads();
-                load_region(tg, sw, ti, a.grad, cfg.apron, __ldg(a.tile_r + sg.tile));
-                __syncthreads();
-            }
-        }
-    }
-}
-
-// ------------------------------------------------------------------ tail ---------------
-// Footprints wider than the apron (the plan's wide list) are splatted straight into global
-// memory, one warp per photon; their gradient records follow the tile path's in the stage.
-
-struct Direct {
-    int pxc, pyc, x0, x1, y0, y1;
-    bool all;
-    float dx0, dy0, m00, m01, m10, m11, e;
-    float sx, sy;
-    double wd, hd;
-    int64_t img_off;
-    int W;
-};
-
-__device__ __forceinline__ bool direct_setup(const TileArgs& a, uint32_t rid, Direct& d) {
-    const int64_t n = a.ph.n;
-    const int s = find_sim_of_photon(a.sims, rid);
-    const pds_sim sim = load_sim(a.sims, s);
-    const int64_t ch = a.ph.cp[rid];
-    const float x = a.ph.X[rid], y = a.ph.X[n + rid];
-    const Footprint f = make_footprint(x, y, a.ph.R[rid], sim.height, sim.width, a.mpr);
-    if (!clip_box(f, sim.height, sim.width, d.x0, d.x1, d.y0, d.y1)) return false;
-    d.pxc = f.px_c;
-    d.pyc = f.py_c;
-    d.all = f.ellipse_all;
-    d.dx0 = corner_offset(f.px_c, sim.width, x);
-    d.dy0 = corner_offset(f.py_c, sim.height, y);
-    d.m00 = a.ph.M[rid];
-    d.m01 = a.ph.M[n + rid];
-    d.m10 = a.ph.M[3 * n + rid];
-    d.m11 = a.ph.M[4 * n + rid];
-    d.e = a.ph.E[rid];
-    d.sx = float(2.0 / double(sim.width));
-    d.sy = float(2.0 / double(sim.height));
-    d.wd = double(float(sim.width));
-    d.hd = double(float(sim.height));
-    d.img_off = sim.image_offset + ch * sim.height * sim.width;
-    if (d.img_off < 0 || d.img_off + int64_t(sim.height) * sim.width > a.image_elems) return false;
-    d.W = sim.width;
-    return true;
-}
-
-__global__ __launch_bounds__(256) void tail_fwd_kernel(TileArgs a) {
-    const int64_t n_big = wide_count(a);
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t w = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_big;
-         w += warps) {
-        const uint32_t rid = __ldg(a.wide + w);
-        Direct d;
-        if (!direct_setup(a, rid, d) || !(d.e > 0.f)) continue;
-        const float e3 = d.e * kThreeOverPi;
-        const int bw = d.x1 - d.x0 + 1;
-        const int64_t total = int64_t(bw) * (d.y1 - d.y0 + 1);
-        float* img = a.out + d.img_off;
-        for (int64_t k = lane; k < total; k += 32) {
-            const int py = d.y0 + int(k / bw), px = d.x0 + int(k % bw);
-            const int kx = px - d.pxc, ky = py - d.pyc;
-            if (!d.all && !ellipse_ok(kx, ky, d.wd, d.hd)) continue;
-            const float dx = fmaf(float(kx), d.sx, d.dx0), dy = fmaf(float(ky), d.sy, d.dy0);
-            const float u0 = fmaf(d.m00, dx, d.m01 * dy), u1 = fmaf(d.m10, dx, d.m11 * dy);
-            const float s = fmaf(u0, u0, u1 * u1);
-            if (s < 1.f) {
-                const float t = 1.f - s;
-                atomicAdd(img + int64_t(py) * d.W + px, t * t * e3);
-            }
-        }
-    }
-}
-
-__global__ __launch_bounds__(256) void tail_bwd_kernel(TileArgs a) {
+__device__ __noinline__ void tail_backward(const TileArgs& a) {
     const int64_t n_tile = tile_count(a), n_big = wide_count(a);
     const int lane = threadIdx.x & 31;
     const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
@@ -1327,6 +1120,168 @@ __global__ __launch_bounds__(256) void tail_bwd_kernel(TileArgs a) {
                         Sy, Sxx, Sxy, Syy);
         }
     }
+}
+
+// Moves the backward on to the next segment's tile (all threads call it).
+__device__ __forceinline__ void next_tile(const TileArgs& a, float* tg, int sw, TileState* t) {
+    __syncthreads();
+    if (threadIdx.x == 0) set_tile(a, next_segment(a, t->sg), t);
+    __syncthreads();
+    load_region(tg, sw, *t, a.grad);
+    __syncthreads();
+}
+
+template <int NT, int MINB>
+__global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_constant__ TileArgs a) {
+    extern __shared__ float tg[];
+    __shared__ TileState t;
+    __shared__ uint32_t chunk_slot;
+    const int sw = a.cfg.sw;
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
+         c = next_chunk(a.queue, &chunk_slot)) {
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        // next_chunk's barrier ends the previous chunk's reads of the tile state and the tile
+        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), &t);
+        __syncthreads();
+        load_region(tg, sw, t, a.grad);
+        __syncthreads();
+        for (uint32_t base = p0; base < p1; base += NT) {
+            const uint32_t i = base + threadIdx.x;
+            // consecutive segments of the batch, as in fwd_tiles_kernel; a photon's gradient
+            // record goes to its sorted position
+            for (int pass = 0; pass <= NT; ++pass) {
+                bool coop = false;
+                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
+                    const Rec r = a.srecs[i];
+                    coop = use_coop(r, a.cfg.coop_r);
+                    if (!coop && !(a.cfg.band && gather_band(r, t.ti, sw, tg, i, a.stage)))
+                        gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
+                }
+                if (a.cfg.coop_r > 0) {
+                    for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
+                        const int src = __ffs(cm) - 1;
+                        const uint32_t slot = base + (threadIdx.x & ~31u) + uint32_t(src);
+                        gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
+                    }
+                }
+                if (t.sg.end >= min(base + NT, p1)) break;
+                next_tile(a, tg, sw, &t);
+            }
+        }
+    }
+    finish_queue(a.queue);
+    tail_backward(a);
+}
+
+// ---- the padded-row walk's kernels (walk 4) ---------------------------------------------
+// The same persistent chunk and segment loop as fwd_tiles_kernel / bwd_tiles_kernel, with the
+// padded-row walk for the photons that have a band. A lane loads its record in the pass of its
+// segment only, and keeps just the row walk's constants across the walk.
+
+template <int NT, int MINB>
+__global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constant__ TileArgs a) {
+    extern __shared__ float acc[];
+    __shared__ TileState ts[2];
+    __shared__ uint32_t chunk_slot;
+    const int sw = a.cfg.sw;
+    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0.f;
+    const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
+         c = next_chunk(a.queue, &chunk_slot)) {
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), ts);
+        __syncthreads();
+        int cur = 0;
+        for (uint32_t base = p0; base < p1; base += NT) {
+            const uint32_t i = base + threadIdx.x;
+            for (int pass = 0; pass <= NT; ++pass) {
+                const TileState& t = ts[cur];
+                RowGeo g;
+                int rows = 0;
+                float e3 = 0.f;
+                bool generic = false, coop = false;
+                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
+                    const Rec r = a.srecs[i];
+                    coop = use_coop(r, a.cfg.coop_r);
+                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
+                        int pxc, pyc, x0, x1, y0, y1;
+                        rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
+                        generic = !prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
+                        rows = generic ? 0 : g.rows;
+                        e3 = r.e * kThreeOverPi;
+                    }
+                }
+                deposit_rows(g, rows, e3, acc_base, sw);
+                if (generic) deposit_generic(a.srecs + i, t.ti, sw, a.cfg.spans, acc);
+                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
+                    deposit_coop(a.srecs + (base + (threadIdx.x & ~31u) + (__ffs(cm) - 1)), t.ti,
+                                 sw, acc_base, threadIdx.x & 31);
+                if (t.sg.end >= min(base + NT, p1)) break;
+                cur = end_segment(a, acc, sw, ts, cur, true);
+            }
+        }
+        end_segment(a, acc, sw, ts, cur, false);
+    }
+    finish_queue(a.queue);
+    tail_forward(a);
+}
+
+template <int NT, int MINB>
+__global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(const __grid_constant__ TileArgs a) {
+    extern __shared__ float tg[];
+    __shared__ TileState t;
+    __shared__ uint32_t chunk_slot;
+    const int sw = a.cfg.sw;
+    const uint32_t tg_base = static_cast<uint32_t>(__cvta_generic_to_shared(tg));
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
+         c = next_chunk(a.queue, &chunk_slot)) {
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        // next_chunk's barrier ends the previous chunk's reads of the tile state and the tile
+        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), &t);
+        __syncthreads();
+        load_region(tg, sw, t, a.grad);
+        __syncthreads();
+        for (uint32_t base = p0; base < p1; base += NT) {
+            const uint32_t i = base + threadIdx.x;
+            for (int pass = 0; pass <= NT; ++pass) {
+                RowGeo g;
+                int rows = 0;
+                float dy0 = 0.f;
+                bool walk = false, generic = false, coop = false;
+                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
+                    const Rec r = a.srecs[i];
+                    coop = use_coop(r, a.cfg.coop_r);
+                    if (!coop) {
+                        int pxc, pyc, x0, x1, y0, y1;
+                        rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
+                        walk = prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
+                        generic = !walk;
+                        rows = walk ? g.rows : 0;
+                        dy0 = r.dy0;
+                    }
+                }
+                const RowMoments m = gather_rows(g, rows, tg_base, sw, t.ti.sy, dy0);
+                if (walk) finish_rows(a.stage, i, a.srecs[i], t.ti, m);
+                if (generic)
+                    gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
+                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
+                    const int src = __ffs(cm) - 1;
+                    const uint32_t slot = base + (threadIdx.x & ~31u) + uint32_t(src);
+                    gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
+                }
+                if (t.sg.end >= min(base + NT, p1)) break;
+                next_tile(a, tg, sw, &t);
+            }
+        }
+    }
+    finish_queue(a.queue);
+    tail_backward(a);
 }
 
 // Spreads the gradient records into the reference's outputs grad_Ep[N], grad_xp[2][N],
@@ -1425,28 +1380,12 @@ __global__ __launch_bounds__(256) void grad_scatter4_kernel(TileArgs a) {
 
 constexpr int kTileThreads = 256;
 
-int num_sms() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Grid of a persistent tile kernel: resident CTAs per SM x SMs, capped by the work.
-template <typename K>
-int persistent_grid(K kernel, size_t smem, int64_t n_units) {
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTileThreads, smem);
-    if (per_sm < 1) per_sm = 1;
-    const int64_t g = int64_t(per_sm) * num_sms();
+template <auto Kernel>
+int persistent_grid(size_t smem, int64_t n_units) {
+    const int64_t g = int64_t(num_sms()) * resident_ctas<Kernel>(kTileThreads, smem);
     const int64_t need = n_units > 0 ? n_units : 1;
     return int(g < need ? g : need);
-}
-
-template <typename K>
-cudaError_t set_smem(K kernel, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
 }
 
 }  // namespace
@@ -1463,58 +1402,46 @@ size_t tile_smem(const TileArgs& a, bool staged) {
 template <int MINB, bool ROWS>
 cudaError_t launch_forward_t(const TileArgs& a, cudaStream_t st) {
     const size_t smem = tile_smem(a, !ROWS);
-    auto kern = ROWS ? fwd_rows_kernel<kTileThreads, MINB> : fwd_tiles_kernel<kTileThreads, MINB>;
-    cudaError_t e = set_smem(kern, smem);
+    constexpr auto kern = ROWS ? fwd_rows_kernel<kTileThreads, MINB>
+                               : fwd_tiles_kernel<kTileThreads, MINB>;
+    const cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int64_t chunks = (a.ph.n + a.cfg.chunk - 1) / a.cfg.chunk;
-    if (chunks > 0) {
-        const int grid = persistent_grid(kern, smem, chunks);
-        kern<<<grid, kTileThreads, smem, st>>>(a);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        const int tgrid = num_sms() * 2;
-        tail_fwd_kernel<<<tgrid, 256, 0, st>>>(a);
-        e = cudaGetLastError();
-    }
-    return e;
+    if (chunks <= 0) return cudaSuccess;
+    kern<<<persistent_grid<kern>(smem, chunks), kTileThreads, smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 template <int MINB, bool ROWS>
 cudaError_t launch_backward_t(const TileArgs& a, cudaStream_t st) {
     const size_t smem = tile_smem(a, false);
-    auto kern = ROWS ? bwd_rows_kernel<kTileThreads, MINB> : bwd_tiles_kernel<kTileThreads, MINB>;
-    cudaError_t e = set_smem(kern, smem);
+    constexpr auto kern = ROWS ? bwd_rows_kernel<kTileThreads, MINB>
+                               : bwd_tiles_kernel<kTileThreads, MINB>;
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int64_t chunks = (a.ph.n + a.cfg.chunk - 1) / a.cfg.chunk;
-    if (chunks > 0) {
-        const int grid = persistent_grid(kern, smem, chunks);
-        kern<<<grid, kTileThreads, smem, st>>>(a);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        const int tgrid = num_sms() * 2;
-        tail_bwd_kernel<<<tgrid, 256, 0, st>>>(a);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        // the quad form needs the inverse map 16-byte aligned (the workspace is) and every
-        // output 4-byte aligned; the rows' own alignment is handled per store
-        // no outputs: the gradients stay in the workspace as records (read by the refraction
-        // backward's records mode)
-        if (!a.gE) return cudaSuccess;
-        const auto al = [](const void* p, uintptr_t m) {
-            return (reinterpret_cast<uintptr_t>(p) & m) == 0;
-        };
-        const bool vec = al(a.inv, 15) && al(a.gE, 3) && al(a.gX, 3) && al(a.gM, 3);
-        const int64_t items = vec ? a.ph.n / 4 : a.ph.n;
-        const int64_t sblocks = items > 0 ? (items + 255) / 256 : 1;
-        const int64_t scap = int64_t(num_sms()) * 16;
-        const unsigned sgrid = unsigned(sblocks < scap ? sblocks : scap);
-        if (vec)
-            grad_scatter4_kernel<<<sgrid, 256, 0, st>>>(a);
-        else
-            grad_scatter_kernel<<<sgrid, 256, 0, st>>>(a);
-        e = cudaGetLastError();
-    }
-    return e;
+    if (chunks <= 0) return cudaSuccess;
+    kern<<<persistent_grid<kern>(smem, chunks), kTileThreads, smem, st>>>(a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    // no outputs: the gradients stay in the workspace as records (read by the refraction
+    // backward's records mode)
+    if (!a.gE) return cudaSuccess;
+    // the quad form needs the inverse map 16-byte aligned (the workspace is) and every
+    // output 4-byte aligned; the rows' own alignment is handled per store
+    const auto al = [](const void* p, uintptr_t m) {
+        return (reinterpret_cast<uintptr_t>(p) & m) == 0;
+    };
+    const bool vec = al(a.inv, 15) && al(a.gE, 3) && al(a.gX, 3) && al(a.gM, 3);
+    const int64_t items = vec ? a.ph.n / 4 : a.ph.n;
+    const int64_t sblocks = items > 0 ? (items + 255) / 256 : 1;
+    const int64_t scap = int64_t(num_sms()) * 16;
+    const unsigned sgrid = unsigned(sblocks < scap ? sblocks : scap);
+    if (vec)
+        grad_scatter4_kernel<<<sgrid, 256, 0, st>>>(a);
+    else
+        grad_scatter_kernel<<<sgrid, 256, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_forward(const TileArgs& a, cudaStream_t st) {

@@ -30,24 +30,25 @@ struct PlanArgs {
     uint32_t* wide;      // [n] out: photon index of the k-th wide photon (count pass)
     uint32_t* counters;  // [0] tile-path, [1] wide, [2] untouched photons; zeroed by caller
     uint32_t* cta_hist;  // [plan_hist_entries] each CTA's window histogram, count -> place
-    uint32_t* cursor;    // [key_big] place cursors (the bucket starts, from the scan)
+    uint32_t* cursor;    // [key_big] place cursors: the bucket starts, from the scan, or zeros
+                         // where the place pass scans (fused)
+    uint32_t* start;     // [key_big + 1] out, fused: the bucket starts, then the total
+    uint32_t* chunk_tile;  // [n / chunk + 1] out: tile of each work chunk's first photon (place)
     Rec* srecs;          // [n] out: records in sorted order (place pass)
     uint32_t* tile_r;    // [tiles] out: the largest box radius max(rx, ry) of each tile's
                          // tile-path photons (count pass); zeroed by the caller
     int64_t range;       // photons per CTA (plan_shape)
     int32_t window;      // buckets of each CTA's shared histogram (plan_shape)
+    int32_t fused;       // 1: the place pass scans the counts itself (plan_fused)
 };
 
-// Bucket scan and the chunks' tiles.
+// Bucket scan.
 struct ScanArgs {
     const uint32_t* counts;
-    const uint32_t* counters;
     uint32_t* part;        // [bucket_scan_parts(nb)] scan partials
     uint32_t* start;       // [nb + 1] out: first sorted position of each bucket, then the total
     uint32_t* cursor;      // [nb] out: a copy of the starts for the place pass
-    uint32_t* chunk_tile;  // [n / chunk + 1] out: tile of each work chunk's first photon
-    int64_t n, nb, n_tiles;
-    int32_t chunk, cb;
+    int64_t nb;
 };
 
 struct TileArgs {
@@ -63,7 +64,8 @@ struct TileArgs {
     const uint32_t* wide;        // photon index of each wide photon
     const uint32_t* tile_r;      // largest box radius of each tile's photons (plan)
     const uint32_t* counters;
-    uint32_t* queue;             // chunk work counter of the tile kernel (zeroed before launch)
+    uint32_t* queue;             // [2] chunk work counter of the tile kernel, then its count of
+                                 // finished CTAs (zero before a launch and after it)
     float* out;                  // forward: flat image buffer (zeroed by caller)
     const float* grad;           // backward: flat upstream gradient buffer
     int64_t image_elems;         // elements of out / grad: image planes past it are not touched
@@ -74,13 +76,13 @@ struct TileArgs {
                                  // photons (workspace)
 };
 
+bool plan_fused(int64_t nb);
 int64_t bucket_scan_parts(int64_t nb);
 void plan_shape(int64_t n, int64_t nb, int32_t* window, int64_t* range);
 int64_t plan_hist_entries(int64_t n, int64_t nb);
 cudaError_t launch_plan_count(const PlanArgs& a, cudaStream_t st);
 cudaError_t launch_bucket_scan(const ScanArgs& a, cudaStream_t st);
 cudaError_t launch_plan_place(const PlanArgs& a, cudaStream_t st);
-cudaError_t launch_chunk_tiles(const ScanArgs& a, cudaStream_t st);
 cudaError_t launch_plan_export(const uint32_t* inv, const uint32_t* start, int64_t nb,
                                uint32_t key_big, uint32_t key_invalid, int64_t n,
                                uint32_t* bucket, uint32_t* slot, cudaStream_t st);
