@@ -351,22 +351,4 @@ __device__ __forceinline__ float corner_offset(int32_t p_c, int32_t W, float x) 
     return corner_offset_step(p_c, corner_step(W), x);
 }
 
-// Predicated shared-memory add without a branch (the compiler otherwise branches around
-// the atomic per pixel).
-__device__ __forceinline__ void red_shared_add_if(bool p, const float* addr, float v) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(addr));
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q red.shared.add.f32 [%0], %1;\n\t}"
-        :: "r"(a), "f"(v), "r"(int(p)) : "memory");
-}
-
-// Shared add of v at shared byte address a + OFF when s < 1 (the kernel's support), as one
-// predicated reduction: no branch per pixel.
-template <int OFF>
-__device__ __forceinline__ void red_shared_inside(uint32_t a, float s, float v) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.lt.f32 q, %1, 0f3F800000;\n\t@q red.shared.add.f32 [%0+%3], %2;\n\t}"
-        :: "r"(a), "f"(s), "f"(v), "n"(OFF) : "memory");
-}
-
 }  // namespace pds

@@ -78,30 +78,174 @@ __device__ __forceinline__ TileInfo decode_tile(const SimTable& st, uint32_t til
     return t;
 }
 
-// One row of a forward deposit: n pixels from shared byte address a, with
-// u = (k M00 sx + b0, k M10 sx + b1) at the k-th pixel, s = |u|^2, and a predicated shared add
-// of E 3/pi (1 - s)^2 where s < 1 (the reference's value > 0, photon_differentials.cu:105-106).
-// Lanes of a warp hold photons of one footprint class, so n is nearly always warp-uniform and
-// the loop stays converged; it is unrolled by two.
-__device__ __forceinline__ void fwd_row(int n, uint32_t a, float b0, float b1, float a00,
-                                        float a10, float e3) {
-    float kf = 0.f;
-    int k = 0;
-    for (; k + 1 < n; k += 2) {
-        const float u0 = fmaf(kf, a00, b0), u1 = fmaf(kf, a10, b1);
-        const float v0 = u0 + a00, v1 = u1 + a10;
-        const float s = fmaf(u0, u0, u1 * u1), s2 = fmaf(v0, v0, v1 * v1);
-        const float t = 1.f - s, t2 = 1.f - s2;
-        red_shared_inside<0>(a, s, (t * e3) * t);
-        red_shared_inside<4>(a, s2, (t2 * e3) * t2);
-        a += 8u;
-        kf += 2.f;
+// A run of sorted positions [begin, end) holding one screen tile's photons (positions and tiles
+// fit in 31 bits: the entry points reject larger calls).
+struct Segment {
+    int tile;
+    uint32_t begin, end;
+};
+
+// End of tile t's photons: the start of its successor's first bucket.
+__device__ __forceinline__ uint32_t tile_end(const TileArgs& a, int t) {
+    return __ldg(a.start + ((int64_t(t) + 1) << a.cfg.class_bits));
+}
+
+__device__ __forceinline__ Segment first_segment(const TileArgs& a, uint32_t chunk, uint32_t p0) {
+    Segment s;
+    // (clamped, like the counters, so that a workspace without a plan stays in its arrays)
+    s.tile = int(min(int64_t(__ldg(a.chunk_tile + chunk)), a.n_tiles - 1));
+    s.begin = p0;
+    s.end = tile_end(a, s.tile);
+    return s;
+}
+
+// The segment after sg (sg.end below the tile path's photon count): the first tile after
+// sg.tile whose range is not empty, found by doubling steps then bisection (empty tiles are
+// usually few, so one probe mostly suffices).
+__device__ __forceinline__ Segment next_segment(const TileArgs& a, const Segment& sg) {
+    const uint32_t p = sg.end;
+    const int t = sg.tile, last = int(a.n_tiles) - 1;
+    int k = 1;
+    while (k < last - t && tile_end(a, t + k) <= p) k <<= 1;
+    int lo = t + (k >> 1) + 1, hi = k < last - t ? t + k : last;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (tile_end(a, mid) > p) hi = mid; else lo = mid + 1;
     }
-    if (k < n) {
-        const float u0 = fmaf(kf, a00, b0), u1 = fmaf(kf, a10, b1);
-        const float s = fmaf(u0, u0, u1 * u1);
-        const float t = 1.f - s;
-        red_shared_inside<0>(a, s, (t * e3) * t);
+    Segment s;
+    s.tile = lo;
+    s.begin = p;
+    s.end = tile_end(a, lo);
+    return s;
+}
+
+// The current segment and its tile, held in shared memory: one thread finds and decodes the next
+// one while the others flush the last (two slots), and the photon loops read the fields they
+// need instead of keeping them all in registers across a walk.
+struct TileState {
+    Segment sg;
+    TileInfo ti;
+    int x0, x1, y0, y1;  // pixels its photons can touch: the tile and the plan's largest radius
+                         // around it, inside the image
+    float scale, unit;   // forward: accumulator counts per unit of energy density (a power of
+                         // two) and its inverse; scale 0: no photon is accumulated
+    uint32_t wrapped;    // forward: non-zero where a pixel's count has wrapped
+};
+
+__device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, TileState* t) {
+    t->sg = sg;
+    const TileInfo ti = decode_tile(a.sims, uint32_t(sg.tile), a.cfg, a.image_elems);
+    t->ti = ti;
+    const int m = a.cfg.apron - int(min(__ldg(a.tile_r + sg.tile), uint32_t(a.cfg.apron)));
+    t->x0 = max(ti.ox + m, 0);
+    t->y0 = max(ti.oy + m, 0);
+    t->x1 = min(ti.ox + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.W - 1);
+    t->y1 = min(ti.oy + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.H - 1);
+}
+
+// ---- the forward's accumulator -----------------------------------------------------------
+// A tile's pixels are summed as 32-bit fixed-point counts: a shared integer add is one native
+// instruction whatever the lanes' addresses, where a shared float add is a compare-and-swap loop
+// of about eight (measured a warp and SM, random pixels of a tile: 3.1 against 8.9 cycles with
+// the loop around it; all lanes in 32 pixels, as in a focused caustic: 3.1 against 34).
+//
+// The count is a power of two chosen per segment from a sample of its photons (set_scale): with
+// c the photons' mean number of covers of a pixel if they were spread over the tile, 2^32
+// counts hold about 64 c typical peaks (at most all of the segment's photons on one pixel). An
+// add is rounded to half a count, so a pixel's sum is off by about 7e-9 sqrt(c) of it where
+// the photons are spread out; a float sum of c adds is off by 1.4e-8 sqrt(c).
+// - A pixel whose count wraps (photons gathered on few pixels) is seen by the lane that causes
+//   it, from the old count that the add returns. The band walk only marks the segment, without
+//   a branch per pixel, and a marked segment is summed again by redo_segment; the other walks
+//   add the 2^32 counts to the image pixel on the spot (add_pixel).
+// - A photon whose peak reaches 2^31 counts (at least 2^6 typical ones), or any photon where no
+//   power of two in float range fits, is added to the image directly, in float (deposit_direct).
+constexpr int kMaxCountBits = 25;  // counts of a typical peak at most, leaving the 2^6 above
+constexpr float kCountLimit = 2147483648.f;
+
+// Sets t's scale from at most 32 photons spread evenly over the sorted positions [begin, end),
+// one a lane (the whole warp calls it): the geometric mean of their energies as a power of two,
+// and their mean support pi / |det M|, at most their box.
+__device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uint32_t end,
+                                          TileState* t) {
+    const uint32_t lane = threadIdx.x & 31, n = end > begin ? end - begin : 0u;
+    float e = 0.f, area = 0.f;
+    if (n > 0) {
+        const Rec r = a.srecs[begin + uint32_t((uint64_t(n) * lane) >> 5)];
+        e = r.e;
+        const float det = fabsf(fmaf(r.m00, r.m11, -r.m01 * r.m10)) * t->ti.sx * t->ti.sy;
+        const float box = float((2 * rec_rx(r.packed) + 1) * (2 * rec_ry(r.packed) + 1));
+        area = fminf(__fdividef(3.1415927f, det), box);  // (NaN, inf: the box)
+    }
+    const bool use = e > 0.f && e < __int_as_float(0x7F800000);
+    const int sum = __reduce_add_sync(0xFFFFFFFFu, use ? (__float_as_int(e) >> 23) - 127 : 0);
+    const int count = __popc(__ballot_sync(0xFFFFFFFFu, use));
+    const int area16 = __reduce_add_sync(0xFFFFFFFFu, int(area * 16.f));  // mean area * 512
+    if (lane == 0) {
+        const int tile = a.cfg.tile;
+        const float pixels = float(min(tile, t->ti.W) * min(tile, t->ti.H));
+        const float peaks = 32.f * float(n) * (float(area16) * (1.f / 512.f)) / pixels;
+        // ceil(log2) of min(peaks, n): the exponent of the next float below, plus one
+        const int room = (__float_as_int(fmaxf(fminf(peaks, float(n)), 1.f) * 0.99999994f) >> 23) - 126;
+        const int bits = min(kMaxCountBits, 30 - room);
+        const int k = count > 0 ? bits - __float2int_rd(float(sum) / float(count)) : 127;
+        const bool fits = k <= 126;
+        t->scale = fits ? __int_as_float((k + 127) << 23) : 0.f;
+        t->unit = fits ? __int_as_float((127 - k) << 23) : 0.f;
+        t->wrapped = 0u;
+    }
+}
+
+// The photon's peak E 3/pi in counts, or 0 for one that goes to the image directly.
+__device__ __forceinline__ float count_peak(const TileState& t, float e) {
+    const float p = (e * kThreeOverPi) * t.scale;
+    return p < kCountLimit ? p : 0.f;
+}
+
+// Adds the 2^32 counts that the pixel at shared byte address `at` has wrapped by to the image.
+__device__ __forceinline__ void carry_pixel(const TileArgs& a, const TileState& t,
+                                            uint32_t acc_base, uint32_t at) {
+    const uint32_t idx = (at - acc_base) >> 2;
+    const int sw = a.cfg.sw;
+    // idx / sw: exact, (idx + 1/2) / sw is at least 1 / (2 sw) from an integer
+    const int y = __float2int_rd((float(idx) + 0.5f) * (1.f / float(sw)));
+    const int x = int(idx) - y * sw;
+    if (t.ti.in_image)
+        atomicAdd(a.out + t.ti.img_off + int64_t(t.ti.oy + y) * t.ti.W + (t.ti.ox + x),
+                  t.unit * 4294967296.f);
+}
+
+// One pixel of a deposit: s = |u|^2 and the photon's peak in counts; adds peak (1 - s)^2 where
+// s < 1 and in (the reference's value > 0, photon_differentials.cu:105-106).
+__device__ __forceinline__ void add_pixel(const TileArgs& a, const TileState& t, uint32_t acc_base,
+                                          uint32_t at, float s, float peak, bool in = true) {
+    if (!(in && s < 1.f)) return;
+    const float d = 1.f - s;
+    const uint32_t v = __float2uint_rn((d * peak) * d);
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+    if (old + v < v) carry_pixel(a, t, acc_base, at);
+}
+
+// Adds the counts v0, v1 to the pixels at shared byte addresses at, at + 4 and counts the wraps.
+// Unconditional (a pixel outside the support gets 0): ptxas branches around a predicated atomic.
+__device__ __forceinline__ void add_pair(uint32_t at, uint32_t v0, uint32_t v1, uint32_t& wraps) {
+    asm volatile(
+        "{\n\t.reg .b32 a, b;\n\t"
+        "atom.shared.add.u32 a, [%1], %2;\n\tatom.shared.add.u32 b, [%1+4], %3;\n\t"
+        "add.cc.u32 a, a, %2;\n\taddc.u32 %0, %0, 0;\n\t"
+        "add.cc.u32 b, b, %3;\n\taddc.u32 %0, %0, 0;\n\t}"
+        : "+r"(wraps) : "r"(at), "r"(v0), "r"(v1) : "memory");
+}
+
+// One row of a forward deposit: n pixels from shared byte address `at`, with
+// u = (k M00 sx + b0, k M10 sx + b1) at the k-th pixel.
+__device__ __forceinline__ void fwd_row(const TileArgs& a, const TileState& t, uint32_t acc_base,
+                                        int n, uint32_t at, float b0, float b1, float a00,
+                                        float a10, float peak) {
+    for (int k = 0; k < n; ++k, at += 4u) {
+        const float u0 = fmaf(float(k), a00, b0), u1 = fmaf(float(k), a10, b1);
+        add_pixel(a, t, acc_base, at, fmaf(u0, u0, u1 * u1), peak);
     }
 }
 
@@ -118,49 +262,130 @@ __device__ __forceinline__ void rec_box(const Rec& r, const TileInfo& ti, int& p
     y1 = min(pyc + ry, ti.H - 1);
 }
 
-// Forward deposit of one photon over its band (see Band): one flattened loop over
-// rows x bw pixels, so the trip count depends only on the band's area (photons of a warp
-// share an area class), the row changing every bw steps. Pixels outside the reference's
-// clipped box are masked off (their add is predicated away). False: the photon has no band.
-__device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, int sw,
-                                             uint32_t acc_base) {
-    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
+// Forward deposit of one photon straight into the image, in float: the photons that the counts
+// cannot hold (see kCountLimit). Rare, and out of line.
+__device__ __noinline__ void deposit_direct(const TileArgs& a, const TileState* tp, const Rec* rp) {
+    const Rec r = *rp;
+    const TileInfo ti = tp->ti;
+    if (!ti.in_image) return;
     int pxc, pyc, x0, x1, y0, y1;
     rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+    const bool all = rec_flags(r.packed) & kFlagEllipseAll;
+    const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, all);
+    const float e3 = r.e * kThreeOverPi;
+    int ky0 = y0 - pyc, ky1 = y1 - pyc;
+    support_rows(sup, r.dy0, ti.isy, ky0, ky1);
+    for (int ky = ky0; ky <= ky1; ++ky) {
+        const float dy = fmaf(float(ky), ti.sy, r.dy0);
+        int kx0 = x0 - pxc, kx1 = x1 - pxc;
+        if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
+        float* row = a.out + ti.img_off + int64_t(pyc + ky) * ti.W + pxc;
+        for (int kx = kx0; kx <= kx1; ++kx) {
+            if (!all && !ellipse_ok(kx, ky, img_wd(ti), img_hd(ti))) continue;
+            const float dx = fmaf(float(kx), ti.sx, r.dx0);
+            const float u0 = fmaf(r.m00, dx, r.m01 * dy), u1 = fmaf(r.m10, dx, r.m11 * dy);
+            const float s = fmaf(u0, u0, u1 * u1);
+            const float d = 1.f - s;
+            if (s < 1.f) atomicAdd(row + kx, (d * e3) * d);
+        }
+    }
+}
+
+// The band walks' rows, two pixels at a time. A row is w = min(bw rounded up to even, box
+// width) pixels wide and starts at the band's start clamped into [kxb0, kxb1 - w + 1]. A clamped
+// row still holds every pixel of its support that lies in the box (the support's pixels of row
+// ky are in [xs, xs + bw - 1]; clamping slides that window into the box without dropping any of
+// them, and when w is the box width the row is the whole box row), so no pixel needs an in-box
+// test. When w is odd, the second pixel of each row's last pair lies just outside the box and
+// is masked: the remaining-pair count there is tail.
+//
+// Row starts are formed without conversions: round-to-nearest of alpha - hw - 1/2 + beta ky, by
+// adding and taking off 1.5 * 2^23 (the sum's low mantissa bits are then the integer itself).
+// That is the floor, or one less where the band starts exactly on a pixel, which still covers
+// the row (bw = floor(2 hw) + 2).
+constexpr float kRoundMagic = 12582912.f;
+constexpr uint32_t kRoundMagicBits = 0x4B400000u;
+
+struct PairWalk {
+    int ky0, rows, npairs, tail;
+    float x0, beta, lo, hi;  // row start before rounding at ky = 0, its step, the clamp range
+};
+
+__device__ __forceinline__ PairWalk pair_walk(const Band& bd, int kxb0, int kxb1, int kyb0,
+                                              int kyb1) {
+    PairWalk p;
+    const int w = min((bd.bw + 1) & ~1, kxb1 - kxb0 + 1);
+    p.ky0 = max(bd.ky0, kyb0);
+    p.rows = min(bd.ky1, kyb1) - p.ky0 + 1;
+    p.npairs = (w + 1) >> 1;
+    p.tail = w & 1;
+    p.x0 = bd.alpha - bd.hw - 0.5f;
+    p.beta = bd.beta;
+    p.lo = float(kxb0);
+    p.hi = float(kxb1 - w + 1);
+    return p;
+}
+
+// Row start of row ky (kyf = float(ky)): kRoundMagic + the start column.
+__device__ __forceinline__ float pair_row(const PairWalk& p, float kyf) {
+    return fminf(fmaxf(fmaf(kyf, p.beta, p.x0), p.lo), p.hi) + kRoundMagic;
+}
+
+__device__ __forceinline__ float2 pair(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float hsum(float2 v) { return v.x + v.y; }
+
+// Forward deposit of one photon over its band (see Band): one flattened loop over the rows'
+// pixel pairs, so the trip count depends only on the band's area (photons of a warp share an
+// area class), the row changing every npairs steps. False: the photon has no band.
+//
+// Bound by instruction issue: the two pixels of a step are the two lanes of sm_100's packed FP32
+// instructions, and a row change, which some lane of the warp makes on nearly every step, is a
+// dozen instructions with no conversion in it.
+__device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, int sw, float peak,
+                                             uint32_t acc_base, uint32_t* wrapped) {
+    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
     const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
                               float(rec_rx(r.packed)) + 1.f);
     if (!bd.on) return false;
-    const int ky0 = max(bd.ky0, y0 - pyc), ky1 = min(bd.ky1, y1 - pyc);
-    if (ky0 > ky1) return true;
-    const int kxb0 = x0 - pxc;
-    const uint32_t kxspan = uint32_t(x1 - x0);
-    const float e3 = r.e * kThreeOverPi;
-    const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
-    const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
-    const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
-    const int bw = bd.bw;
-    const int total = (ky1 - ky0 + 1) * bw;
-    int ky = ky0, c = 0;
-    int xs = band_start(bd, ky);
-    float c0 = fmaf(float(ky), m01sy, c00), c1 = fmaf(float(ky), m11sy, c10);
-    uint32_t row = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc - ti.ox));
-    for (int q = 0; q < total; ++q) {
-        const int kx = xs + c;
-        const bool in = uint32_t(kx - kxb0) <= kxspan;
-        const float kf = float(kx);
-        const float u0 = fmaf(kf, a00, c0), u1 = fmaf(kf, a10, c1);
-        const float s = fmaf(u0, u0, u1 * u1);
-        const float t = 1.f - s;
-        red_shared_inside<0>(row + 4u * uint32_t(kx), in ? s : 2.f, (t * e3) * t);
-        if (++c == bw) {
-            c = 0;
-            ++ky;
-            xs = band_start(bd, ky);
-            c0 += m01sy;
-            c1 += m11sy;
-            row += 4u * uint32_t(sw);
-        }
+    int pxc, pyc, x0, x1, y0, y1;
+    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+    const PairWalk p = pair_walk(bd, x0 - pxc, x1 - pxc, y0 - pyc, y1 - pyc);
+    if (p.rows <= 0) return true;
+    const float2 A00 = pair(r.m00 * ti.sx), A10 = pair(r.m10 * ti.sx);
+    const float2 E3 = pair(peak);
+    const float2 M01 = pair(r.m01 * ti.sy), M11 = pair(r.m11 * ti.sy);
+    const float2 C0 = pair(fmaf(r.m00, r.dx0, r.m01 * r.dy0));
+    const float2 C1 = pair(fmaf(r.m10, r.dx0, r.m11 * r.dy0));
+    float2 KY = pair(float(p.ky0));
+    float m = pair_row(p, KY.x);
+    // (wrapping arithmetic: the magic number's bits come off again with each row's start)
+    uint32_t row = acc_base + 4u * (uint32_t((pyc + p.ky0 - ti.oy) * sw + (pxc - ti.ox)) -
+                                    kRoundMagicBits);
+    int rem = p.npairs;
+    uint32_t wraps = 0u;
+    for (int q = p.rows * p.npairs; q > 0; --q) {
+        const uint32_t at = row + 4u * __float_as_uint(m);
+        const float2 KF = make_float2(m - kRoundMagic, m - (kRoundMagic - 1.f));
+        const float2 U0 = __ffma2_rn(KF, A00, __ffma2_rn(KY, M01, C0));
+        const float2 U1 = __ffma2_rn(KF, A10, __ffma2_rn(KY, M11, C1));
+        const float2 S = __ffma2_rn(U0, U0, __fmul2_rn(U1, U1));
+        // 1 - s, or 0 outside the support and at the pixel after an odd row
+        const float2 D = __ffma2_rn(S, pair(-1.f), pair(1.f));
+        const float2 T = make_float2(fmaxf(D.x, 0.f), rem == p.tail ? 0.f : fmaxf(D.y, 0.f));
+        const float2 V = __fmul2_rn(__fmul2_rn(T, E3), T);
+        add_pair(at, __float2uint_rn(V.x), __float2uint_rn(V.y), wraps);
+        // the next pair: two columns on, or the next row's start (selected, not branched to:
+        // some lane changes rows on nearly every step)
+        const bool wrap = --rem == 0;
+        const float2 KY1 = __fadd2_rn(KY, pair(1.f));
+        const float m1 = pair_row(p, KY1.x);
+        m = wrap ? m1 : m + 2.f;
+        KY.x = wrap ? KY1.x : KY.x;
+        KY.y = wrap ? KY1.y : KY.y;
+        row += wrap ? 4u * uint32_t(sw) : 0u;
+        rem = wrap ? p.npairs : rem;
     }
+    if (wraps) *wrapped = 1u;
     return true;
 }
 
@@ -170,53 +395,38 @@ __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, i
 // image-half-size ellipse test somewhere in their box (tiny images only) take the per-pixel test
 // path. Out of line: with the band walk on, hardly any photon comes here, and inlined its
 // registers were spilled around every photon's band walk.
-__device__ __noinline__ void deposit_generic(const Rec* rp, TileInfo ti, int sw, bool spans,
-                                             float* acc) {
+__device__ __noinline__ void deposit_generic(const TileArgs& a, const TileState* tp, const Rec* rp,
+                                             float peak, uint32_t acc_base) {
     const Rec r = *rp;
-    const uint32_t p = r.packed;
-    const int pxc = ti.ox + rec_lx(p), pyc = ti.oy + rec_ly(p);
-    const int rx = rec_rx(p), ry = rec_ry(p);
-    const int x0 = max(pxc - rx, 0), x1 = min(pxc + rx, ti.W - 1);
-    const int y0 = max(pyc - ry, 0), y1 = min(pyc + ry, ti.H - 1);
-    const float e3 = r.e * kThreeOverPi;
-    const bool all = rec_flags(p) & kFlagEllipseAll;
-    const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, spans && all);
+    const TileState& t = *tp;
+    const TileInfo ti = t.ti;
+    const int sw = a.cfg.sw;
+    int pxc, pyc, x0, x1, y0, y1;
+    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
+    const bool all = rec_flags(r.packed) & kFlagEllipseAll;
+    const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, (a.cfg.spans || a.cfg.band) && all);
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
     const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
     // u at the centre pixel's corner: M (dx0, dy0)
     const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
-    const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
     int ky0 = y0 - pyc, ky1 = y1 - pyc;
     support_rows(sup, r.dy0, ti.isy, ky0, ky1);
-    if (all) {
-        // Each lane starts its row walk at a different row: co-located photons in one warp
-        // (focused caustics) then add into different rows at the same time instead of
-        // serialising on one shared address.
-        const int nrows = ky1 - ky0 + 1;
-        int ky = nrows > 0 ? ky0 + int(threadIdx.x & 31) % nrows : ky0;
-        for (int j = 0; j < nrows; ++j, ky = (ky == ky1) ? ky0 : ky + 1) {
-            const float dy = fmaf(float(ky), ti.sy, r.dy0);
-            int kx0 = x0 - pxc, kx1 = x1 - pxc;
-            if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
+    for (int ky = ky0; ky <= ky1; ++ky) {
+        const float dy = fmaf(float(ky), ti.sy, r.dy0);
+        int kx0 = x0 - pxc, kx1 = x1 - pxc;
+        if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
+        const uint32_t at = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc + kx0 - ti.ox));
+        if (all) {
             const float kf = float(kx0);
-            const float b0 = fmaf(kf, a00, fmaf(float(ky), m01sy, c00));
-            const float b1 = fmaf(kf, a10, fmaf(float(ky), m11sy, c10));
-            const uint32_t a = acc_base +
-                               4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc + kx0 - ti.ox));
-            fwd_row(kx1 - kx0 + 1, a, b0, b1, a00, a10, e3);
-        }
-    } else {
-        for (int ky = ky0; ky <= ky1; ++ky) {
-            const float dy = fmaf(float(ky), ti.sy, r.dy0);
+            fwd_row(a, t, acc_base, kx1 - kx0 + 1, at, fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
+                    fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak);
+        } else {
             const float c0 = fmaf(r.m00, r.dx0, r.m01 * dy);
             const float c1 = fmaf(r.m10, r.dx0, r.m11 * dy);
-            const uint32_t arow = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc - ti.ox));
-            for (int kx = x0 - pxc; kx <= x1 - pxc; ++kx) {
+            for (int kx = kx0; kx <= kx1; ++kx) {
                 if (!ellipse_ok(kx, ky, img_wd(ti), img_hd(ti))) continue;
                 const float u0 = fmaf(float(kx), a00, c0), u1 = fmaf(float(kx), a10, c1);
-                const float s = fmaf(u0, u0, u1 * u1);
-                const float t = 1.f - s;
-                red_shared_inside<0>(arow + 4u * uint32_t(kx), s, (t * e3) * t);
+                add_pixel(a, t, acc_base, at + 4u * uint32_t(kx - kx0), fmaf(u0, u0, u1 * u1), peak);
             }
         }
     }
@@ -283,16 +493,6 @@ __device__ __forceinline__ int row_begin(const RowGeo& g, int ky, float& s, floa
     return xs;
 }
 
-// Shared add of v at shared byte address a + OFF when c < w and s < 1, as one predicated
-// reduction.
-template <int OFF>
-__device__ __forceinline__ void red_row(uint32_t a, float s, float v, int c, int w) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.lt.s32 q, %3, %4;\n\t"
-        "setp.lt.and.f32 q, %1, 0f3F800000, q;\n\t@q red.shared.add.f32 [%0+%5], %2;\n\t}"
-        :: "r"(a), "f"(s), "f"(v), "r"(c), "r"(w), "n"(OFF) : "memory");
-}
-
 // Shared load of the float at shared byte address a when c < w, else 0.
 __device__ __forceinline__ float lds_row(uint32_t a, int c, int w) {
     float v;
@@ -304,39 +504,23 @@ __device__ __forceinline__ float lds_row(uint32_t a, int c, int w) {
 }
 
 // Forward deposit of the warp's photons by padded rows. rows = 0 for lanes with nothing to
-// walk (their g is not read). Lanes start at rotated rows (lane mod rows), so co-located
-// photons of a caustic add into different rows, and so different banks, at the same time.
-// Every lane of the warp calls it.
-__device__ __forceinline__ void deposit_rows(const RowGeo& g, int rows, float e3, uint32_t acc_base,
-                                             int sw) {
+// walk (their g is not read). Every lane of the warp calls it.
+__device__ __forceinline__ void deposit_rows(const TileArgs& a, const TileState& t, const RowGeo& g,
+                                             int rows, float peak, uint32_t acc_base) {
     const int rm = __reduce_max_sync(0xFFFFFFFFu, rows);
     if (rm == 0) return;
     const int wm = __reduce_max_sync(0xFFFFFFFFu, rows > 0 ? g.w : 0);
-    const int rot = rows > 1 ? int(threadIdx.x & 31) % rows : 0;
     const float dd = 2.f * g.A;
     for (int j = 0; j < rm; ++j) {
         const int wl = j < rows ? g.w : 0;
-        int jj = j + rot;
-        jj = jj >= rows ? jj - rows : jj;
-        const int ky = g.ky0 + jj;
+        const int ky = g.ky0 + j;
         float s, d;
         const int xs = row_begin(g, ky, s, d);
-        uint32_t a = acc_base + 4u * uint32_t(g.off + ky * sw + xs);
-        int c = 0;
-        for (; c + 2 <= wm; c += 2) {
-            const float t = 1.f - s;
-            red_row<0>(a, s, (t * e3) * t, c, wl);
+        uint32_t at = acc_base + 4u * uint32_t(g.off + ky * a.cfg.sw + xs);
+        for (int c = 0; c < wm; ++c, at += 4u) {
+            add_pixel(a, t, acc_base, at, s, peak, c < wl);
             s += d;
             d += dd;
-            const float t2 = 1.f - s;
-            red_row<4>(a, s, (t2 * e3) * t2, c + 1, wl);
-            s += d;
-            d += dd;
-            a += 8u;
-        }
-        if (c < wm) {
-            const float t = 1.f - s;
-            red_row<0>(a, s, (t * e3) * t, c, wl);
         }
     }
 }
@@ -448,90 +632,34 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 // Forward deposit of one photon by the whole warp (see use_coop).
-__device__ __noinline__ void deposit_coop(const Rec* rp, TileInfo ti, int sw, uint32_t acc_base,
-                                          int lane) {
+__device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp, const Rec* rp,
+                                          uint32_t acc_base) {
     const Rec r = *rp;
+    const TileState& t = *tp;
+    const TileInfo ti = t.ti;
+    const float peak = count_peak(t, r.e);
+    if (!(peak > 0.f)) {
+        if ((threadIdx.x & 31) == 0) deposit_direct(a, tp, rp);
+        return;
+    }
     int pxc, pyc, x0, x1, y0, y1;
     rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
-    const float e3 = r.e * kThreeOverPi;
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
     const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
     const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
     const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, true);
     int ky0 = y0 - pyc, ky1 = y1 - pyc;
     support_rows(sup, r.dy0, ti.isy, ky0, ky1);
-    for (int ky = ky0 + lane; ky <= ky1; ky += 32) {
+    for (int ky = ky0 + int(threadIdx.x & 31); ky <= ky1; ky += 32) {
         const float dy = fmaf(float(ky), ti.sy, r.dy0);
         int kx0 = x0 - pxc, kx1 = x1 - pxc;
         if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
         const float kf = float(kx0);
-        const float b0 = fmaf(kf, a00, fmaf(float(ky), m01sy, c00));
-        const float b1 = fmaf(kf, a10, fmaf(float(ky), m11sy, c10));
-        const uint32_t a = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc + kx0 - ti.ox));
-        fwd_row(kx1 - kx0 + 1, a, b0, b1, a00, a10, e3);
+        fwd_row(a, t, acc_base, kx1 - kx0 + 1,
+                acc_base + 4u * uint32_t((pyc + ky - ti.oy) * a.cfg.sw + (pxc + kx0 - ti.ox)),
+                fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
+                fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak);
     }
-}
-
-// A run of sorted positions [begin, end) holding one screen tile's photons (positions and tiles
-// fit in 31 bits: the entry points reject larger calls).
-struct Segment {
-    int tile;
-    uint32_t begin, end;
-};
-
-// End of tile t's photons: the start of its successor's first bucket.
-__device__ __forceinline__ uint32_t tile_end(const TileArgs& a, int t) {
-    return __ldg(a.start + ((int64_t(t) + 1) << a.cfg.class_bits));
-}
-
-__device__ __forceinline__ Segment first_segment(const TileArgs& a, uint32_t chunk, uint32_t p0) {
-    Segment s;
-    // (clamped, like the counters, so that a workspace without a plan stays in its arrays)
-    s.tile = int(min(int64_t(__ldg(a.chunk_tile + chunk)), a.n_tiles - 1));
-    s.begin = p0;
-    s.end = tile_end(a, s.tile);
-    return s;
-}
-
-// The segment after sg (sg.end below the tile path's photon count): the first tile after
-// sg.tile whose range is not empty, found by doubling steps then bisection (empty tiles are
-// usually few, so one probe mostly suffices).
-__device__ __forceinline__ Segment next_segment(const TileArgs& a, const Segment& sg) {
-    const uint32_t p = sg.end;
-    const int t = sg.tile, last = int(a.n_tiles) - 1;
-    int k = 1;
-    while (k < last - t && tile_end(a, t + k) <= p) k <<= 1;
-    int lo = t + (k >> 1) + 1, hi = k < last - t ? t + k : last;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (tile_end(a, mid) > p) hi = mid; else lo = mid + 1;
-    }
-    Segment s;
-    s.tile = lo;
-    s.begin = p;
-    s.end = tile_end(a, lo);
-    return s;
-}
-
-// The current segment and its tile, held in shared memory: one thread finds and decodes the next
-// one while the others flush the last (two slots), and the photon loops read the fields they
-// need instead of keeping them all in registers across a walk.
-struct TileState {
-    Segment sg;
-    TileInfo ti;
-    int x0, x1, y0, y1;  // pixels its photons can touch: the tile and the plan's largest radius
-                         // around it, inside the image
-};
-
-__device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, TileState* t) {
-    t->sg = sg;
-    const TileInfo ti = decode_tile(a.sims, uint32_t(sg.tile), a.cfg, a.image_elems);
-    t->ti = ti;
-    const int m = a.cfg.apron - int(min(__ldg(a.tile_r + sg.tile), uint32_t(a.cfg.apron)));
-    t->x0 = max(ti.ox + m, 0);
-    t->y0 = max(ti.oy + m, 0);
-    t->x1 = min(ti.ox + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.W - 1);
-    t->y1 = min(ti.oy + a.cfg.tile + 2 * a.cfg.apron - 1 - m, ti.H - 1);
 }
 
 // Next chunk of sorted photons for this CTA: a shared work counter (zero when the kernel starts)
@@ -628,7 +756,8 @@ __device__ __noinline__ void tail_forward(const TileArgs& a) {
 // clears them: warps take rows, lanes take consecutive columns. When image rows are 16-byte
 // aligned the adds are 4-wide vector reductions (red.global.add.v4.f32) over 4-aligned column
 // groups; columns of a group outside the range add zero. All-zero groups are skipped.
-__device__ __forceinline__ void flush_rows(float* acc, int sw, const TileState& t, float* out) {
+__device__ __forceinline__ void flush_rows(uint32_t* acc, int sw, const TileState& t, float* out) {
+    const float unit = t.unit;
     const int x0 = t.x0, x1 = t.x1, y1 = t.y1;
     const int ox = t.ti.ox, oy = t.ti.oy, W = t.ti.W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -638,13 +767,13 @@ __device__ __forceinline__ void flush_rows(float* acc, int sw, const TileState& 
     if (!t.ti.in_image) {
         // a plane outside the caller's buffer (an inconsistent simulation table): clear only
         for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
-            float* arow = acc + (gy - oy) * sw - ox;
-            for (int gx = x0 + lane; gx <= x1; gx += 32) arow[gx] = 0.f;
+            uint32_t* arow = acc + (gy - oy) * sw - ox;
+            for (int gx = x0 + lane; gx <= x1; gx += 32) arow[gx] = 0u;
         }
     } else if (vec) {
         const int g0 = x0 >> 2, g1 = x1 >> 2;
         for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
-            float* arow = acc + (gy - oy) * sw - ox;
+            uint32_t* arow = acc + (gy - oy) * sw - ox;
             float* grow = img + int64_t(gy) * W;
             for (int g = g0 + lane; g <= g1; g += 32) {
                 const int gx = g << 2;
@@ -654,8 +783,8 @@ __device__ __forceinline__ void flush_rows(float* acc, int sw, const TileState& 
                     const int c = gx + j;
                     v[j] = 0.f;
                     if (c >= x0 && c <= x1) {
-                        v[j] = arow[c];
-                        arow[c] = 0.f;
+                        v[j] = float(arow[c]) * unit;
+                        arow[c] = 0u;
                     }
                 }
                 if (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f)
@@ -665,26 +794,57 @@ __device__ __forceinline__ void flush_rows(float* acc, int sw, const TileState& 
         }
     } else {
         for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
-            float* arow = acc + (gy - oy) * sw - ox;
+            uint32_t* arow = acc + (gy - oy) * sw - ox;
             float* grow = img + int64_t(gy) * W;
             for (int gx = x0 + lane; gx <= x1; gx += 32) {
-                const float v = arow[gx];
-                if (v != 0.f) {
-                    atomicAdd(grow + gx, v);
-                    arow[gx] = 0.f;
+                const uint32_t v = arow[gx];
+                if (v != 0u) {
+                    atomicAdd(grow + gx, float(v) * unit);
+                    arow[gx] = 0u;
                 }
             }
         }
     }
 }
 
-// Ends a segment of the forward (all threads call it): the accumulator's pixels into the image;
-// with more, one thread of the last warp (which has the fewest rows) finds the next segment
-// meanwhile. Returns the slot of the tile state to use from here on.
-__device__ __forceinline__ int end_segment(const TileArgs& a, float* acc, int sw, TileState* ts,
-                                           int cur, bool more) {
+// Starts a segment of the forward whose photons below p1 are to be splatted (a whole warp calls
+// it).
+__device__ __forceinline__ void start_segment(const TileArgs& a, const Segment& sg, uint32_t p1,
+                                              TileState* t) {
+    if ((threadIdx.x & 31) == 0) set_tile(a, sg, t);
+    __syncwarp();
+    set_scale(a, sg.begin, min(sg.end, p1), t);
+}
+
+// Sums the segment's photons [begin, end) again where a pixel's count has wrapped: from zero, by
+// the walk whose adds carry a wrap on (the photons that went to the image directly stay there).
+// All threads call it, between barriers.
+__device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, const TileState* t,
+                                          uint32_t begin, uint32_t end) {
+    const int sw = a.cfg.sw;
+    for (int k = threadIdx.x; k < sw * sw; k += blockDim.x) acc[k] = 0u;
     __syncthreads();
-    if (more && threadIdx.x == blockDim.x - 1) set_tile(a, next_segment(a, ts[cur].sg), ts + (cur ^ 1));
+    const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
+    for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
+        const float peak = count_peak(*t, a.srecs[i].e);
+        if (!(rec_flags(a.srecs[i].packed) & kFlagFwdSkip) && peak > 0.f)
+            deposit_generic(a, t, a.srecs + i, peak, acc_base);
+    }
+    __syncthreads();
+}
+
+// Ends a segment of the forward (all threads call it): the accumulator's pixels into the image;
+// where photons below p1 are left, the last warp (which has the fewest rows) meanwhile starts
+// the next segment. p0: the work chunk's first photon. Returns the slot of the tile state to use
+// from here on.
+__device__ __forceinline__ int end_segment(const TileArgs& a, uint32_t* acc, int sw, TileState* ts,
+                                           int cur, uint32_t p0, uint32_t p1) {
+    __syncthreads();
+    const Segment sg = ts[cur].sg;
+    if (ts[cur].wrapped) redo_segment(a, acc, ts + cur, max(sg.begin, p0), min(sg.end, p1));
+    const bool more = sg.end < p1;
+    if (more && threadIdx.x >= blockDim.x - 32)
+        start_segment(a, next_segment(a, sg), p1, ts + (cur ^ 1));
     flush_rows(acc, sw, ts[cur], a.out);
     __syncthreads();
     return more ? cur ^ 1 : cur;
@@ -692,12 +852,12 @@ __device__ __forceinline__ int end_segment(const TileArgs& a, float* acc, int sw
 
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_constant__ TileArgs a) {
-    extern __shared__ float acc[];
+    extern __shared__ uint32_t acc[];
     __shared__ TileState ts[2];
     __shared__ uint32_t chunk_slot;
     const int sw = a.cfg.sw;
     Rec* stage = reinterpret_cast<Rec*>(acc + stage_offset_floats(sw));
-    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0.f;
+    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0u;
     const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
     const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
     const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
@@ -707,7 +867,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
         if (p0 + threadIdx.x < p1)
             stage_rec_async(stage + threadIdx.x, a.srecs + p0 + threadIdx.x);
         cp_async_commit();
-        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), ts);
+        if (threadIdx.x < 32) start_segment(a, first_segment(a, c, p0), p1, ts);
         __syncthreads();
         int cur = 0, buf = 0;
         for (uint32_t base = p0; base < p1; base += NT, buf ^= 1) {
@@ -725,21 +885,28 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
                 if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
                     const Rec r = *slot;
                     coop = use_coop(r, a.cfg.coop_r);
-                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip) &&
-                        !(a.cfg.band && deposit_band(r, t.ti, sw, acc_base)))
-                        deposit_generic(slot, t.ti, sw, a.cfg.spans, acc);
+                    const float peak = count_peak(t, r.e);
+                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
+                        if (!(peak > 0.f))
+                            deposit_direct(a, &t, slot);
+                        else if (!(a.cfg.band && deposit_band(r, t.ti, sw, peak, acc_base,
+                                                              &ts[cur].wrapped)))
+                            deposit_generic(a, &t, slot, peak, acc_base);
+                    }
                 }
+                // lanes wait for their warp's longest walk here: without it they would run on into
+                // the next batch a few at a time
+                __syncwarp();
                 if (a.cfg.coop_r > 0) {
-                    __syncwarp();
                     for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
-                        deposit_coop(stage + buf * NT + (threadIdx.x & ~31u) + (__ffs(cm) - 1),
-                                     t.ti, sw, acc_base, threadIdx.x & 31);
+                        deposit_coop(a, &t, stage + buf * NT + (threadIdx.x & ~31u) + (__ffs(cm) - 1),
+                                     acc_base);
                 }
                 if (t.sg.end >= min(base + NT, p1)) break;
-                cur = end_segment(a, acc, sw, ts, cur, true);
+                cur = end_segment(a, acc, sw, ts, cur, p0, p1);
             }
         }
-        end_segment(a, acc, sw, ts, cur, false);
+        end_segment(a, acc, sw, ts, cur, p0, p1);
     }
     finish_queue(a.queue);
     tail_forward(a);
@@ -879,9 +1046,6 @@ __device__ __forceinline__ int band_row_start(const Band& bd, const BandWalk& bw
 struct BandMoments {
     float sE, A0t, B1t, B2, Sy, Sxy, Syy;
 };
-
-__device__ __forceinline__ float2 pair(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float hsum(float2 v) { return v.x + v.y; }
 
 __device__ __forceinline__ BandMoments gather_band_rows(const Band& bd, const BandWalk& bw,
                                                         int ky, int ky1, const float* row,
@@ -1159,6 +1323,7 @@ __global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_consta
                     if (!coop && !(a.cfg.band && gather_band(r, t.ti, sw, tg, i, a.stage)))
                         gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
                 }
+                __syncwarp();  // as in fwd_tiles_kernel
                 if (a.cfg.coop_r > 0) {
                     for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
                         const int src = __ffs(cm) - 1;
@@ -1182,18 +1347,18 @@ __global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_consta
 
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constant__ TileArgs a) {
-    extern __shared__ float acc[];
+    extern __shared__ uint32_t acc[];
     __shared__ TileState ts[2];
     __shared__ uint32_t chunk_slot;
     const int sw = a.cfg.sw;
-    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0.f;
+    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0u;
     const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
     const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
     const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
     for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
          c = next_chunk(a.queue, &chunk_slot)) {
         const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
-        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), ts);
+        if (threadIdx.x < 32) start_segment(a, first_segment(a, c, p0), p1, ts);
         __syncthreads();
         int cur = 0;
         for (uint32_t base = p0; base < p1; base += NT) {
@@ -1202,7 +1367,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
                 const TileState& t = ts[cur];
                 RowGeo g;
                 int rows = 0;
-                float e3 = 0.f;
+                float peak = 0.f;
                 bool generic = false, coop = false;
                 if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
                     const Rec r = a.srecs[i];
@@ -1210,21 +1375,25 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
                     if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
                         int pxc, pyc, x0, x1, y0, y1;
                         rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
+                        peak = count_peak(t, r.e);
                         generic = !prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
-                        rows = generic ? 0 : g.rows;
-                        e3 = r.e * kThreeOverPi;
+                        rows = generic || !(peak > 0.f) ? 0 : g.rows;
+                        if (!(peak > 0.f)) {
+                            generic = false;
+                            deposit_direct(a, &t, a.srecs + i);
+                        }
                     }
                 }
-                deposit_rows(g, rows, e3, acc_base, sw);
-                if (generic) deposit_generic(a.srecs + i, t.ti, sw, a.cfg.spans, acc);
+                deposit_rows(a, t, g, rows, peak, acc_base);
+                if (generic) deposit_generic(a, &t, a.srecs + i, peak, acc_base);
                 for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
-                    deposit_coop(a.srecs + (base + (threadIdx.x & ~31u) + (__ffs(cm) - 1)), t.ti,
-                                 sw, acc_base, threadIdx.x & 31);
+                    deposit_coop(a, &t, a.srecs + (base + (threadIdx.x & ~31u) + (__ffs(cm) - 1)),
+                                 acc_base);
                 if (t.sg.end >= min(base + NT, p1)) break;
-                cur = end_segment(a, acc, sw, ts, cur, true);
+                cur = end_segment(a, acc, sw, ts, cur, p0, p1);
             }
         }
-        end_segment(a, acc, sw, ts, cur, false);
+        end_segment(a, acc, sw, ts, cur, p0, p1);
     }
     finish_queue(a.queue);
     tail_forward(a);
