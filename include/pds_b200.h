@@ -46,13 +46,14 @@ extern "C" {
 /* Kernel tuning. A NULL pointer or a zero field selects the default. */
 typedef struct pds_config {
     int32_t tile;       /* screen-tile edge in pixels: 16, 32 or 64 (default 64) */
-    int32_t chunk;      /* sorted photons per CTA work item, multiple of 256 (default 2048;
-                           lowered, to no less than 256, when the call has too few photons to
-                           give every resident tile CTA about four work items) */
+    int32_t chunk;      /* sorted photons per CTA work item, multiple of 256 (default 2048, up to
+                           8192 for calls whose photons still make 48 work items an SM; either
+                           is lowered, to no less than 256, when the call has too few photons
+                           to give every resident tile CTA about four work items) */
     int32_t class_bits; /* footprint-size bits appended to the sort key (photons of a tile
                            are then grouped by footprint size; with the band walk, classes
-                           of 1/k octave of the band's area, k = 1 up to 3 bits, 2 for 4,
-                           3 for 5; 6: the row walk's classes, 3 bits of band rows and 3
+                           of 1/k octave of the band walk's pixels, k = 1 up to 3 bits, 2
+                           for 4, 3 for 5; 6: the row walk's classes, 3 bits of band rows and 3
                            of row width inside the box): 1..6, or -1 for none (default 5) */
     int32_t apron_max;  /* largest footprint radius (px) the tile path holds (default 32);
                            larger footprints take the direct path */
@@ -64,9 +65,7 @@ typedef struct pds_config {
                            (2, 3 and 4 give the same result: pixels outside the support add
                            exactly zero); default 3 */
     int32_t min_blocks; /* resident CTAs per SM the tile kernels are compiled for: 2, 3 or 4
-                           (fewer: more registers per thread; more: more warps); a value sets
-                           both directions; default (0): 3 for the forward, whose CTAs also
-                           stage their next records in shared memory, and 4 for the backward */
+                           (fewer: more registers per thread; more: more warps); default 3 */
     int32_t coop_radius; /* footprints with a radius (px) of at least this are splatted by a
                            whole warp instead of one thread; -1 never; default -1 */
 } pds_config;

@@ -71,14 +71,19 @@ int resolve_cfg(const pds_config* in, pds_config& out) {
     return PDS_OK;
 }
 
-// Photons per tile-kernel work chunk: the configured chunk, lowered for small photon counts
-// so that every resident CTA of the tile kernels (3 per SM) gets about four chunks; at least
-// 256 photons (one CTA-wide batch).
-int32_t effective_chunk(int32_t chunk, int64_t n) {
-    const int sms = pds::num_sms();
-    const int64_t target = (n + int64_t(sms) * 12 - 1) / (int64_t(sms) * 12);
-    const int64_t c = (target + 255) / 256 * 256;
-    return int32_t(c < 256 ? 256 : (c < chunk ? c : chunk));
+// Photons per tile-kernel work chunk: the configured chunk (2048 by default), lowered for small
+// photon counts so that every resident CTA of the tile kernels (3 per SM) gets about four
+// chunks; at least 256 photons (one CTA-wide batch). Where none is configured it grows with the
+// photon count, up to 8192, while 48 chunks an SM are left: a chunk ends with its tile's pixels
+// added to the image or the next tile's staged, 6% of the forward at 2048 photons.
+int32_t effective_chunk(const pds_config* in, int32_t chunk, int64_t n) {
+    const int64_t sms = pds::num_sms();
+    const auto share = [&](int64_t per_sm) {
+        const int64_t target = (n + sms * per_sm - 1) / (sms * per_sm);
+        return (target + 255) / 256 * 256;
+    };
+    if (!(in && in->chunk)) chunk = int32_t(std::clamp<int64_t>(share(48), chunk, 8192));
+    return int32_t(std::clamp<int64_t>(share(12), 256, chunk));
 }
 
 int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resolved& r) {
@@ -91,7 +96,7 @@ int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resol
     if (inv >= (uint64_t(1) << 32))
         return fail(PDS_ERR_UNSUPPORTED, "sort key space exceeds 32 bits; lower class_bits");
     r.cfg.tile = c.tile;
-    r.cfg.chunk = effective_chunk(c.chunk, n);
+    r.cfg.chunk = effective_chunk(in, c.chunk, n);
     r.cfg.class_bits = c.class_bits;
     r.cfg.apron = mpr < 0 ? 0 : (mpr < c.apron_max ? mpr : c.apron_max);
     // odd pitch: the rows of one column of the accumulator fall in different banks
@@ -100,10 +105,7 @@ int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resol
     r.cfg.spans = (c.walk == 2 || c.walk == 4) ? 1 : 0;
     r.cfg.band = c.walk == 3 ? 1 : 0;
     r.cfg.rows = c.walk == 4 ? 1 : 0;
-    // default: the forward at 3 CTAs an SM (room for its record staging buffers), the
-    // backward at 4 (measured best for each); an explicit min_blocks sets both
     r.cfg.min_blocks = c.min_blocks;
-    r.cfg.min_blocks_bwd = (in && in->min_blocks) ? c.min_blocks : 4;
     r.cfg.coop_r = c.coop_radius > 0 ? c.coop_radius : 0;
     r.n_buckets = n_tiles << c.class_bits;
     r.key_big = uint32_t(r.n_buckets);

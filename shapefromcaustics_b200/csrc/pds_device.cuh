@@ -73,8 +73,7 @@ struct Cfg {
     int32_t spans;       // 1: walk only the support's rows / row spans; 0: the whole box
     int32_t band;        // 1: walk each footprint's sheared band (see Band)
     int32_t rows;        // 1: walk the bands' rows padded to a common count and width per warp
-    int32_t min_blocks;  // resident CTAs per SM the forward tile kernels' register budget targets
-    int32_t min_blocks_bwd;  // the same for the backward tile kernels
+    int32_t min_blocks;  // resident CTAs per SM the tile kernels' register budget targets
     int32_t coop_r;      // footprint radius from which a photon is splatted by a whole warp
 };
 
@@ -230,7 +229,8 @@ __device__ __forceinline__ bool support_cols(const Support& g, float dy, float d
 // bw = floor(2 hw) + 2. The band is ~4/pi of the support's area (plus a column), where the
 // reference's box can be 40 times it for thin rotated footprints. Pixels whose float s is
 // below 1 only by rounding at the support's edge may fall outside; they add (1 - s)^2 ~ 0.
-// Degenerate, near-singular or non-finite M: on = false (walk the box).
+// Degenerate, near-singular or non-finite M: on = false (walk the box). The padded-row walk
+// takes its rows from here; the default walk forms the same band in pixel units (PairWalk).
 struct Band {
     bool on;
     int ky0, ky1;  // support rows
@@ -269,6 +269,39 @@ __device__ __forceinline__ Band make_band(float m00, float m01, float m10, float
 
 __device__ __forceinline__ int band_start(const Band& b, int ky) {
     return __float2int_rd(fmaf(float(ky), b.beta, b.alpha - b.hw));
+}
+
+// The band walks take rows two pixels at a time: pairs of a row of half-width hw, floor(hw + 1)
+// (the nearest integer to hw + 1/2, from the low mantissa bits of its sum with 1.5 * 2^23).
+constexpr float kRoundMagic = 12582912.f;
+constexpr uint32_t kRoundMagicBits = 0x4B400000u;
+
+__device__ __forceinline__ int band_pairs(float hw) {
+    return __float_as_int((hw + 0.5f) + kRoundMagic) - int(kRoundMagicBits);
+}
+
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Steps of a photon's band walk inside its box (unclipped): what its footprint class is made of.
+// M in pixel units (columns times 2 / W, 2 / H), dyp = dy0 in pixels.
+__device__ __forceinline__ int band_steps(float m00, float m01, float m10, float m11, float dyp,
+                                          int rx, int ry) {
+    const float A = fmaf(m00, m00, m10 * m10);
+    const float det = fmaf(m00, m11, -m01 * m10);
+    const float hw = rsqrt_fast(A);
+    const float ey = A * hw * rcp_fast(fabsf(det));
+    if (!(A > 0.f && A < 1e30f && hw <= float(rx) + 1.f && ey < 1e6f)) return (2 * rx + 1) * (ry + 1);
+    const int rows = min(__float2int_rd(ey - dyp), ry) - max(__float2int_ru(-ey - dyp), -ry) + 1;
+    return min(band_pairs(hw), rx + 1) * max(rows, 1);
 }
 
 // The rows a photon's band walk visits inside its clipped box [kxb0, kxb1] x [kyb0, kyb1]

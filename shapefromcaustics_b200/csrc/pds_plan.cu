@@ -119,15 +119,13 @@ __device__ __forceinline__ uint32_t bin_photon(const PlanArgs& a, const pds_sim&
                                              x0 - f.px_c, x1 - f.px_c, y0 - f.py_c, y1 - f.py_c)
                             : cls_max;
     } else if (a.cfg.band) {
-        // photons of a warp then have similar band areas (trip counts): classes of 1/k octave
-        // of the area, k = 1, 2, 3 for up to 3, 4 and 5 class bits
-        const float dx0 = corner_offset_step(f.px_c, s2w, x);
-        const float sy = float(s2h);  // 2 / H, the division done once per simulation
-        const Band bd = make_band(m00, m01, m10, m11, dx0, dy0, sy, 0.5f * float(sim.width),
-                                  0.5f * float(sim.height), float(f.rx) + 1.f);
+        // photons of a warp then have similar trip counts of the band walk: classes of 1/k octave
+        // of its pixels, k = 1, 2, 3 for up to 3, 4 and 5 class bits
+        const float sx = float(s2w), sy = float(s2h);  // 2 / W, 2 / H
         int area = (2 * f.rx + 1) * (2 * f.ry + 1);
-        if (bd.on && f.ellipse_all)
-            area = min(area, (min(bd.ky1, f.ry) - max(bd.ky0, -f.ry) + 1) * bd.bw);
+        if (f.ellipse_all)
+            area = 2 * band_steps(m00 * sx, m01 * sy, m10 * sx, m11 * sy,
+                                  dy0 * (0.5f * float(sim.height)), f.rx, f.ry);
         // floor(k log2 area) = floor(log2 area^k), exactly
         const int k = cb <= 3 ? 1 : cb - 2;
         const uint64_t a1 = uint64_t(max(area, 1));

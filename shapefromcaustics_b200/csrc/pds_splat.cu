@@ -130,10 +130,12 @@ struct TileState {
     float scale, unit;   // forward: accumulator counts per unit of energy density (a power of
                          // two) and its inverse; scale 0: no photon is accumulated
     uint32_t wrapped;    // forward: non-zero where a pixel's count has wrapped
+    uint32_t groups;     // groups of 32 photons that warps have taken
 };
 
 __device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, TileState* t) {
     t->sg = sg;
+    t->groups = 0u;
     const TileInfo ti = decode_tile(a.sims, uint32_t(sg.tile), a.cfg, a.image_elems);
     t->ti = ti;
     const int m = a.cfg.apron - int(min(__ldg(a.tile_r + sg.tile), uint32_t(a.cfg.apron)));
@@ -291,98 +293,132 @@ __device__ __noinline__ void deposit_direct(const TileArgs& a, const TileState* 
     }
 }
 
-// The band walks' rows, two pixels at a time. A row is w = min(bw rounded up to even, box
-// width) pixels wide and starts at the band's start clamped into [kxb0, kxb1 - w + 1]. A clamped
-// row still holds every pixel of its support that lies in the box (the support's pixels of row
-// ky are in [xs, xs + bw - 1]; clamping slides that window into the box without dropping any of
-// them, and when w is the box width the row is the whole box row), so no pixel needs an in-box
-// test. When w is odd, the second pixel of each row's last pair lies just outside the box and
-// is masked: the remaining-pair count there is tail.
+// The band walks: the rows of a photon's band (see Band) inside its box, two pixels at a time. A
+// row is w = min(2 floor(hw + 1), box width) pixels wide and starts at the first pixel at or
+// after the band's left edge xc - hw, clamped into [kxb0, kxb1 - w + 1]. The support's pixels of
+// a row are at most floor(2 hw) + 1 <= 2 floor(hw + 1) in a row, so the window holds them all;
+// clamping slides it into the box without dropping any that lies there, and when w is the box
+// width the row is the whole box row, so no pixel needs an in-box test. When w is odd, the second
+// pixel of each row's last pair lies just outside the box and is masked: the remaining-pair count
+// is tail there. (A pixel that rounding puts just outside the window is at the support's edge to
+// within some 1e-6 of a pixel: it adds (1 - s)^2 ~ 1e-12 of the peak.)
 //
-// Row starts are formed without conversions: round-to-nearest of alpha - hw - 1/2 + beta ky, by
-// adding and taking off 1.5 * 2^23 (the sum's low mantissa bits are then the integer itself).
-// That is the floor, or one less where the band starts exactly on a pixel, which still covers
-// the row (bw = floor(2 hw) + 2).
-constexpr float kRoundMagic = 12582912.f;
-constexpr uint32_t kRoundMagicBits = 0x4B400000u;
+// With rho = ky + dy0 / sy the photon's row offset in pixels, the support of a row is centred on
+// the column xc = beta rho - dx0 / sx, and with e = kx - xc
+//   s = |M d|^2 = A e^2 + B rho^2,  A = |M (sx, 0)|^2,  B = (det M sx sy)^2 / A,
+// so a pixel costs three operations (e, e^2, 1 - s = (1 - B rho^2) - A e^2) where u = M d and
+// |u|^2 cost six, and nothing cancels: both terms of s are positive.
+//
+// Row starts are formed without conversions: round-to-nearest of xc - hw + 1/2, by adding and
+// taking off 1.5 * 2^23 (the sum's low mantissa bits are then the integer itself).
 
 struct PairWalk {
-    int ky0, rows, npairs, tail;
-    float x0, beta, lo, hi;  // row start before rounding at ky = 0, its step, the clamp range
+    int rows, npairs, tail;
+    float ky0;            // first row
+    float dyp, dxp, beta; // dy0 / sy, dx0 / sx, the centre's shift a row
+    float A, B;
+    float hw5, lo, hi;    // hw - 1/2, the clamp range of the row starts
+    uint32_t row;         // 4 * (accumulator index of the first row's column 0 - kRoundMagicBits)
 };
 
-__device__ __forceinline__ PairWalk pair_walk(const Band& bd, int kxb0, int kxb1, int kyb0,
-                                              int kyb1) {
-    PairWalk p;
-    const int w = min((bd.bw + 1) & ~1, kxb1 - kxb0 + 1);
-    p.ky0 = max(bd.ky0, kyb0);
-    p.rows = min(bd.ky1, kyb1) - p.ky0 + 1;
+// False where the photon has no band (make_band's conditions, and photons that fail the
+// reference's image-half-size ellipse test somewhere in their box). It is a third of a small
+// photon's instructions, so everything is in pixel units and the reciprocals are the hardware's;
+// what s depends on is then made exact to the last place: det M and the columns' product are
+// formed without cancellation (a product's rounding error is added back) and the quotients by A
+// corrected by their residue.
+__device__ __forceinline__ bool pair_walk(const Rec& r, const TileInfo& ti, int sw, PairWalk& p) {
+    const float m00 = r.m00 * ti.sx, m10 = r.m10 * ti.sx, m01 = r.m01 * ti.sy, m11 = r.m11 * ti.sy;
+    const float A = fmaf(m00, m00, m10 * m10);
+    const float cd = m01 * m10, cb = m10 * m11;
+    const float d1 = fmaf(m00, m11, -cd);
+    const float det = d1 - fmaf(m01, m10, -cd);
+    const float hw = rsqrt_fast(A), iA = rcp_fast(A);
+    const float ey = A * hw * rcp_fast(fabsf(det));  // the support's half-height, sqrt(A) / |det|
+    const uint32_t bits = r.packed;
+    const int rx = rec_rx(bits), ry = rec_ry(bits), lx = rec_lx(bits), ly = rec_ly(bits);
+    if (!((bits & kFlagEllipseAll) && A > 0.f && A < 1e30f && hw <= float(rx) + 1.f && ey < 1e6f &&
+          fabsf(det) > 1e-3f * (fabsf(d1 + cd) + fabsf(cd))))
+        return false;
+    const float bco = fmaf(m00, m01, cb) + fmaf(m10, m11, -cb);
+    const float qd = det * iA, qb = bco * iA;
+    p.A = A;
+    p.B = fmaf(fmaf(-A, qd, det), iA, qd) * det;
+    p.beta = -fmaf(fmaf(-A, qb, bco), iA, qb);
+    p.dxp = r.dx0 * ti.isx;
+    p.dyp = r.dy0 * ti.isy;
+    // the clipped box, in offsets from the centre pixel
+    const int pxc = ti.ox + lx, pyc = ti.oy + ly;
+    const int kxb0 = -min(rx, pxc), kxb1 = min(rx, ti.W - 1 - pxc);
+    const int boxw = kxb1 - kxb0 + 1;
+    const int w = min(2 * band_pairs(hw), boxw);
+    const int ky0 = max(__float2int_ru(-ey - p.dyp), -min(ry, pyc));
+    p.rows = min(__float2int_rd(ey - p.dyp), min(ry, ti.H - 1 - pyc)) - ky0 + 1;
     p.npairs = (w + 1) >> 1;
     p.tail = w & 1;
-    p.x0 = bd.alpha - bd.hw - 0.5f;
-    p.beta = bd.beta;
+    p.ky0 = float(ky0);
+    p.hw5 = hw - 0.5f;
     p.lo = float(kxb0);
     p.hi = float(kxb1 - w + 1);
-    return p;
+    p.row = 4u * (uint32_t((ly + ky0) * sw + lx) - kRoundMagicBits);
+    return true;
 }
 
-// Row start of row ky (kyf = float(ky)): kRoundMagic + the start column.
-__device__ __forceinline__ float pair_row(const PairWalk& p, float kyf) {
-    return fminf(fmaxf(fmaf(kyf, p.beta, p.x0), p.lo), p.hi) + kRoundMagic;
+// The start of a row: its first pixel's offset e from the row's centre, the magic sum whose bits
+// hold its column, and 1 - B rho^2.
+struct PairRow {
+    float m, e, d, rho;
+};
+
+__device__ __forceinline__ PairRow pair_row(const PairWalk& p, float ky) {
+    PairRow r;
+    r.rho = ky + p.dyp;
+    const float xc = fmaf(r.rho, p.beta, -p.dxp);
+    r.m = fminf(fmaxf(xc - p.hw5, p.lo), p.hi) + kRoundMagic;
+    r.e = (r.m - kRoundMagic) - xc;
+    r.d = fmaf(-p.B * r.rho, r.rho, 1.f);
+    return r;
 }
 
 __device__ __forceinline__ float2 pair(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float hsum(float2 v) { return v.x + v.y; }
 
-// Forward deposit of one photon over its band (see Band): one flattened loop over the rows'
-// pixel pairs, so the trip count depends only on the band's area (photons of a warp share an
-// area class), the row changing every npairs steps. False: the photon has no band.
+// Forward deposit of one photon over its band: one flattened loop over the rows' pixel pairs, so
+// the trip count depends only on the band's area (photons of a warp share an area class), the
+// row changing every npairs steps. False: the photon has no band.
 //
-// Bound by instruction issue: the two pixels of a step are the two lanes of sm_100's packed FP32
-// instructions, and a row change, which some lane of the warp makes on nearly every step, is a
-// dozen instructions with no conversion in it.
+// Bound by instruction issue. A row change, which some lane of the warp makes on nearly every
+// step, is selected rather than branched to (2^22 photons on caustic curves 403 against 430 us;
+// the backward, with more to select, is faster with the branch).
 __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, int sw, float peak,
                                              uint32_t acc_base, uint32_t* wrapped) {
-    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
-    const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
-                              float(rec_rx(r.packed)) + 1.f);
-    if (!bd.on) return false;
-    int pxc, pyc, x0, x1, y0, y1;
-    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
-    const PairWalk p = pair_walk(bd, x0 - pxc, x1 - pxc, y0 - pyc, y1 - pyc);
-    if (p.rows <= 0) return true;
-    const float2 A00 = pair(r.m00 * ti.sx), A10 = pair(r.m10 * ti.sx);
-    const float2 E3 = pair(peak);
-    const float2 M01 = pair(r.m01 * ti.sy), M11 = pair(r.m11 * ti.sy);
-    const float2 C0 = pair(fmaf(r.m00, r.dx0, r.m01 * r.dy0));
-    const float2 C1 = pair(fmaf(r.m10, r.dx0, r.m11 * r.dy0));
-    float2 KY = pair(float(p.ky0));
-    float m = pair_row(p, KY.x);
-    // (wrapping arithmetic: the magic number's bits come off again with each row's start)
-    uint32_t row = acc_base + 4u * (uint32_t((pyc + p.ky0 - ti.oy) * sw + (pxc - ti.ox)) -
-                                    kRoundMagicBits);
+    PairWalk p;
+    if (!pair_walk(r, ti, sw, p)) return false;
+    const float2 P = pair(peak);
+    float ky = p.ky0;
+    PairRow c = pair_row(p, ky);
+    // (wrapping arithmetic: the magic number's bits come off with each row's start)
+    uint32_t row = acc_base + p.row;
+    uint32_t at = row + 4u * __float_as_uint(c.m);
     int rem = p.npairs;
     uint32_t wraps = 0u;
     for (int q = p.rows * p.npairs; q > 0; --q) {
-        const uint32_t at = row + 4u * __float_as_uint(m);
-        const float2 KF = make_float2(m - kRoundMagic, m - (kRoundMagic - 1.f));
-        const float2 U0 = __ffma2_rn(KF, A00, __ffma2_rn(KY, M01, C0));
-        const float2 U1 = __ffma2_rn(KF, A10, __ffma2_rn(KY, M11, C1));
-        const float2 S = __ffma2_rn(U0, U0, __fmul2_rn(U1, U1));
+        const float e1 = c.e + 1.f;
         // 1 - s, or 0 outside the support and at the pixel after an odd row
-        const float2 D = __ffma2_rn(S, pair(-1.f), pair(1.f));
-        const float2 T = make_float2(fmaxf(D.x, 0.f), rem == p.tail ? 0.f : fmaxf(D.y, 0.f));
-        const float2 V = __fmul2_rn(__fmul2_rn(T, E3), T);
+        const float t0 = fmaxf(fmaf(-p.A * c.e, c.e, c.d), 0.f);
+        const float t1 = rem == p.tail ? 0.f : fmaxf(fmaf(-p.A * e1, e1, c.d), 0.f);
+        const float2 T = make_float2(t0, t1);
+        const float2 V = __fmul2_rn(__fmul2_rn(T, P), T);
         add_pair(at, __float2uint_rn(V.x), __float2uint_rn(V.y), wraps);
-        // the next pair: two columns on, or the next row's start (selected, not branched to:
-        // some lane changes rows on nearly every step)
+        // the next pair: two columns on, or the next row's start
         const bool wrap = --rem == 0;
-        const float2 KY1 = __fadd2_rn(KY, pair(1.f));
-        const float m1 = pair_row(p, KY1.x);
-        m = wrap ? m1 : m + 2.f;
-        KY.x = wrap ? KY1.x : KY.x;
-        KY.y = wrap ? KY1.y : KY.y;
-        row += wrap ? 4u * uint32_t(sw) : 0u;
+        const PairRow n = pair_row(p, ky + 1.f);
+        const uint32_t row1 = row + 4u * uint32_t(sw);
+        at = wrap ? row1 + 4u * __float_as_uint(n.m) : at + 8u;
+        c.e = wrap ? n.e : c.e + 2.f;
+        c.d = wrap ? n.d : c.d;
+        ky = wrap ? ky + 1.f : ky;
+        row = wrap ? row1 : row;
         rem = wrap ? p.npairs : rem;
     }
     if (wraps) *wrapped = 1u;
@@ -528,7 +564,7 @@ __device__ __forceinline__ void deposit_rows(const TileArgs& a, const TileState&
 // Backward moments of the warp's photons by padded rows (no rotation: the gathers read).
 // Per row it keeps sum t g, sum t g c and sum t g c^2 over the row's columns c and folds them
 // into the photon's moments in the integer x offset kx = xs + c and the normalised y offset,
-// as gather_band_rows does. Every lane of the warp calls it.
+// at the row's end. Every lane of the warp calls it.
 struct RowMoments {
     float sE, A0t, B1t, B2t, Sy, Sxy, Syy;
 };
@@ -610,27 +646,6 @@ __device__ __forceinline__ bool use_coop(const Rec& r, int coop_r) {
            (rec_rx(p) >= coop_r || rec_ry(p) >= coop_r);
 }
 
-// Records of the next batch of photons are copied global -> shared asynchronously while the
-// current batch is splatted (two buffers of kTileThreads records after the tile's shared
-// region). Each thread copies and later reads only its own slot, so no barrier is needed:
-// cp.async.wait_group makes the thread's own copies visible to it.
-__device__ __forceinline__ int stage_offset_floats(int sw) { return (sw * sw + 3) & ~3; }
-
-__device__ __forceinline__ void stage_rec_async(Rec* dst, const Rec* src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    const char* g = reinterpret_cast<const char*>(src);
-    asm volatile(
-        "cp.async.cg.shared.global [%0], [%1], 16;\n\t"
-        "cp.async.cg.shared.global [%2], [%3], 16;"
-        :: "r"(d), "l"(g), "r"(d + 16u), "l"(g + 16) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
 // Forward deposit of one photon by the whole warp (see use_coop).
 __device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp, const Rec* rp,
                                           uint32_t acc_base) {
@@ -662,14 +677,46 @@ __device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp
     }
 }
 
-// Next chunk of sorted photons for this CTA: a shared work counter (zero when the kernel starts)
-// hands chunks out in order as CTAs finish, so CTAs that drew chunks of large
-// footprints do not hold up the others. Nothing waits on it.
-__device__ __forceinline__ uint32_t next_chunk(uint32_t* queue, uint32_t* slot) {
-    __syncthreads();
-    if (threadIdx.x == 0) *slot = atomicAdd(queue, 1u);
-    __syncthreads();
-    return *slot;
+// Next chunk of sorted photons for this CTA (the whole warp calls it): a shared work counter
+// (zero when the kernel starts) hands chunks out in order as CTAs finish, so CTAs that drew
+// chunks of large footprints do not hold up the others. Nothing waits on it.
+__device__ __forceinline__ uint32_t take_chunk(uint32_t* queue) {
+    uint32_t c = 0u;
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(queue, 1u);
+    return __shfl_sync(0xFFFFFFFFu, c, 0);
+}
+
+__device__ __forceinline__ void prefetch_l1(const void* p) {
+    asm volatile("prefetch.global.L1 [%0];" :: "l"(p));
+}
+
+// Calls walk(i, valid) with whole warps over the photons [begin, end) of t's segment, a group of 32
+// at a time: warps take groups as they finish, from the end of the range (the footprint classes
+// ascend, so the long walks come first and the short ones fill the gaps), and each warp prefetches
+// the records of its next group. With fixed groups the warps that drew long walks, or that
+// prepared the next tile, kept the others waiting at the segment's end (a quarter of the
+// warps' time in the forward of 2^22 photons on caustic curves). Each warp calls ending() once,
+// after the first of its groups that leaves at most one a warp, or when there is none left.
+template <class Walk, class Ending>
+__device__ __forceinline__ void walk_segment(const TileArgs& a, TileState* t, uint32_t begin,
+                                             uint32_t end, Walk walk, Ending ending) {
+    const uint32_t lane = threadIdx.x & 31, n = end > begin ? end - begin : 0u;
+    uint32_t g = take_chunk(&t->groups) * 32u;
+    bool ended = false;
+    while (g < n) {
+        const uint32_t next = take_chunk(&t->groups) * 32u;
+        if (next + lane < n) prefetch_l1(a.srecs + (end - 1u - next - lane));
+        walk(end - 1u - g - lane, g + lane < n);
+        // lanes wait for their warp's longest walk here: without it they would run on into the
+        // next group a few at a time
+        __syncwarp();
+        if (!ended && next + blockDim.x >= n) {
+            ended = true;
+            ending();
+        }
+        g = next;
+    }
+    if (!ended) ending();
 }
 
 // Called by every CTA after it drew its last chunk: the last CTA to do so leaves the work counter
@@ -833,83 +880,82 @@ __device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, cons
     __syncthreads();
 }
 
-// Ends a segment of the forward (all threads call it): the accumulator's pixels into the image;
-// where photons below p1 are left, the last warp (which has the fewest rows) meanwhile starts
-// the next segment. p0: the work chunk's first photon. Returns the slot of the tile state to use
-// from here on.
-__device__ __forceinline__ int end_segment(const TileArgs& a, uint32_t* acc, int sw, TileState* ts,
-                                           int cur, uint32_t p0, uint32_t p1) {
+// The forward's chunks (all threads of the CTA call it): walk(t, i, valid) splats photon i of
+// segment t's tile into acc (whole warps call it), which each segment's end adds to the image.
+// Warp 0 takes and prepares the next chunk while the others end the current one, and the last
+// warp (which has the fewest rows to flush) the next segment while the others flush.
+template <class Walk>
+__device__ __forceinline__ void forward_chunks(const TileArgs& a, uint32_t* acc, Walk walk) {
+    __shared__ TileState ts[3];
+    __shared__ uint32_t chunks[2];
+    const int sw = a.cfg.sw;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    auto prepare = [&](TileState* t, uint32_t* slot) {
+        const uint32_t c = take_chunk(a.queue);
+        if (c < nchunks)
+            start_segment(a, first_segment(a, c, c * chunk), min(c * chunk + chunk, n_tile), t);
+        if (threadIdx.x == 0) *slot = c;
+    };
+    if (warp == 0) prepare(ts, chunks);
+    for (int k = threadIdx.x; k < sw * sw; k += blockDim.x) acc[k] = 0u;
     __syncthreads();
-    const Segment sg = ts[cur].sg;
-    if (ts[cur].wrapped) redo_segment(a, acc, ts + cur, max(sg.begin, p0), min(sg.end, p1));
-    const bool more = sg.end < p1;
-    if (more && threadIdx.x >= blockDim.x - 32)
-        start_segment(a, next_segment(a, sg), p1, ts + (cur ^ 1));
-    flush_rows(acc, sw, ts[cur], a.out);
-    __syncthreads();
-    return more ? cur ^ 1 : cur;
+    int cur = 0, alt = 1, pre = 2;
+    for (int par = 0;; par ^= 1) {
+        const uint32_t c = chunks[par];
+        if (c >= nchunks) break;
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        // every pass but the first covers at least one photon, so chunk + 1 passes suffice
+        for (uint32_t pass = 0; pass <= chunk; ++pass) {
+            const Segment sg = ts[cur].sg;
+            const uint32_t begin = max(sg.begin, p0), end = min(sg.end, p1);
+            const bool more = sg.end < p1;
+            walk_segment(
+                a, ts + cur, begin, end, [&](uint32_t i, bool valid) { walk(ts[cur], i, valid); },
+                [&] { if (!more && warp == 0) prepare(ts + pre, chunks + (par ^ 1)); });
+            __syncthreads();
+            if (ts[cur].wrapped) redo_segment(a, acc, ts + cur, begin, end);
+            if (more && threadIdx.x >= blockDim.x - 32)
+                start_segment(a, next_segment(a, sg), p1, ts + alt);
+            flush_rows(acc, sw, ts[cur], a.out);
+            __syncthreads();
+            if (!more) break;
+            const int old = cur;
+            cur = alt;
+            alt = old;
+        }
+        const int old = cur;
+        cur = pre;
+        pre = old;
+    }
+    finish_queue(a.queue);
+    tail_forward(a);
 }
 
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ uint32_t acc[];
-    __shared__ TileState ts[2];
-    __shared__ uint32_t chunk_slot;
-    const int sw = a.cfg.sw;
-    Rec* stage = reinterpret_cast<Rec*>(acc + stage_offset_floats(sw));
-    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0u;
     const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
-    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
-    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
-    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
-         c = next_chunk(a.queue, &chunk_slot)) {
-        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
-        if (p0 + threadIdx.x < p1)
-            stage_rec_async(stage + threadIdx.x, a.srecs + p0 + threadIdx.x);
-        cp_async_commit();
-        if (threadIdx.x < 32) start_segment(a, first_segment(a, c, p0), p1, ts);
-        __syncthreads();
-        int cur = 0, buf = 0;
-        for (uint32_t base = p0; base < p1; base += NT, buf ^= 1) {
-            const uint32_t i = base + threadIdx.x;
-            cp_async_wait_all();
-            const Rec* slot = stage + buf * NT + threadIdx.x;
-            if (i + NT < p1) stage_rec_async(stage + (buf ^ 1) * NT + threadIdx.x, a.srecs + i + NT);
-            cp_async_commit();
-            // The batch's segments (runs of one tile) are consecutive thread ranges; each
-            // pass handles one and flushes the tile's accumulator when the next one starts.
-            // Every pass but the first covers at least one photon, so NT + 1 passes suffice.
-            for (int pass = 0; pass <= NT; ++pass) {
-                const TileState& t = ts[cur];
-                bool coop = false;
-                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
-                    const Rec r = *slot;
-                    coop = use_coop(r, a.cfg.coop_r);
-                    const float peak = count_peak(t, r.e);
-                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
-                        if (!(peak > 0.f))
-                            deposit_direct(a, &t, slot);
-                        else if (!(a.cfg.band && deposit_band(r, t.ti, sw, peak, acc_base,
-                                                              &ts[cur].wrapped)))
-                            deposit_generic(a, &t, slot, peak, acc_base);
-                    }
-                }
-                // lanes wait for their warp's longest walk here: without it they would run on into
-                // the next batch a few at a time
-                __syncwarp();
-                if (a.cfg.coop_r > 0) {
-                    for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
-                        deposit_coop(a, &t, stage + buf * NT + (threadIdx.x & ~31u) + (__ffs(cm) - 1),
-                                     acc_base);
-                }
-                if (t.sg.end >= min(base + NT, p1)) break;
-                cur = end_segment(a, acc, sw, ts, cur, p0, p1);
+    forward_chunks(a, acc, [&](TileState& t, uint32_t i, bool valid) {
+        bool coop = false;
+        if (valid) {
+            const Rec r = a.srecs[i];
+            coop = use_coop(r, a.cfg.coop_r);
+            const float peak = count_peak(t, r.e);
+            if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
+                if (!(peak > 0.f))
+                    deposit_direct(a, &t, a.srecs + i);
+                else if (!(a.cfg.band && deposit_band(r, t.ti, a.cfg.sw, peak, acc_base, &t.wrapped)))
+                    deposit_generic(a, &t, a.srecs + i, peak, acc_base);
             }
         }
-        end_segment(a, acc, sw, ts, cur, p0, p1);
-    }
-    finish_queue(a.queue);
-    tail_forward(a);
+        if (a.cfg.coop_r > 0) {
+            __syncwarp();
+            for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
+                deposit_coop(a, &t, a.srecs + __shfl_sync(0xFFFFFFFFu, i, __ffs(cm) - 1), acc_base);
+        }
+    });
 }
 
 // Stages the upstream gradient that a tile's photons read (clipped to the image): the tile and
@@ -917,7 +963,8 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
 // tile_r, at most the apron), and the column after them (the band walk reads, and discards,
 // the pixel after an odd row's end; the pitch sw = tile + 2 apron + 1 has room for it). The
 // apron's outer margin, which no photon of the tile reaches, is not loaded. Warps take rows,
-// lanes take consecutive columns.
+// lanes take consecutive columns; the copies are asynchronous, so that a warp's rows are all in
+// flight together (four-byte copies: the odd pitch aligns nothing wider).
 __device__ __forceinline__ void load_region(float* tg, int sw, const TileState& t,
                                             const float* grad) {
     const int gx1 = min(t.x1 + 1, t.ti.W - 1), y1 = t.y1;
@@ -929,9 +976,16 @@ __device__ __forceinline__ void load_region(float* tg, int sw, const TileState& 
     for (int gy = t.y0 + warp; gy <= y1; gy += nw) {
         float* trow = tg + (gy - oy) * sw - ox;
         const float* grow = img + int64_t(gy) * W;
-        for (int gx = t.x0 + lane; gx <= gx1; gx += 32)
-            trow[gx] = in_image ? __ldg(grow + gx) : 0.f;
+        for (int gx = t.x0 + lane; gx <= gx1; gx += 32) {
+            if (in_image)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;"
+                             :: "r"(uint32_t(__cvta_generic_to_shared(trow + gx))), "l"(grow + gx)
+                             : "memory");
+            else
+                trow[gx] = 0.f;
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 __device__ __forceinline__ void store_grad(GradRec* stage, uint32_t rid, float gE, float gx0,
@@ -1009,124 +1063,64 @@ __device__ __forceinline__ void bwd_row(int n, const float* q, float k0, float b
     }
 }
 
-// The backward walks the band inside the clipped box. A row is w = min(bw rounded up to
-// even, box width) pixels wide and starts at the band's start clamped into
-// [kxb0, kxb1 - w + 1]. A clamped row still holds every pixel of its support that lies in the
-// box (the support's pixels of row ky are in [xs, xs + bw - 1]; clamping slides that window
-// into the box without dropping any of them, and when w is the box width the row is the whole
-// box row), so no pixel needs an in-box test. Rows are walked two pixels at a time; when w is
-// odd, the second pixel of each row's last pair lies just outside the box and is masked.
-struct BandWalk {
-    int w, npairs, tail, kxb0, kxlast;
-};
-
-__device__ __forceinline__ BandWalk band_walk(const Band& bd, int kxb0, int kxb1) {
-    BandWalk b;
-    b.w = min((bd.bw + 1) & ~1, kxb1 - kxb0 + 1);
-    b.npairs = (b.w + 1) >> 1;
-    b.tail = b.w & 1;  // value of the remaining-pair count at which the mask applies
-    b.kxb0 = kxb0;
-    b.kxlast = kxb1 - b.w + 1;
-    return b;
-}
-
-__device__ __forceinline__ int band_row_start(const Band& bd, const BandWalk& bw, int ky) {
-    return min(max(band_start(bd, ky), bw.kxb0), bw.kxlast);
-}
-
-// Backward moments over the band rows ky0..ky1 (ky0 <= ky1). Per row it keeps sum t g and
-// sum t g kx (kx the integer pixel offset) and folds them into the y moments at the row
-// change; sum t g kx^2 and sum t^2 g run over the whole band. The masked pixel of an odd row
-// (just outside the box) is read from the staged tile's spare column (the pitch is odd:
-// tile + 2 apron + 1, and a box never reaches past column tile + 2 apron - 1) and its product
-// discarded. The two pixels of a step are evaluated as the two lanes of sm_100's packed FP32
-// instructions (__ffma2_rn / __fmul2_rn / __fadd2_rn: one instruction for both pixels, each
-// lane rounded as its scalar counterpart); the even and odd pixels keep separate partial sums,
-// added where a row or the band ends.
-struct BandMoments {
-    float sE, A0t, B1t, B2, Sy, Sxy, Syy;
-};
-
-__device__ __forceinline__ BandMoments gather_band_rows(const Band& bd, const BandWalk& bw,
-                                                        int ky, int ky1, const float* row,
-                                                        int sw, float a00, float a10, float c0,
-                                                        float c1, float m01sy, float m11sy,
-                                                        float sy, float dy0, float sx,
-                                                        float dx0) {
-    BandMoments m = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float2 A00 = pair(a00), A10 = pair(a10);
-    float2 C0 = pair(c0), C1 = pair(c1);
-    float2 SE = pair(0.f), B2 = pair(0.f), A0 = pair(0.f), B1 = pair(0.f);
-    int xs = band_row_start(bd, bw, ky);
-    float2 KF = make_float2(float(xs), float(xs + 1));
-    const float* q = row + xs;
-    int rem = bw.npairs;
-    for (;;) {
-        // u = M d at the two pixels, s = |u|^2, t = max(1 - s, 0)
-        const float2 U0 = __ffma2_rn(KF, A00, C0), U1 = __ffma2_rn(KF, A10, C1);
-        const float2 S = __ffma2_rn(U0, U0, __fmul2_rn(U1, U1));
-        const float2 T = make_float2(fmaxf(1.f - S.x, 0.f), fmaxf(1.f - S.y, 0.f));
-        const float2 Q = make_float2(q[0], rem == bw.tail ? 0.f : q[1]);
-        const float2 G = __fmul2_rn(T, Q);
-        SE = __ffma2_rn(T, G, SE);
-        A0 = __fadd2_rn(A0, G);
-        const float2 TK = __fmul2_rn(G, KF);
-        B1 = __fadd2_rn(B1, TK);
-        B2 = __ffma2_rn(TK, KF, B2);
-        KF = __fadd2_rn(KF, pair(2.f));
-        q += 2;
-        if (--rem == 0) {
-            const float a0 = hsum(A0), b1 = hsum(B1);
-            const float dy = fmaf(float(ky), sy, dy0);
-            const float sdx = fmaf(sx, b1, dx0 * a0);
-            m.Sy = fmaf(dy, a0, m.Sy);
-            m.Sxy = fmaf(dy, sdx, m.Sxy);
-            m.Syy = fmaf(dy * dy, a0, m.Syy);
-            m.A0t += a0;
-            m.B1t += b1;
-            if (++ky > ky1) break;
-            A0 = pair(0.f);
-            B1 = pair(0.f);
-            rem = bw.npairs;
-            xs = band_row_start(bd, bw, ky);
-            KF = make_float2(float(xs), float(xs + 1));
-            C0 = __fadd2_rn(C0, pair(m01sy));
-            C1 = __fadd2_rn(C1, pair(m11sy));
-            row += sw;
-            q = row + xs;
-        }
-    }
-    m.sE = hsum(SE);
-    m.B2 = hsum(B2);
-    return m;
-}
-
-// Backward gather of one photon over its band's rows in the box (see BandWalk); with no row
-// inside the box (ky0 > ky1) its gradients are zero. False: the photon has no band.
+// Backward gather of one photon over its band's rows in the box, two pixels a step (PairWalk;
+// the pixel after an odd row is read from the staged tile's spare column, the pitch is odd: tile +
+// 2 apron + 1, and a box never reaches past column tile + 2 apron - 1, and its value discarded).
+// With no row inside the box its gradients are zero. False: the photon has no band.
+//
+// Bound by the FP32 pipe and instruction issue. The moments run over the whole band, in the walk's own coordinates: with
+// t = 1 - s, sums of t^2 g, t g e, t g e^2, t g rho, t g e rho, t g rho^2, from which those
+// of the offset d = (sx (e + beta rho), sy rho) follow once per photon. The two pixels of a step
+// are the two lanes of packed FP32 instructions with partial sums of their own. (Folding a row's
+// sums at its end instead cost about 28 instructions that some lane of the warp ran on nearly
+// every step, and kept the lanes apart.)
 __device__ __forceinline__ bool gather_band(const Rec& r, const TileInfo& ti, int sw,
                                             const float* tg, uint32_t slot, GradRec* stage) {
-    if (!(rec_flags(r.packed) & kFlagEllipseAll)) return false;
-    const Band bd = make_band(r.m00, r.m01, r.m10, r.m11, r.dx0, r.dy0, ti.sy, ti.isx, ti.isy,
-                              float(rec_rx(r.packed)) + 1.f);
-    if (!bd.on) return false;
-    int pxc, pyc, x0, x1, y0, y1;
-    rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
-    const int ky0 = max(bd.ky0, y0 - pyc), ky1 = min(bd.ky1, y1 - pyc);
-    const int kxb0 = x0 - pxc, kxb1 = x1 - pxc;
-    const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
-    const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
-    const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
-    const float c0 = fmaf(float(ky0), m01sy, c00), c1 = fmaf(float(ky0), m11sy, c10);
-    const float* row = tg + (pyc + ky0 - ti.oy) * sw + (pxc - ti.ox);
-    BandMoments m = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (ky0 <= ky1)
-        m = gather_band_rows(bd, band_walk(bd, kxb0, kxb1), ky0, ky1, row, sw, a00, a10, c0,
-                             c1, m01sy, m11sy, ti.sy, r.dy0, ti.sx, r.dx0);
-    const float Sx = fmaf(ti.sx, m.B1t, r.dx0 * m.A0t);
-    const float Sxx = fmaf(ti.sx * ti.sx, m.B2,
-                           fmaf(2.f * ti.sx * r.dx0, m.B1t, r.dx0 * r.dx0 * m.A0t));
-    finish_grad(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, m.sE, Sx, m.Sy, Sxx, m.Sxy,
-                m.Syy);
+    float2 SE = pair(0.f), GE = pair(0.f), GEE = pair(0.f), GR = pair(0.f),
+           GER = pair(0.f), GRR = pair(0.f);
+    PairWalk p;
+    if (!pair_walk(r, ti, sw, p)) return false;
+    {
+        float ky = p.ky0;
+        PairRow c = pair_row(p, ky);
+        float2 R = pair(c.rho);
+        // (wrapping arithmetic, as in deposit_band)
+        uint32_t row = p.row;
+        uint32_t at = row + 4u * __float_as_uint(c.m);
+        const char* base = reinterpret_cast<const char*>(tg);
+        int rem = p.npairs;
+        for (int q = p.rows * p.npairs; q > 0; --q) {
+            const float* g = reinterpret_cast<const float*>(base + at);
+            const float2 Q = make_float2(g[0], rem == p.tail ? 0.f : g[1]);
+            const float2 E = make_float2(c.e, c.e + 1.f);
+            const float2 T = make_float2(fmaxf(fmaf(-p.A * E.x, E.x, c.d), 0.f),
+                                         fmaxf(fmaf(-p.A * E.y, E.y, c.d), 0.f));
+            const float2 G = __fmul2_rn(T, Q);
+            const float2 X = __fmul2_rn(G, E), Y = __fmul2_rn(G, R);
+            SE = __ffma2_rn(T, G, SE);
+            GE = __fadd2_rn(GE, X);
+            GEE = __ffma2_rn(X, E, GEE);
+            GR = __fadd2_rn(GR, Y);
+            GER = __ffma2_rn(X, R, GER);
+            GRR = __ffma2_rn(Y, R, GRR);
+            at += 8u;
+            c.e += 2.f;
+            if (--rem == 0) {
+                ky += 1.f;
+                c = pair_row(p, ky);
+                R = pair(c.rho);
+                row += 4u * uint32_t(sw);
+                at = row + 4u * __float_as_uint(c.m);
+                rem = p.npairs;
+            }
+        }
+    }
+    const float gr = hsum(GR), grr = hsum(GRR), ger = hsum(GER);
+    const float bgr = p.beta * grr;
+    const float Sx = ti.sx * fmaf(p.beta, gr, hsum(GE)), Sy = ti.sy * gr;
+    const float Sxx = (ti.sx * ti.sx) * fmaf(p.beta, fmaf(2.f, ger, bgr), hsum(GEE));
+    const float Sxy = (ti.sx * ti.sy) * (ger + bgr), Syy = (ti.sy * ti.sy) * grr;
+    finish_grad(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, hsum(SE), Sx, Sy, Sxx, Sxy, Syy);
     return true;
 }
 
@@ -1286,58 +1280,82 @@ __device__ __noinline__ void tail_backward(const TileArgs& a) {
     }
 }
 
-// Moves the backward on to the next segment's tile (all threads call it).
-__device__ __forceinline__ void next_tile(const TileArgs& a, float* tg, int sw, TileState* t) {
+// The backward's chunks (all threads of the CTA call it): walk(t, i, valid) gathers photon i of
+// segment t's tile from tg (whole warps call it). Warp 0 prepares the next segment, or takes and
+// prepares the next chunk, while the others end the current one.
+template <class Walk>
+__device__ __forceinline__ void backward_chunks(const TileArgs& a, float* tg, Walk walk) {
+    __shared__ TileState ts[3];
+    __shared__ uint32_t chunks[2];
+    const int sw = a.cfg.sw;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
+    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
+    auto prepare = [&](TileState* t, uint32_t* slot) {
+        const uint32_t c = take_chunk(a.queue);
+        if (threadIdx.x == 0) {
+            if (c < nchunks) set_tile(a, first_segment(a, c, c * chunk), t);
+            *slot = c;
+        }
+    };
+    if (warp == 0) prepare(ts, chunks);
     __syncthreads();
-    if (threadIdx.x == 0) set_tile(a, next_segment(a, t->sg), t);
-    __syncthreads();
-    load_region(tg, sw, *t, a.grad);
-    __syncthreads();
+    int cur = 0, alt = 1, pre = 2;
+    for (int par = 0;; par ^= 1) {
+        const uint32_t c = chunks[par];
+        if (c >= nchunks) break;
+        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
+        for (uint32_t pass = 0; pass <= chunk; ++pass) {
+            load_region(tg, sw, ts[cur], a.grad);
+            __syncthreads();
+            const Segment sg = ts[cur].sg;
+            const uint32_t begin = max(sg.begin, p0), end = min(sg.end, p1);
+            const bool more = sg.end < p1;
+            walk_segment(
+                a, ts + cur, begin, end, [&](uint32_t i, bool valid) { walk(ts[cur], i, valid); },
+                [&] {
+                    if (warp != 0) return;
+                    if (!more)
+                        prepare(ts + pre, chunks + (par ^ 1));
+                    else if (threadIdx.x == 0)
+                        set_tile(a, next_segment(a, sg), ts + alt);
+                });
+            __syncthreads();
+            if (!more) break;
+            const int old = cur;
+            cur = alt;
+            alt = old;
+        }
+        const int old = cur;
+        cur = pre;
+        pre = old;
+    }
+    finish_queue(a.queue);
+    tail_backward(a);
 }
 
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ float tg[];
-    __shared__ TileState t;
-    __shared__ uint32_t chunk_slot;
-    const int sw = a.cfg.sw;
-    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
-    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
-    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
-         c = next_chunk(a.queue, &chunk_slot)) {
-        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
-        // next_chunk's barrier ends the previous chunk's reads of the tile state and the tile
-        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), &t);
-        __syncthreads();
-        load_region(tg, sw, t, a.grad);
-        __syncthreads();
-        for (uint32_t base = p0; base < p1; base += NT) {
-            const uint32_t i = base + threadIdx.x;
-            // consecutive segments of the batch, as in fwd_tiles_kernel; a photon's gradient
-            // record goes to its sorted position
-            for (int pass = 0; pass <= NT; ++pass) {
-                bool coop = false;
-                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
-                    const Rec r = a.srecs[i];
-                    coop = use_coop(r, a.cfg.coop_r);
-                    if (!coop && !(a.cfg.band && gather_band(r, t.ti, sw, tg, i, a.stage)))
-                        gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
-                }
-                __syncwarp();  // as in fwd_tiles_kernel
-                if (a.cfg.coop_r > 0) {
-                    for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                        const int src = __ffs(cm) - 1;
-                        const uint32_t slot = base + (threadIdx.x & ~31u) + uint32_t(src);
-                        gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
-                    }
-                }
-                if (t.sg.end >= min(base + NT, p1)) break;
-                next_tile(a, tg, sw, &t);
+    backward_chunks(a, tg, [&](TileState& t, uint32_t i, bool valid) {
+        const int sw = a.cfg.sw;
+        bool coop = false;
+        if (valid) {
+            const Rec r = a.srecs[i];
+            coop = use_coop(r, a.cfg.coop_r);
+            // a photon's gradient record goes to its sorted position
+            if (!coop && !(a.cfg.band && gather_band(r, t.ti, sw, tg, i, a.stage)))
+                gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
+        }
+        if (a.cfg.coop_r > 0) {
+            __syncwarp();
+            for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
+                const int src = __ffs(cm) - 1;
+                const uint32_t slot = __shfl_sync(0xFFFFFFFFu, i, src);
+                gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
             }
         }
-    }
-    finish_queue(a.queue);
-    tail_backward(a);
+    });
 }
 
 // ---- the padded-row walk's kernels (walk 4) ---------------------------------------------
@@ -1348,109 +1366,69 @@ __global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_consta
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ uint32_t acc[];
-    __shared__ TileState ts[2];
-    __shared__ uint32_t chunk_slot;
-    const int sw = a.cfg.sw;
-    for (int k = threadIdx.x; k < sw * sw; k += NT) acc[k] = 0u;
     const uint32_t acc_base = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
-    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
-    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
-    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
-         c = next_chunk(a.queue, &chunk_slot)) {
-        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
-        if (threadIdx.x < 32) start_segment(a, first_segment(a, c, p0), p1, ts);
-        __syncthreads();
-        int cur = 0;
-        for (uint32_t base = p0; base < p1; base += NT) {
-            const uint32_t i = base + threadIdx.x;
-            for (int pass = 0; pass <= NT; ++pass) {
-                const TileState& t = ts[cur];
-                RowGeo g;
-                int rows = 0;
-                float peak = 0.f;
-                bool generic = false, coop = false;
-                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
-                    const Rec r = a.srecs[i];
-                    coop = use_coop(r, a.cfg.coop_r);
-                    if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
-                        int pxc, pyc, x0, x1, y0, y1;
-                        rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
-                        peak = count_peak(t, r.e);
-                        generic = !prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
-                        rows = generic || !(peak > 0.f) ? 0 : g.rows;
-                        if (!(peak > 0.f)) {
-                            generic = false;
-                            deposit_direct(a, &t, a.srecs + i);
-                        }
-                    }
+    forward_chunks(a, acc, [&](TileState& t, uint32_t i, bool valid) {
+        RowGeo g;
+        int rows = 0;
+        float peak = 0.f;
+        bool generic = false, coop = false;
+        if (valid) {
+            const Rec r = a.srecs[i];
+            coop = use_coop(r, a.cfg.coop_r);
+            if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
+                int pxc, pyc, x0, x1, y0, y1;
+                rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
+                peak = count_peak(t, r.e);
+                if (!(peak > 0.f)) {
+                    deposit_direct(a, &t, a.srecs + i);
+                } else {
+                    generic = !prep_rows(r, t.ti, a.cfg.sw, pxc, pyc, x0, x1, y0, y1, g);
+                    rows = generic ? 0 : g.rows;
                 }
-                deposit_rows(a, t, g, rows, peak, acc_base);
-                if (generic) deposit_generic(a, &t, a.srecs + i, peak, acc_base);
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
-                    deposit_coop(a, &t, a.srecs + (base + (threadIdx.x & ~31u) + (__ffs(cm) - 1)),
-                                 acc_base);
-                if (t.sg.end >= min(base + NT, p1)) break;
-                cur = end_segment(a, acc, sw, ts, cur, p0, p1);
             }
         }
-        end_segment(a, acc, sw, ts, cur, p0, p1);
-    }
-    finish_queue(a.queue);
-    tail_forward(a);
+        __syncwarp();
+        deposit_rows(a, t, g, rows, peak, acc_base);
+        if (generic) deposit_generic(a, &t, a.srecs + i, peak, acc_base);
+        __syncwarp();
+        for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
+            deposit_coop(a, &t, a.srecs + __shfl_sync(0xFFFFFFFFu, i, __ffs(cm) - 1), acc_base);
+    });
 }
 
 template <int NT, int MINB>
 __global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ float tg[];
-    __shared__ TileState t;
-    __shared__ uint32_t chunk_slot;
-    const int sw = a.cfg.sw;
     const uint32_t tg_base = static_cast<uint32_t>(__cvta_generic_to_shared(tg));
-    const uint32_t n_tile = uint32_t(tile_count(a)), chunk = uint32_t(a.cfg.chunk);
-    const uint32_t nchunks = (n_tile + chunk - 1) / chunk;
-    for (uint32_t c = next_chunk(a.queue, &chunk_slot); c < nchunks;
-         c = next_chunk(a.queue, &chunk_slot)) {
-        const uint32_t p0 = c * chunk, p1 = min(p0 + chunk, n_tile);
-        // next_chunk's barrier ends the previous chunk's reads of the tile state and the tile
-        if (threadIdx.x == 0) set_tile(a, first_segment(a, c, p0), &t);
-        __syncthreads();
-        load_region(tg, sw, t, a.grad);
-        __syncthreads();
-        for (uint32_t base = p0; base < p1; base += NT) {
-            const uint32_t i = base + threadIdx.x;
-            for (int pass = 0; pass <= NT; ++pass) {
-                RowGeo g;
-                int rows = 0;
-                float dy0 = 0.f;
-                bool walk = false, generic = false, coop = false;
-                if (i < p1 && i >= t.sg.begin && i < t.sg.end) {
-                    const Rec r = a.srecs[i];
-                    coop = use_coop(r, a.cfg.coop_r);
-                    if (!coop) {
-                        int pxc, pyc, x0, x1, y0, y1;
-                        rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
-                        walk = prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
-                        generic = !walk;
-                        rows = walk ? g.rows : 0;
-                        dy0 = r.dy0;
-                    }
-                }
-                const RowMoments m = gather_rows(g, rows, tg_base, sw, t.ti.sy, dy0);
-                if (walk) finish_rows(a.stage, i, a.srecs[i], t.ti, m);
-                if (generic)
-                    gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
-                for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
-                    const int src = __ffs(cm) - 1;
-                    const uint32_t slot = base + (threadIdx.x & ~31u) + uint32_t(src);
-                    gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
-                }
-                if (t.sg.end >= min(base + NT, p1)) break;
-                next_tile(a, tg, sw, &t);
+    backward_chunks(a, tg, [&](TileState& t, uint32_t i, bool valid) {
+        const int sw = a.cfg.sw;
+        RowGeo g;
+        int rows = 0;
+        float dy0 = 0.f;
+        bool walk = false, generic = false, coop = false;
+        if (valid) {
+            const Rec r = a.srecs[i];
+            coop = use_coop(r, a.cfg.coop_r);
+            if (!coop) {
+                int pxc, pyc, x0, x1, y0, y1;
+                rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
+                walk = prep_rows(r, t.ti, sw, pxc, pyc, x0, x1, y0, y1, g);
+                generic = !walk;
+                rows = walk ? g.rows : 0;
+                dy0 = r.dy0;
             }
         }
-    }
-    finish_queue(a.queue);
-    tail_backward(a);
+        __syncwarp();
+        const RowMoments m = gather_rows(g, rows, tg_base, sw, t.ti.sy, dy0);
+        if (walk) finish_rows(a.stage, i, a.srecs[i], t.ti, m);
+        if (generic) gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
+        __syncwarp();
+        for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
+            const int src = __ffs(cm) - 1;
+            const uint32_t slot = __shfl_sync(0xFFFFFFFFu, i, src);
+            gather_coop(a.srecs + slot, t.ti, sw, tg, slot, src, a.stage);
+        }
+    });
 }
 
 // Spreads the gradient records into the reference's outputs grad_Ep[N], grad_xp[2][N],
@@ -1560,17 +1538,12 @@ int persistent_grid(size_t smem, int64_t n_units) {
 }  // namespace
 
 
-// Dynamic shared memory of a tile kernel: the tile's region (sw x sw floats) and, for the
-// band forward (staged), the two record buffers after it.
-size_t tile_smem(const TileArgs& a, bool staged) {
-    const size_t sw = size_t(a.cfg.sw);
-    if (!staged) return sw * sw * sizeof(float);
-    return (((sw * sw + 3) & ~size_t(3)) * sizeof(float)) + 2 * size_t(kTileThreads) * sizeof(Rec);
-}
+// Dynamic shared memory of a tile kernel: the tile's region, sw x sw words.
+size_t tile_smem(const TileArgs& a) { return size_t(a.cfg.sw) * size_t(a.cfg.sw) * 4; }
 
 template <int MINB, bool ROWS>
 cudaError_t launch_forward_t(const TileArgs& a, cudaStream_t st) {
-    const size_t smem = tile_smem(a, !ROWS);
+    const size_t smem = tile_smem(a);
     constexpr auto kern = ROWS ? fwd_rows_kernel<kTileThreads, MINB>
                                : fwd_tiles_kernel<kTileThreads, MINB>;
     const cudaError_t e = allow_smem<kern>(smem);
@@ -1583,7 +1556,7 @@ cudaError_t launch_forward_t(const TileArgs& a, cudaStream_t st) {
 
 template <int MINB, bool ROWS>
 cudaError_t launch_backward_t(const TileArgs& a, cudaStream_t st) {
-    const size_t smem = tile_smem(a, false);
+    const size_t smem = tile_smem(a);
     constexpr auto kern = ROWS ? bwd_rows_kernel<kTileThreads, MINB>
                                : bwd_tiles_kernel<kTileThreads, MINB>;
     cudaError_t e = allow_smem<kern>(smem);
@@ -1626,12 +1599,12 @@ cudaError_t launch_forward(const TileArgs& a, cudaStream_t st) {
 
 cudaError_t launch_backward(const TileArgs& a, cudaStream_t st) {
     if (a.cfg.rows) {
-        if (a.cfg.min_blocks_bwd >= 4) return launch_backward_t<4, true>(a, st);
-        return a.cfg.min_blocks_bwd == 3 ? launch_backward_t<3, true>(a, st)
+        if (a.cfg.min_blocks >= 4) return launch_backward_t<4, true>(a, st);
+        return a.cfg.min_blocks == 3 ? launch_backward_t<3, true>(a, st)
                                      : launch_backward_t<2, true>(a, st);
     }
-    if (a.cfg.min_blocks_bwd >= 4) return launch_backward_t<4, false>(a, st);
-    return a.cfg.min_blocks_bwd == 3 ? launch_backward_t<3, false>(a, st)
+    if (a.cfg.min_blocks >= 4) return launch_backward_t<4, false>(a, st);
+    return a.cfg.min_blocks == 3 ? launch_backward_t<3, false>(a, st)
                                  : launch_backward_t<2, false>(a, st);
 }
 
