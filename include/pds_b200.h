@@ -194,6 +194,27 @@ int pds_batch_backward_planned_f32(const float* grad, const float* Ep, const flo
                                    void* workspace, size_t workspace_bytes,
                                    const pds_config* cfg, void* stream);
 
+/* ---- splat inputs of traced photons ----------------------------------------------- */
+/* Replaces model/caustics.py:224-239 (change_of_basis_matrix, splat_photons) up to the splat: the
+ * splat inputs Ep[N], Mp[2][3][N], cp[N], radius[N] of photons with receiver-plane differentials
+ * Du[3][N], Dv[3][N], receiver normals normal[3][N], flux[N] and channel[N]; degenerate photons
+ * (Du . (Dv x normal) = 0) get channel -1. */
+int pds_splat_inputs_f32(const float* Du, const float* Dv, const float* normal, const float* flux,
+                         const int64_t* channel, int64_t n_photons, float* Ep, float* Mp,
+                         int64_t* cp, float* radius, void* stream);
+
+/* Their backward together with the splat's spread: from the gradient records that
+ * pds_backward_planned_f32 (with its gradient outputs NULL) left in the workspace of the plan of
+ * these photons (channels, height, width and cfg as passed to the splat calls), writes
+ * grad_xp[2][N] and, where not NULL, grad_Du[3][N], grad_Dv[3][N], grad_normal[3][N],
+ * grad_flux[N]. */
+int pds_splat_inputs_backward_planned_f32(const float* Du, const float* Dv, const float* normal,
+                                          const float* flux, int64_t n_photons, int64_t channels,
+                                          int64_t height, int64_t width, const void* workspace,
+                                          size_t workspace_bytes, const pds_config* cfg,
+                                          float* grad_xp, float* grad_Du, float* grad_Dv,
+                                          float* grad_normal, float* grad_flux, void* stream);
+
 /* ---- refraction to the receiver for a height-field glass plate --------------------- */
 /* Replaces, for a plate whose top face is a height field lit by collimated light, the
  * reference's refraction chain from the traced hit to the splat inputs:

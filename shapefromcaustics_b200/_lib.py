@@ -92,6 +92,10 @@ SIGNATURES = {
     "pds_batch_backward_planned_f32": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _I64, _P, _I32,
                                                       _I64, _I64, _I32, _P, _P, _P, _P, _SZ, _CFG,
                                                       _P]),
+    "pds_splat_inputs_f32": (ctypes.c_int, [_P, _P, _P, _P, _P, _I64, _P, _P, _P, _P, _P]),
+    "pds_splat_inputs_backward_planned_f32": (ctypes.c_int, [_P, _P, _P, _P, _I64, _I64, _I64,
+                                                             _I64, _P, _SZ, _CFG, _P, _P, _P, _P,
+                                                             _P, _P]),
     "pds_refract_forward_f32": (ctypes.c_int, [_P, _I32, _I32, ctypes.POINTER(PdsPlate), _P, _P,
                                                _P, _P, _I64, _P, _P, _P, _P, _P, _P]),
     "pds_refract_backward_f32": (ctypes.c_int, [_P, _I32, _I32, ctypes.POINTER(PdsPlate), _P, _P,

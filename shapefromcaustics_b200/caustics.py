@@ -15,7 +15,10 @@ gradient), so shapes stay static and nothing waits on the device.
 """
 import torch
 
+from . import photon_differential
+from ._lib import check, lib
 from .photon_differential import PDS
+from .splatting import SplatPlan, _cfg_ref, _ptr, _stream
 
 __all__ = ["change_of_basis_matrix", "splat_inputs", "splat_photons"]
 
@@ -43,9 +46,75 @@ def splat_inputs(Du, Dv, normal, flux, channel):
     return Ep.contiguous(), Mp.contiguous(), cp.contiguous(), radius.contiguous()
 
 
+class _SplatPhotons(torch.autograd.Function):
+    """``splat_inputs`` and the splat in one node: one kernel each way for the splat inputs
+    (``pds_splat_inputs_f32``), the backward's reading the splat gradients as the plan's records.
+    Plain float32 CUDA tensors only (``_fusable``)."""
+
+    @staticmethod
+    def forward(ctx, Du, Dv, normal, flux, xy, channel, output_size, max_pixel_radius):
+        n, dev = flux.numel(), flux.device
+        Ep, radius = torch.empty_like(flux), torch.empty_like(flux)
+        Mp = torch.empty((2, 3, n), dtype=torch.float32, device=dev)
+        cp = torch.empty((1, n), dtype=torch.int64, device=dev)
+        with torch.cuda.device(dev):
+            check(lib().pds_splat_inputs_f32(_ptr(Du), _ptr(Dv), _ptr(normal), _ptr(flux),
+                                             _ptr(channel), n, _ptr(Ep), _ptr(Mp), _ptr(cp),
+                                             _ptr(radius), _stream(dev)))
+        plan = SplatPlan(Ep, xy, Mp, cp, radius, output_size, max_pixel_radius)
+        out = plan.forward()
+        ctx.save_for_backward(Du, Dv, normal, flux, xy, channel, Ep, Mp, cp, radius)
+        ctx.shape = (plan.C, plan.H, plan.W)
+        ctx.mpr = plan.mpr
+        ctx.cfg = plan.cfg
+        ctx.plan_ws = plan.ws if photon_differential._keep_plan else None
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        Du, Dv, normal, flux, xy, channel, Ep, Mp, cp, radius = ctx.saved_tensors
+        ws, ctx.plan_ws = ctx.plan_ws, None
+        plan = SplatPlan.planned((Ep, xy, Mp, cp, radius), ctx.shape, ctx.mpr, ctx.cfg, ws)
+        if torch.is_grad_enabled():  # create_graph: the splat inputs' own torch operations
+            gE, gX, gM = plan.backward(grad.contiguous())
+            E, M, _, _ = splat_inputs(Du, Dv, normal, flux, channel)
+            wanted = [t for t, w in zip((Du, Dv, normal, flux), ctx.needs_input_grad) if w]
+            got = iter(torch.autograd.grad((E, M), wanted, (gE, gM), create_graph=True,
+                                           allow_unused=True) if wanted else ())
+            grads = [next(got) if w else None for w in ctx.needs_input_grad[:4]]
+            return (*grads, gX, None, None, None)
+        plan.backward(grad.contiguous(), records=True)
+        gX = torch.empty_like(xy)
+        grads = [torch.empty_like(t) if w else None
+                 for t, w in zip((Du, Dv, normal, flux), ctx.needs_input_grad)]
+        with torch.cuda.device(flux.device):
+            check(lib().pds_splat_inputs_backward_planned_f32(
+                _ptr(Du), _ptr(Dv), _ptr(normal), _ptr(flux), flux.numel(), *ctx.shape,
+                _ptr(plan.ws), plan.ws.numel(), _cfg_ref(ctx.cfg), _ptr(gX),
+                *(_ptr(g) for g in grads), _stream(flux.device)))
+        return (*grads, gX if ctx.needs_input_grad[4] else None, None, None, None)
+
+
+def _fusable(Du, Dv, normal, flux, xy, channel):
+    """Whether the kernels take these photons as they are: plain float32 CUDA tensors of one
+    device, [3, N] each, [N] fluxes, an int64 [N] channel (anything else, broadcast shapes among
+    it, goes through the torch operations)."""
+    n = flux.numel()
+    real = (Du, Dv, normal, flux, xy)
+    return (n > 0 and flux.shape == (n,) and Du.shape == Dv.shape == normal.shape == (3, n) and
+            xy.shape == (2, n) and channel.shape == (n,) and channel.dtype == torch.int64 and
+            all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and
+                t.device == flux.device for t in (*real, channel)) and
+            all(t.dtype == torch.float32 for t in real))
+
+
 def splat_photons(Du, Dv, normal, flux, positions_xy, channel, output_size, max_pixel_radius=20):
     """``model/caustics.py:233-239``: splat photons given their receiver-plane position
     ``positions_xy [2, N]`` (normalised receiver coordinates) and differentials."""
+    if _fusable(Du, Dv, normal, flux, positions_xy, channel):
+        return _SplatPhotons.apply(*(t.contiguous() for t in (Du, Dv, normal, flux, positions_xy,
+                                                              channel)),
+                                   tuple(output_size), max_pixel_radius)
     Ep, Mp, cp, radius = splat_inputs(Du, Dv, normal, flux, channel)
     return PDS.apply(Ep, positions_xy.contiguous(), Mp, cp, radius, tuple(output_size),
                      max_pixel_radius)

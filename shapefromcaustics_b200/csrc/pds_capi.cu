@@ -670,6 +670,47 @@ static int plan_records(const void* ws, size_t ws_bytes, int64_t n, int64_t n_ti
     return PDS_OK;
 }
 
+int pds_splat_inputs_f32(const float* Du, const float* Dv, const float* normal, const float* flux,
+                         const int64_t* channel, int64_t n, float* Ep, float* Mp, int64_t* cp,
+                         float* radius, void* stream) {
+    if (n < 0) return fail(PDS_ERR_INVALID_ARGUMENT, "negative photon count");
+    if (n > 0 && (!Du || !Dv || !normal || !flux || !channel || !Ep || !Mp || !cp || !radius))
+        return fail(PDS_ERR_INVALID_ARGUMENT, "null photon array");
+    pds::BasisArgs a = {};
+    a.Du = Du; a.Dv = Dv; a.normal = normal; a.flux = flux; a.channel = channel; a.n = n;
+    a.Ep = Ep; a.Mp = Mp; a.cp = cp; a.radius = radius;
+    const cudaError_t e = pds::launch_basis(false, a, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "basis_fwd_kernel");
+    return PDS_OK;
+}
+
+int pds_splat_inputs_backward_planned_f32(const float* Du, const float* Dv, const float* normal,
+                                          const float* flux, int64_t n, int64_t C, int64_t H,
+                                          int64_t W, const void* ws, size_t ws_bytes,
+                                          const pds_config* cfg, float* gX, float* gDu, float* gDv,
+                                          float* gN, float* gflux, void* stream) {
+    if (n < 0) return fail(PDS_ERR_INVALID_ARGUMENT, "negative photon count");
+    if (n > 0 && (!Du || !Dv || !normal || !flux))
+        return fail(PDS_ERR_INVALID_ARGUMENT, "null photon array");
+    if (n > 0 && !gX) return fail(PDS_ERR_INVALID_ARGUMENT, "null gradient array");
+    pds_sim sim;
+    int64_t nt;
+    int rc = single_tiles(cfg, C, H, W, &nt, &sim, n);
+    if (rc) return rc;
+    pds::GradRecords rec;
+    rc = plan_records(ws, ws_bytes, n, nt, cfg, &rec);
+    if (rc) return rc;
+    pds::BasisArgs a = {};
+    a.Du = Du; a.Dv = Dv; a.normal = normal; a.flux = flux; a.n = n;
+    a.rec_inv = rec.inv;
+    a.rec_stage = reinterpret_cast<const float4*>(rec.stage);
+    a.rec_counters = rec.counters;
+    a.gX = gX; a.gDu = gDu; a.gDv = gDv; a.gN = gN; a.gflux = gflux;
+    const cudaError_t e = pds::launch_basis(true, a, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "basis_bwd_kernel");
+    return PDS_OK;
+}
+
 int pds_refract_backward_planned_f32(const float* h, int32_t rows, int32_t cols,
                                      const pds_plate* plate, const float* px, const float* py,
                                      const float* flux, int64_t n, int64_t C, int64_t H,

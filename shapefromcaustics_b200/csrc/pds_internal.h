@@ -102,6 +102,22 @@ cudaError_t launch_refract_point(bool backward, const float* h, int H, int W,
                                  const float* gE, const float* gX, const float* gM, float* gh,
                                  cudaStream_t st);
 
+// splat inputs of traced photons (pds_basis.cu); vectors [3][n]
+struct BasisArgs {
+    const float *Du, *Dv, *normal, *flux;
+    int64_t n;
+    // forward
+    const int64_t* channel;
+    float *Ep, *Mp, *radius;
+    int64_t* cp;
+    // backward: the plan's gradient records; gX [2][n], the others may be null (not wanted)
+    const uint32_t* rec_inv;
+    const float4* rec_stage;
+    const uint32_t* rec_counters;
+    float *gDu, *gDv, *gN, *gflux, *gX;
+};
+cudaError_t launch_basis(bool backward, const BasisArgs& a, cudaStream_t st);
+
 // photon source (pds_source.cu)
 cudaError_t launch_source(int32_t rows, int32_t cols, int32_t per_texel, float texel,
                           uint64_t seed, uint64_t offset, int64_t n, float* px, float* py,

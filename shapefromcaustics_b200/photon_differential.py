@@ -36,18 +36,8 @@ class PDS(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_pds):
         Ep, xp, Mp, cp, radius = ctx.saved_tensors
-        if ctx.plan_ws is not None:
-            plan = SplatPlan.__new__(SplatPlan)
-            plan.n = Ep.size(0)
-            plan.C, plan.H, plan.W = ctx.output_size
-            plan.mpr = ctx.max_pixel_radius
-            plan.cfg = ctx.cfg
-            plan.device = Ep.device
-            plan.inputs = (Ep, xp, Mp, cp, radius)
-            plan.ws = ctx.plan_ws
-        else:
-            plan = SplatPlan(Ep, xp, Mp, cp, radius, ctx.output_size, ctx.max_pixel_radius,
-                             config=ctx.cfg)
+        plan = SplatPlan.planned((Ep, xp, Mp, cp, radius), ctx.output_size, ctx.max_pixel_radius,
+                                 ctx.cfg, ctx.plan_ws)
         grad_Ep, grad_xp, grad_Mp = plan.backward(grad_pds.contiguous())
         ctx.plan_ws = None
         return grad_Ep, grad_xp, grad_Mp, None, None, None, None

@@ -127,17 +127,7 @@ class PlateSplat(torch.autograd.Function):
             Ep, xp, Mp, cp, radius = ctx.inputs
         else:
             Ep, xp, Mp, cp, radius = refract_forward(h, px, py, flux, ctx.params)
-        if ctx.plan_ws is not None:
-            plan = SplatPlan.__new__(SplatPlan)
-            plan.n = Ep.numel()
-            plan.C, plan.H, plan.W = ctx.shape
-            plan.mpr = ctx.mpr
-            plan.cfg = ctx.cfg
-            plan.device = h.device
-            plan.inputs = (Ep, xp, Mp, cp, radius)
-            plan.ws = ctx.plan_ws
-        else:
-            plan = SplatPlan(Ep, xp, Mp, cp, radius, ctx.shape, ctx.mpr, config=ctx.cfg)
+        plan = SplatPlan.planned((Ep, xp, Mp, cp, radius), ctx.shape, ctx.mpr, ctx.cfg, ctx.plan_ws)
         # the splat gradients stay in the plan's workspace as records, read there by the
         # refraction backward
         plan.backward(grad_img.contiguous(), records=True)

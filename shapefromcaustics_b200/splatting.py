@@ -82,6 +82,9 @@ def _stream(device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+_cfg_ref = ctypes.byref
+
+
 def _output_size(output_size):
     s = [int(v) for v in output_size]
     if len(s) != 3:
@@ -114,6 +117,22 @@ class SplatPlan:
             check(lib().pds_plan_f32(*(_ptr(t) for t in self.inputs), n, self.C, self.H,
                                      self.W, self.mpr, _ptr(self.ws), self.ws.numel(),
                                      ctypes.byref(self.cfg), _stream(self.device)))
+
+    @classmethod
+    def planned(cls, inputs, output_size, max_pixel_radius, config, ws):
+        """The plan that another object built in the workspace ``ws`` from the same photon
+        tensors (a forward's, for its backward); with ``ws`` None it is built again."""
+        if ws is None:
+            return cls(*inputs, output_size, max_pixel_radius, config=config)
+        plan = cls.__new__(cls)
+        plan.n = inputs[0].size(0)
+        plan.C, plan.H, plan.W = output_size
+        plan.mpr = max_pixel_radius
+        plan.cfg = config
+        plan.device = inputs[0].device
+        plan.inputs = inputs
+        plan.ws = ws
+        return plan
 
     def forward(self, out=None):
         if out is None:
