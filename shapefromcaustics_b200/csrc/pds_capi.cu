@@ -275,6 +275,7 @@ int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     a.chunk_tile = b.chunk_tile;
     a.fused = fused ? 1 : 0;
     pds::plan_shape(ph.n, r.n_buckets, &a.window, &a.range);
+    a.window_tiles = pds::plan_window_tiles(a.window, r.cfg.class_bits);
     e = pds::launch_plan_count(a, s);
     if (e != cudaSuccess) return cuda_fail(e, "plan count pass");
     if (!fused) {

@@ -218,9 +218,11 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
             }
         }
     } else {
-        zero_window(hist, a.window);
+        zero_window(hist, a.window + a.window_tiles);
     }
     __syncthreads();
+    // the window's tiles' largest radii (kb0 is a tile's first bucket)
+    uint32_t* radii = hist + a.window;
     uint32_t c_tile = 0, c_inv = 0;
     const int64_t* __restrict__ cp = a.ph.cp;
     const float* __restrict__ X = a.ph.X;
@@ -310,10 +312,12 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
             const uint32_t j = key - kb0;
             if (j < uint32_t(a.window)) atomicAdd(hist + j, 1u);
             else atomicAdd(a.counts + key, 1u);
-            // the tile's largest box radius (the backward stages only the tile's pixels within
-            // it): an atomic only where the photon's radius exceeds the value seen (a stale,
-            // lower value only costs a redundant atomic; the value only grows)
+            // the tile's largest box radius (the backward stages, and the forward flushes, only
+            // the tile's pixels within it), kept per CTA like the histogram: an atomic only
+            // where the photon's radius exceeds the value seen (a stale, lower value only costs
+            // a redundant atomic; the value only grows)
             uint32_t* tr = a.tile_r + (key >> a.cfg.class_bits);
+            if (j < uint32_t(a.window) && a.window_tiles) tr = radii + (j >> a.cfg.class_bits);
             if (uint32_t(rmax) > *tr) atomicMax(tr, uint32_t(rmax));
         }
         // wide photons: appended to the wide list (one atomic per warp)
@@ -339,6 +343,10 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
         const uint32_t c = hist[j];
         mine[j] = c;
         if (c) atomicAdd(a.counts + kb0 + j, c);
+    }
+    for (int j = threadIdx.x; j < a.window_tiles; j += blockDim.x) {
+        const uint32_t m = radii[j];
+        if (m) atomicMax(a.tile_r + (kb0 >> a.cfg.class_bits) + j, m);
     }
     c_tile = __reduce_add_sync(0xFFFFFFFFu, c_tile);
     c_inv = __reduce_add_sync(0xFFFFFFFFu, c_inv);
@@ -502,6 +510,14 @@ bool plan_fused(int64_t nb) { return nb <= kFusedBuckets; }
 
 int64_t bucket_scan_parts(int64_t nb) { return (nb + kScanItems - 1) / kScanItems; }
 
+// Tiles of a window whose radii the count pass keeps in shared memory after the histogram (with
+// global atomics, the first photons of every CTA all met on a few tiles: 262144 photons of a plate
+// 37 us, 11 us this way): all of them, or none where the two do not fit together (no class bits).
+int32_t plan_window_tiles(int32_t window, int32_t class_bits) {
+    const int64_t tiles = (int64_t(window) + (int64_t(1) << class_bits) - 1) >> class_bits;
+    return size_t(window + tiles) * 4 <= kMaxDynamicSmem ? int32_t(tiles) : 0;
+}
+
 // Window and photons per CTA of the two plan passes: the window holds a simulation's buckets
 // where it can (at most kMaxWindow); as many CTAs per SM as the window's shared memory allows,
 // at most kPlanMaxCtas in all (the size of the kept histograms), and the photons are split
@@ -527,10 +543,11 @@ int64_t plan_hist_entries(int64_t n, int64_t nb) {
 template <bool PLACE>
 cudaError_t launch_pass(const PlanArgs& a, cudaStream_t st) {
     if (a.ph.n <= 0) return cudaSuccess;
-    const cudaError_t e = allow_smem<plan_pass_kernel<PLACE>>(size_t(a.window) * 4);
+    const size_t smem = size_t(a.window + (PLACE ? 0 : a.window_tiles)) * 4;
+    const cudaError_t e = allow_smem<plan_pass_kernel<PLACE>>(smem);
     if (e != cudaSuccess) return e;
-    plan_pass_kernel<PLACE><<<unsigned((a.ph.n + a.range - 1) / a.range), kPlanKernelThreads,
-                              size_t(a.window) * 4, st>>>(a);
+    plan_pass_kernel<PLACE><<<unsigned((a.ph.n + a.range - 1) / a.range), kPlanKernelThreads, smem,
+                              st>>>(a);
     return cudaGetLastError();
 }
 

@@ -39,6 +39,7 @@ struct PlanArgs {
                          // tile-path photons (count pass); zeroed by the caller
     int64_t range;       // photons per CTA (plan_shape)
     int32_t window;      // buckets of each CTA's shared histogram (plan_shape)
+    int32_t window_tiles;  // tiles of the window whose radii are kept there too (count pass)
     int32_t fused;       // 1: the place pass scans the counts itself (plan_fused)
 };
 
@@ -78,6 +79,7 @@ struct TileArgs {
 
 bool plan_fused(int64_t nb);
 int64_t bucket_scan_parts(int64_t nb);
+int32_t plan_window_tiles(int32_t window, int32_t class_bits);
 void plan_shape(int64_t n, int64_t nb, int32_t* window, int64_t* range);
 int64_t plan_hist_entries(int64_t n, int64_t nb);
 cudaError_t launch_plan_count(const PlanArgs& a, cudaStream_t st);
