@@ -258,6 +258,11 @@ int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     if (e != cudaSuccess) return cuda_fail(e, "plan: counter reset");
     pds::PlanArgs a;
     a.ph = ph;
+    a.Y = ph.n > 0 ? ph.X + ph.n : nullptr;
+    a.M01 = ph.n > 0 ? ph.M + ph.n : nullptr;
+    a.M10 = ph.n > 0 ? ph.M + 3 * ph.n : nullptr;
+    a.M11 = ph.n > 0 ? ph.M + 4 * ph.n : nullptr;
+    a.tile_shift = r.cfg.tile == 64 ? 6 : (r.cfg.tile == 32 ? 5 : 4);
     a.sims = st;
     a.mpr = mpr;
     a.cfg = r.cfg;

@@ -87,62 +87,115 @@ __device__ __forceinline__ void zero_window(uint32_t* hist, int window) {
     for (int j = threadIdx.x; j < window; j += blockDim.x) hist[j] = 0u;
 }
 
+// What binning needs of a simulation, kept by each thread along its photons.
+struct SimGeo {
+    int32_t W, H, tiles_x, tiles_y, channels;
+    uint32_t tile_base;
+    float sx, sy;     // 2 / W, 2 / H
+    double s2w, s2h;  // the same, for the corner offsets
+    uint32_t end;     // first photon after the simulation's
+};
+
+__device__ __forceinline__ SimGeo load_geo(const SimTable& t, int s) {
+    const pds_sim sim = load_sim(t, s);
+    SimGeo g;
+    g.W = sim.width;
+    g.H = sim.height;
+    g.tiles_x = sim.tiles_x;
+    g.tiles_y = sim.tiles_y;
+    g.channels = sim.channels;
+    g.tile_base = uint32_t(sim.tile_base);
+    g.s2w = corner_step(sim.width);
+    g.s2h = corner_step(sim.height);
+    g.sx = float(g.s2w);
+    g.sy = float(g.s2h);
+    g.end = uint32_t(min(sim_end(t, s), int64_t(UINT32_MAX)));
+    return g;
+}
+
+// One photon's inputs.
+struct PhotonIn {
+    int64_t ch;
+    float x, y, rad, e, m00, m01, m10, m11;
+};
+
+template <bool PLACE>
+__device__ __forceinline__ PhotonIn load_photon(const PlanArgs& a, uint32_t i) {
+    PhotonIn p;
+    p.ch = __ldg(a.ph.cp + i);
+    p.x = __ldg(a.ph.X + i);
+    p.y = __ldg(a.Y + i);
+    p.rad = __ldg(a.ph.R + i);
+    p.m00 = __ldg(a.ph.M + i);
+    p.m01 = __ldg(a.M01 + i);
+    p.m10 = __ldg(a.M10 + i);
+    p.m11 = __ldg(a.M11 + i);
+    p.e = PLACE ? __ldg(a.ph.E + i) : 0.f;
+    return p;
+}
+
 // The bucket of one photon (key_invalid, key_big, or (tile << cb) | class), for the tile path
 // its box radius max(rx, ry) in rmax, and when PLACE its 32-byte record. Both passes run it on
-// the same inputs, so they agree on every key.
+// the same inputs, so they agree on every key. The passes are bound by instruction issue, so
+// all but the reference's double-precision footprint is 32-bit integer and float work.
 template <bool PLACE>
-__device__ __forceinline__ uint32_t bin_photon(const PlanArgs& a, const pds_sim& sim, double s2w,
-                                               double s2h, int64_t ch, float x, float y,
-                                               float rad, float e, float m00, float m01,
-                                               float m10, float m11, Rec& r, int& rmax) {
-    const int T = a.cfg.tile, A = a.cfg.apron, cb = a.cfg.class_bits;
+__device__ __forceinline__ uint32_t bin_photon(const PlanArgs& a, const SimGeo& g,
+                                               const PhotonIn& p, Rec& r, int& rmax) {
+    const int A = a.cfg.apron, cb = a.cfg.class_bits;
     const uint32_t cls_max = (1u << cb) - 1u;
-    if (!(ch >= 0 && ch < sim.channels)) return a.key_invalid;
-    const Footprint f = make_footprint(x, y, rad, sim.height, sim.width, a.mpr);
-    int32_t x0, x1, y0, y1;
-    if (!clip_box(f, sim.height, sim.width, x0, x1, y0, y1)) return a.key_invalid;
-    if (f.rx > A || f.ry > A) return a.key_big;
+    if (uint64_t(p.ch) >= uint64_t(g.channels)) return a.key_invalid;  // (negative ones too)
+    const Footprint f = make_footprint(p.x, p.y, p.rad, g.H, g.W, a.mpr);
+    if (f.rx < 0 || f.ry < 0) return a.key_invalid;
+    // the clipped box; the centre is held within reach of 32 bits, far outside any image (an
+    // empty box stays empty: tile-path radii are at most A), and wider footprints are clipped
+    // in 64 bits
+    if (f.rx > A || f.ry > A) {
+        int32_t x0, x1, y0, y1;
+        return clip_box(f, g.H, g.W, x0, x1, y0, y1) ? a.key_big : a.key_invalid;
+    }
+    const int pxc = min(max(f.px_c, -65536), 131072), pyc = min(max(f.py_c, -65536), 131072);
+    const int x0 = max(pxc - f.rx, 0), x1 = min(pxc + f.rx, g.W - 1);
+    const int y0 = max(pyc - f.ry, 0), y1 = min(pyc + f.ry, g.H - 1);
+    if (x0 > x1 || y0 > y1) return a.key_invalid;
     rmax = max(f.rx, f.ry);
-    const int pcx = min(max(f.px_c, 0), sim.width - 1);
-    const int pcy = min(max(f.py_c, 0), sim.height - 1);
     // the tile edge is a power of two (16, 32 or 64, checked by the configuration), so the
     // tile of a (non-negative) centre pixel is a shift, not an integer division
-    const int tsh = __ffs(T) - 1;
-    const int tx = pcx >> tsh, ty = pcy >> tsh;
-    const uint32_t tile = uint32_t(sim.tile_base) +
-                          uint32_t((int32_t(ch) * sim.tiles_y + ty) * sim.tiles_x + tx);
-    const float dy0 = corner_offset_step(f.py_c, s2h, y);
-    uint32_t cls = min(uint32_t(max(f.rx, f.ry)), cls_max);
+    const int tx = min(max(pxc, 0), g.W - 1) >> a.tile_shift;
+    const int ty = min(max(pyc, 0), g.H - 1) >> a.tile_shift;
+    const uint32_t tile = g.tile_base + uint32_t((int32_t(p.ch) * g.tiles_y + ty) * g.tiles_x + tx);
+    const float dy0 = corner_offset_step(f.py_c, g.s2h, p.y);
+    uint32_t cls = min(uint32_t(rmax), cls_max);
     if (cb == kRowClassBits) {
         // the row walk's classes: rows and row width inside the box
-        cls = f.ellipse_all ? plan_row_class(m00, m01, m10, m11, dy0, sim.width, sim.height, f.rx,
-                                             x0 - f.px_c, x1 - f.px_c, y0 - f.py_c, y1 - f.py_c)
+        cls = f.ellipse_all ? plan_row_class(p.m00, p.m01, p.m10, p.m11, dy0, g.W, g.H, f.rx,
+                                             x0 - pxc, x1 - pxc, y0 - pyc, y1 - pyc)
                             : cls_max;
     } else if (a.cfg.band) {
         // photons of a warp then have similar trip counts of the band walk: classes of 1/k octave
         // of its pixels, k = 1, 2, 3 for up to 3, 4 and 5 class bits
-        const float sx = float(s2w), sy = float(s2h);  // 2 / W, 2 / H
         int area = (2 * f.rx + 1) * (2 * f.ry + 1);
         if (f.ellipse_all)
-            area = 2 * band_steps(m00 * sx, m01 * sy, m10 * sx, m11 * sy,
-                                  dy0 * (0.5f * float(sim.height)), f.rx, f.ry);
-        // floor(k log2 area) = floor(log2 area^k), exactly
+            area = 2 * band_steps(p.m00 * g.sx, p.m01 * g.sy, p.m10 * g.sx, p.m11 * g.sy,
+                                  dy0 * (0.5f * float(g.H)), f.rx, f.ry);
+        // floor(k log2 area), from the exponent of area^k in float
         const int k = cb <= 3 ? 1 : cb - 2;
-        const uint64_t a1 = uint64_t(max(area, 1));
-        const uint64_t ak = k == 1 ? a1 : (k == 2 ? a1 * a1 : a1 * a1 * a1);
-        const int lg = 63 - __clzll(ak);
+        const float a1 = float(max(area, 1));
+        const float ak = k == 1 ? a1 : (k == 2 ? a1 * a1 : a1 * a1 * a1);
+        const int lg = (__float_as_int(ak) >> 23) - 127;
         cls = min(uint32_t(max(lg - k, 0)), cls_max);
     }
     if (PLACE) {
-        const uint32_t flags = (f.ellipse_all ? kFlagEllipseAll : 0u) | (e > 0.f ? 0u : kFlagFwdSkip);
-        r.dx0 = corner_offset_step(f.px_c, s2w, x);
+        const uint32_t flags =
+            (f.ellipse_all ? kFlagEllipseAll : 0u) | (p.e > 0.f ? 0u : kFlagFwdSkip);
+        r.dx0 = corner_offset_step(f.px_c, g.s2w, p.x);
         r.dy0 = dy0;
-        r.m00 = m00;
-        r.m01 = m01;
-        r.m10 = m10;
-        r.m11 = m11;
-        r.e = e;
-        r.packed = pack_rec(f.px_c - (tx * T - A), f.py_c - (ty * T - A), f.rx, f.ry, flags);
+        r.m00 = p.m00;
+        r.m01 = p.m01;
+        r.m10 = p.m10;
+        r.m11 = p.m11;
+        r.e = p.e;
+        r.packed = pack_rec(pxc - ((tx << a.tile_shift) - A), pyc - ((ty << a.tile_shift) - A), f.rx,
+                            f.ry, flags);
     }
     return (tile << cb) | cls;
 }
@@ -224,67 +277,25 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
     // the window's tiles' largest radii (kb0 is a tile's first bucket)
     uint32_t* radii = hist + a.window;
     uint32_t c_tile = 0, c_inv = 0;
-    const int64_t* __restrict__ cp = a.ph.cp;
-    const float* __restrict__ X = a.ph.X;
-    const float* __restrict__ R = a.ph.R;
-    const float* __restrict__ E = a.ph.E;
-    const float* __restrict__ M = a.ph.M;
     // The thread's simulation is followed along its photons (contiguous per simulation) rather
     // than searched per photon: one table load when a simulation boundary is crossed.
-    int sidx = find_sim_of_photon(a.sims, min(r0 + int64_t(threadIdx.x), n - 1));
-    pds_sim sim = load_sim(a.sims, sidx);
-    int64_t next_begin = sim_end(a.sims, sidx);
-    // the pixel pitch in normalised coordinates (2 / W, 2 / H) of the thread's simulation,
-    // kept across photons by the count pass (24% faster on 2^23 photons); the place pass, one
-    // spilled register short, divides per photon instead (8% faster that way)
-    double s2w = 0.0, s2h = 0.0;
-    if (!PLACE) {
-        s2w = corner_step(sim.width);
-        s2h = corner_step(sim.height);
-    }
+    const uint32_t end = uint32_t(r1);
+    uint32_t i = uint32_t(r0) + threadIdx.x;
+    int sidx = find_sim_of_photon(a.sims, min(int64_t(i), n - 1));
+    SimGeo geo = load_geo(a.sims, sidx);
+    PhotonIn next = {};
+    if (i < end) next = load_photon<PLACE>(a, i);
     // whole warps step together (the wide list's ballot needs every lane)
-    int64_t nch = 0;
-    float nx = 0.f, ny = 0.f, nrad = 0.f, ne = 0.f, n00 = 0.f, n01 = 0.f, n10 = 0.f, n11 = 0.f;
-    {
-        const int64_t i = r0 + threadIdx.x;
-        if (i < r1) {
-            nch = __ldg(cp + i); nx = __ldg(X + i); ny = __ldg(X + n + i); nrad = __ldg(R + i);
-            n00 = __ldg(M + i); n01 = __ldg(M + n + i);
-            n10 = __ldg(M + 3 * n + i); n11 = __ldg(M + 4 * n + i);
-            if (PLACE) ne = __ldg(E + i);
-        }
-    }
-    for (int64_t base = r0; base < r1; base += blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        const bool valid = i < r1;
-        const int64_t ch = nch;
-        const float x = nx, y = ny, rad = nrad, e = ne, m00 = n00, m01 = n01, m10 = n10,
-                    m11 = n11;
-        {
-            const int64_t j = i + blockDim.x;
-            if (j < r1) {
-                nch = __ldg(cp + j); nx = __ldg(X + j); ny = __ldg(X + n + j);
-                nrad = __ldg(R + j); n00 = __ldg(M + j);
-                n01 = __ldg(M + n + j); n10 = __ldg(M + 3 * n + j); n11 = __ldg(M + 4 * n + j);
-                if (PLACE) ne = __ldg(E + j);
-            }
-        }
+    for (uint32_t base = uint32_t(r0); base < end; base += blockDim.x, i += blockDim.x) {
+        const bool valid = i < end;
+        const PhotonIn ph = next;
+        if (i + blockDim.x < end) next = load_photon<PLACE>(a, i + blockDim.x);
         uint32_t key = a.key_invalid;
         int rmax = 0;
         Rec r;
         if (valid) {
-            while (i >= next_begin) {  // at most the table's length in all
-                ++sidx;
-                sim = load_sim(a.sims, sidx);
-                next_begin = sim_end(a.sims, sidx);
-                if (!PLACE) {
-                    s2w = corner_step(sim.width);
-                    s2h = corner_step(sim.height);
-                }
-            }
-            key = bin_photon<PLACE>(a, sim, PLACE ? corner_step(sim.width) : s2w,
-                                    PLACE ? corner_step(sim.height) : s2h, ch, x, y, rad, e,
-                                    m00, m01, m10, m11, r, rmax);
+            while (i >= geo.end) geo = load_geo(a.sims, ++sidx);  // at most the table's length in all
+            key = bin_photon<PLACE>(a, geo, ph, r, rmax);
         }
         const bool tile_path = key < a.key_big;
         if (PLACE) {
@@ -328,7 +339,7 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
             wbase = __shfl_sync(0xFFFFFFFFu, wbase, __ffs(wm) - 1);
             if (wide) {
                 const uint32_t k = wbase + __popc(wm & lanemask_lt());
-                a.wide[k] = uint32_t(i);
+                a.wide[k] = i;
                 a.inv[i] = kWideBit | k;
             }
         }

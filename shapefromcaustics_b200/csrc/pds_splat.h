@@ -20,6 +20,8 @@ struct Photons {
 
 struct PlanArgs {
     Photons ph;
+    const float *Y, *M01, *M10, *M11;  // the other rows of ph.X and ph.M
+    int32_t tile_shift;                // log2 of the tile edge
     SimTable sims;
     int32_t mpr;
     Cfg cfg;
