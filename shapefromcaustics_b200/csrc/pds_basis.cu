@@ -68,8 +68,9 @@ __global__ __launch_bounds__(256) void basis_bwd_kernel(BasisArgs a) {
         const bool have = r != kInvalidPos && slot < n;
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
         if (have) {
-            lo = __ldg(a.rec_stage + 2 * slot);
-            hi = __ldg(a.rec_stage + 2 * slot + 1);
+            const Words8 w = load_words8(a.rec_stage + 2 * slot);
+            lo = w.lo;
+            hi = w.hi;
         }
         const float gE = lo.x;
         a.gX[i] = lo.y;

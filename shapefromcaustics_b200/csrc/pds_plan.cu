@@ -306,7 +306,7 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
                 // both passes bin with the same code on the same inputs, so every position is
                 // below the tile-path count; the guard keeps a mismatch inside the arrays
                 if (pos < uint32_t(n)) {
-                    a.srecs[pos] = r;
+                    store_rec(a.srecs + pos, r);
                     a.inv[i] = pos;
                     // the first photon of a work chunk (a multiple of 256 positions)
                     if ((pos & 255u) == 0u && pos % uint32_t(a.cfg.chunk) == 0u)

@@ -168,7 +168,8 @@ __device__ __forceinline__ bool photon_grads(const RefractArgs& a, int64_t i, in
     const uint32_t v = __ldg(a.rec_inv + i);
     const int64_t slot = (v & kWideBit) ? n_tile + int64_t(v & ~kWideBit) : int64_t(v);
     if (v == kInvalidPos || slot >= n) return false;
-    const float4 lo = __ldg(a.rec_stage + 2 * slot), hi = __ldg(a.rec_stage + 2 * slot + 1);
+    const Words8 w = load_words8(a.rec_stage + 2 * slot);
+    const float4 lo = w.lo, hi = w.hi;
     gE = lo.x; gx = lo.y; gy = lo.z; g0 = lo.w;
     g1 = hi.x; g3 = hi.y; g4 = hi.z;
     return true;

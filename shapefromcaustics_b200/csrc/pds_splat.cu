@@ -173,7 +173,7 @@ __device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uin
     const uint32_t lane = threadIdx.x & 31, n = end > begin ? end - begin : 0u;
     float e = 0.f, area = 0.f;
     if (n > 0) {
-        const Rec r = a.srecs[begin + uint32_t((uint64_t(n) * lane) >> 5)];
+        const Rec r = load_rec(a.srecs + (begin + uint32_t((uint64_t(n) * lane) >> 5)));
         e = r.e;
         const float det = fabsf(fmaf(r.m00, r.m11, -r.m01 * r.m10)) * t->ti.sx * t->ti.sy;
         const float box = float((2 * rec_rx(r.packed) + 1) * (2 * rec_ry(r.packed) + 1));
@@ -940,7 +940,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
     forward_chunks(a, acc, [&](TileState& t, uint32_t i, bool valid) {
         bool coop = false;
         if (valid) {
-            const Rec r = a.srecs[i];
+            const Rec r = load_rec(a.srecs + i);
             coop = use_coop(r, a.cfg.coop_r);
             const float peak = count_peak(t, r.e);
             if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
@@ -988,12 +988,20 @@ __device__ __forceinline__ void load_region(float* tg, int sw, const TileState& 
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// WIDE: one 256-bit store. (Not in functions that are called: there this toolkit's ptxas loses the
+// alignment of the eight registers, or crashes.)
+template <bool WIDE>
 __device__ __forceinline__ void store_grad(GradRec* stage, uint32_t rid, float gE, float gx0,
                                            float gx1, float g00, float g01, float g10,
                                            float g11) {
-    float4* d = reinterpret_cast<float4*>(stage + rid);
-    d[0] = make_float4(gE, gx0, gx1, g00);
-    d[1] = make_float4(g01, g10, g11, 0.f);
+    const float4 lo = make_float4(gE, gx0, gx1, g00), hi = make_float4(g01, g10, g11, 0.f);
+    if (WIDE) {
+        store_words8(stage + rid, lo, hi);
+    } else {
+        float4* d = reinterpret_cast<float4*>(stage + rid);
+        d[0] = lo;
+        d[1] = hi;
+    }
 }
 
 // The moments of one photon turned into its gradients. With a = -12/pi E t g (the
@@ -1001,13 +1009,14 @@ __device__ __forceinline__ void store_grad(GradRec* stage, uint32_t rid, float g
 //   S  = sum t^2 g,  Sd = sum t g d,  Sdd = sum t g d d^T  (d the normalised offset)
 // give  dL/dE = 3/pi S,  dL/dx = -M^T (c M Sd),  dL/dM = c M Sdd  with c = -12/pi E
 // (:195-205 summed over the pixels; u = M d).
+template <bool WIDE>
 __device__ __forceinline__ void finish_grad(GradRec* stage, uint32_t rid, float e, float m00,
                                             float m01, float m10, float m11, float sE, float Sx,
                                             float Sy, float Sxx, float Sxy, float Syy) {
     const float c = -kTwelveOverPi * e;
     const float v0 = c * fmaf(m00, Sx, m01 * Sy);
     const float v1 = c * fmaf(m10, Sx, m11 * Sy);
-    store_grad(stage, rid, kThreeOverPi * sE, -fmaf(m00, v0, m10 * v1),
+    store_grad<WIDE>(stage, rid, kThreeOverPi * sE, -fmaf(m00, v0, m10 * v1),
                -fmaf(m01, v0, m11 * v1), c * fmaf(m00, Sxx, m01 * Sxy),
                c * fmaf(m00, Sxy, m01 * Syy), c * fmaf(m10, Sxx, m11 * Sxy),
                c * fmaf(m10, Sxy, m11 * Syy));
@@ -1021,7 +1030,7 @@ __device__ __forceinline__ void finish_rows(GradRec* stage, uint32_t slot, const
     const float Sxx = fmaf(ti.sx * ti.sx, m.B2t,
                            fmaf(2.f * ti.sx * r.dx0, m.B1t, r.dx0 * r.dx0 * m.A0t));
     const float Sxy = fmaf(ti.sx, m.Sxy, r.dx0 * m.Sy);
-    finish_grad(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, m.sE, Sx, m.Sy, Sxx, Sxy, m.Syy);
+    finish_grad<true>(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, m.sE, Sx, m.Sy, Sxx, Sxy, m.Syy);
 }
 
 // One row of a backward gather: n pixels from q, the first at pixel offset k0 (relative to
@@ -1120,7 +1129,7 @@ __device__ __forceinline__ bool gather_band(const Rec& r, const TileInfo& ti, in
     const float Sx = ti.sx * fmaf(p.beta, gr, hsum(GE)), Sy = ti.sy * gr;
     const float Sxx = (ti.sx * ti.sx) * fmaf(p.beta, fmaf(2.f, ger, bgr), hsum(GEE));
     const float Sxy = (ti.sx * ti.sy) * (ger + bgr), Syy = (ti.sy * ti.sy) * grr;
-    finish_grad(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, hsum(SE), Sx, Sy, Sxx, Sxy, Syy);
+    finish_grad<true>(stage, slot, r.e, r.m00, r.m01, r.m10, r.m11, hsum(SE), Sx, Sy, Sxx, Sxy, Syy);
     return true;
 }
 
@@ -1179,7 +1188,7 @@ __device__ __noinline__ void gather_generic(const Rec* rp, TileInfo ti, int sw, 
     }
     const float Sx = fmaf(ti.sx, B1t, r.dx0 * A0t);
     const float Sxx = fmaf(ti.sx * ti.sx, B2, fmaf(2.f * ti.sx * r.dx0, B1t, r.dx0 * r.dx0 * A0t));
-    finish_grad(stage, rid, r.e, r.m00, r.m01, r.m10, r.m11, sE, Sx, Sy, Sxx, Sxy, Syy);
+    finish_grad<false>(stage, rid, r.e, r.m00, r.m01, r.m10, r.m11, sE, Sx, Sy, Sxx, Sxy, Syy);
 }
 
 // Backward gather of one photon by the whole warp (see use_coop): lanes take rows and walk
@@ -1226,7 +1235,7 @@ __device__ __noinline__ void gather_coop(const Rec* rp, TileInfo ti, int sw, con
     if (lane == owner) {
         const float Sx = fmaf(ti.sx, B1t, r.dx0 * A0t);
         const float Sxx = fmaf(ti.sx * ti.sx, B2, fmaf(2.f * ti.sx * r.dx0, B1t, r.dx0 * r.dx0 * A0t));
-        finish_grad(stage, rid, r.e, r.m00, r.m01, r.m10, r.m11, sE, Sx, Sy, Sxx, Sxy, Syy);
+        finish_grad<false>(stage, rid, r.e, r.m00, r.m01, r.m10, r.m11, sE, Sx, Sy, Sxx, Sxy, Syy);
     }
 }
 
@@ -1274,7 +1283,7 @@ __device__ __noinline__ void tail_backward(const TileArgs& a) {
             if (!any) {
                 d.m00 = d.m01 = d.m10 = d.m11 = d.e = 0.f;
             }
-            finish_grad(a.stage, uint32_t(n_tile + w), d.e, d.m00, d.m01, d.m10, d.m11, sE, Sx,
+            finish_grad<false>(a.stage, uint32_t(n_tile + w), d.e, d.m00, d.m01, d.m10, d.m11, sE, Sx,
                         Sy, Sxx, Sxy, Syy);
         }
     }
@@ -1341,7 +1350,7 @@ __global__ __launch_bounds__(NT, MINB) void bwd_tiles_kernel(const __grid_consta
         const int sw = a.cfg.sw;
         bool coop = false;
         if (valid) {
-            const Rec r = a.srecs[i];
+            const Rec r = load_rec(a.srecs + i);
             coop = use_coop(r, a.cfg.coop_r);
             // a photon's gradient record goes to its sorted position
             if (!coop && !(a.cfg.band && gather_band(r, t.ti, sw, tg, i, a.stage)))
@@ -1373,7 +1382,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
         float peak = 0.f;
         bool generic = false, coop = false;
         if (valid) {
-            const Rec r = a.srecs[i];
+            const Rec r = load_rec(a.srecs + i);
             coop = use_coop(r, a.cfg.coop_r);
             if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
                 int pxc, pyc, x0, x1, y0, y1;
@@ -1407,7 +1416,7 @@ __global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(const __grid_constan
         float dy0 = 0.f;
         bool walk = false, generic = false, coop = false;
         if (valid) {
-            const Rec r = a.srecs[i];
+            const Rec r = load_rec(a.srecs + i);
             coop = use_coop(r, a.cfg.coop_r);
             if (!coop) {
                 int pxc, pyc, x0, x1, y0, y1;
@@ -1420,7 +1429,7 @@ __global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(const __grid_constan
         }
         __syncwarp();
         const RowMoments m = gather_rows(g, rows, tg_base, sw, t.ti.sy, dy0);
-        if (walk) finish_rows(a.stage, i, a.srecs[i], t.ti, m);
+        if (walk) finish_rows(a.stage, i, load_rec(a.srecs + i), t.ti, m);
         if (generic) gather_generic(a.srecs + i, t.ti, sw, a.cfg.spans, tg, i, a.stage);
         __syncwarp();
         for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1) {
@@ -1437,13 +1446,13 @@ __global__ __launch_bounds__(NT, MINB) void bwd_rows_kernel(const __grid_constan
 // Photons that touch no pixel get zeros.
 __device__ __forceinline__ void grad_record(const TileArgs& a, int64_t n, int64_t n_tile,
                                             uint32_t v, float4& lo, float4& hi) {
-    const float4* st = reinterpret_cast<const float4*>(a.stage);
     const int64_t slot = (v & kWideBit) ? n_tile + int64_t(v & ~kWideBit) : int64_t(v);
     lo = make_float4(0.f, 0.f, 0.f, 0.f);
     hi = lo;
     if (v != kInvalidPos && slot < n) {
-        lo = st[2 * slot];
-        hi = st[2 * slot + 1];
+        const Words8 w = load_words8(a.stage + slot);
+        lo = w.lo;
+        hi = w.hi;
     }
 }
 
