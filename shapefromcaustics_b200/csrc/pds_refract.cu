@@ -233,15 +233,12 @@ __global__ __launch_bounds__(256, 5) void refract_fwd_kernel(RefractArgs a) {
     }
 }
 
-// Adds d L / d height of one photon to its 4x4 texel patch (x0-1..x0+2, y0-1..y0+2) from the
+// d L / d height of one photon on its 4x4 texel patch (x0-1..x0+2, y0-1..y0+2) from the
 // derivatives c[k] of L with respect to its seven surface scalars: the transposed bilinear
 // stencil for the height (k = 0) and the transposed bilinear and Sobel stencils for the normal
-// scalars (k = 1..6). Patch texels outside the field fold onto the border (replicate padding).
-// add(row, col, value) receives the non-zero patch entries.
-template <class Add>
-__device__ __forceinline__ void scatter_patch(int H, int W, float texel, const Bilin& b,
-                                              const float c[K], Add add) {
-    float patch[4][4];
+// scalars (k = 1..6).
+__device__ __forceinline__ void patch_values(float texel, const Bilin& b, const float c[K],
+                                             float patch[4][4]) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -275,15 +272,33 @@ __device__ __forceinline__ void scatter_patch(int H, int W, float texel, const B
             patch[r][q + 2] -= gny;
         }
     }
+}
+
+// The patch's texels: add(row, col, value) for each; those outside the field fold onto the border
+// (replicate padding).
+template <class Add>
+__device__ __forceinline__ void for_patch(int H, int W, const Bilin& b, const float patch[4][4],
+                                          Add add) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int ii = min(max(b.y0 - 1 + r, 0), H - 1);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int jj = min(max(b.x0 - 1 + q, 0), W - 1);
-            if (patch[r][q] != 0.f) add(ii, jj, patch[r][q]);
+            add(ii, jj, patch[r][q]);
         }
     }
+}
+
+// Adds a photon's patch: add(row, col, value) receives its non-zero entries.
+template <class Add>
+__device__ __forceinline__ void scatter_patch(int H, int W, float texel, const Bilin& b,
+                                              const float c[K], Add add) {
+    float patch[4][4];
+    patch_values(texel, b, c, patch);
+    for_patch(H, W, b, patch, [&](int ii, int jj, float v) {
+        if (v != 0.f) add(ii, jj, v);
+    });
 }
 
 // The height-field gradient of a CTA's photons: where the CTA's photons share a compact patch
@@ -381,6 +396,118 @@ __device__ __forceinline__ void bounds_reset(int* bb) {
     bb[0] = INT_MAX; bb[1] = INT_MIN; bb[2] = INT_MAX; bb[3] = INT_MIN;
 }
 
+// The derivatives c of photon i with respect to its surface scalars and its cell b; false (c = 0)
+// where its gradient is zero.
+template <bool REC>
+__device__ __forceinline__ bool photon_adjoint(const RefractArgs& a, int64_t i, int64_t n_tile,
+                                               float& texel, Bilin& b, float c[K]) {
+    const int64_t n = a.n;
+    const float px = a.px[i], py = a.py[i], flux = a.flux[i];
+    // (the record's load waits for the inverse map's; both are on their way before the texels')
+    float gE = 0.f, gx, gy, g0, g1, g3, g4;
+    const bool touched = !REC || photon_grads(a, i, n_tile, gE, gx, gy, g0, g1, g3, g4);
+    const PlateParams P = photon_params(a, i);
+    texel = P.texel;
+    b = bilin(px, py, P.texel, a.H, a.W);
+    float s[K];
+    surface_scalars(a.h, a.H, a.W, P.texel, b, s);
+    if (REC)
+        return touched && plate_chain_adjoint(s, px, py, P, gx, gy, g0, g1, g3, g4, 4.f * flux * gE, c);
+    return plate_chain_adjoint(s, px, py, P, a.gX[i], a.gX[n + i], a.gM[i], a.gM[n + i],
+                               a.gM[3 * n + i], a.gM[4 * n + i], 4.f * flux * a.gE[i], c);
+}
+
+// The backward on fields of kSpreadTexels texels and more: every photon adds its patch to the
+// field by global reductions, a warp's 32 photons of neighbouring texels at a time; the L2 does
+// them without the compare-and-swap loops (2.2 tries each), zeroing, flushes and barriers of a
+// shared patch region. Reductions on one 32-byte sector take about 27 ns each, so what is left
+// to avoid is many of them at once:
+// - small fields, where every sector takes the reductions of thousands of warps: 64^2 texels
+//   with 256 photons each 74 us with regions, 138 us this way; the lines cross near 110^2;
+// - photons of one texel in a row: where a warp's cells lie in a 2 x 2 block its patches are summed
+//   by shuffles first (photons in texel order, 64 a texel, on 256^2: 1.8 ms without).
+// No loop and CTAs of two warps: the scheduler refills an SM by the warp, and 11 CTAs leave 88
+// registers a thread (2^26 photons of a 1024^2 field: 4.45 ms with regions, 3.81 looping at
+// three CTAs of 256, 3.29 without the loop, 3.07 at six of 128, 2.92 at eleven of 64).
+constexpr int64_t kSpreadTexels = 16384;
+constexpr int kSpreadThreads = 64;
+
+// The patches of a warp whose cells lie in the 2 x 2 block at (x0, y0), summed over the warp: the
+// 5 x 5 texels they cover as 32 values a lane, halved in every exchange, so that lane k is left
+// with texel k's sum and adds it to the field. (Out of line: its registers would be spilled in
+// every photon's sweep.)
+struct Scalars {
+    float c[K];
+};
+__device__ __noinline__ void spread_block(float* gh, int H, int W, bool active, float texel, Bilin b,
+                                          Scalars sc, int x0, int y0) {
+    float patch[4][4], c[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) c[k] = active ? sc.c[k] : 0.f;
+    patch_values(texel, b, c, patch);
+    const bool dx = b.x0 > x0, dy = b.y0 > y0;
+    float v[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+        const int r = k / 5, q = k % 5;
+        const auto at = [&](int pr) {  // the patch's row pr, moved by dx
+            if (pr < 0 || pr > 3) return 0.f;
+            const float moved = q > 0 ? patch[pr][q - 1] : 0.f, own = q < 4 ? patch[pr][q] : 0.f;
+            return dx ? moved : own;
+        };
+        v[k] = k < 25 ? (dy ? at(r - 1) : at(r)) : 0.f;
+    }
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool upper = lane & half;
+#pragma unroll
+        for (int k = 0; k < half; ++k) {
+            const float give = upper ? v[k] : v[k + half], keep = upper ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, half);
+        }
+    }
+    if (lane < 25 && v[0] != 0.f) {
+        const int ii = min(max(y0 - 1 + lane / 5, 0), H - 1);
+        const int jj = min(max(x0 - 1 + lane % 5, 0), W - 1);
+        atomicAdd(gh + int64_t(ii) * W + jj, v[0]);
+    }
+}
+
+template <bool REC>
+__global__ __launch_bounds__(kSpreadThreads, 11) void refract_bwd_spread_kernel(RefractArgs a) {
+    const int64_t n = a.n;
+    // tile-path photons of the plan whose gradient records are read (records mode)
+    const int64_t n_tile = REC ? min(int64_t(__ldg(a.rec_counters)), n) : 0;
+    const int64_t i = int64_t(blockIdx.x) * kSpreadThreads + threadIdx.x;
+    Bilin b = {0, 0, 0.f, 0.f};
+    float c[K], texel = a.P.texel;
+    const bool active = i < n && photon_adjoint<REC>(a, i, n_tile, texel, b, c);
+    // all cells next to the first lane's (which always has a photon), and then in a 2 x 2 block?
+    const int fx = __shfl_sync(0xFFFFFFFFu, b.x0, 0), fy = __shfl_sync(0xFFFFFFFFu, b.y0, 0);
+    bool block = __all_sync(0xFFFFFFFFu, i >= n || (abs(b.x0 - fx) <= 1 && abs(b.y0 - fy) <= 1));
+    int x0 = 0, y0 = 0;
+    if (block) {
+        x0 = __reduce_min_sync(0xFFFFFFFFu, i < n ? b.x0 : fx);
+        y0 = __reduce_min_sync(0xFFFFFFFFu, i < n ? b.y0 : fy);
+        block = __all_sync(0xFFFFFFFFu, i >= n || (b.x0 - x0 <= 1 && b.y0 - y0 <= 1));
+    }
+    if (!block) {
+        if (active)
+            scatter_patch(a.H, a.W, texel, b, c, [&](int ii, int jj, float v) {
+                atomicAdd(a.gh + int64_t(ii) * a.W + jj, v);
+            });
+        return;
+    }
+    Scalars sc;
+#pragma unroll
+    for (int k = 0; k < K; ++k) sc.c[k] = c[k];
+    spread_block(a.gh, a.H, a.W, active, texel, b, sc, x0, y0);
+}
+
+// The backward on smaller fields: CTAs sum their photons' patches in shared memory where these
+// share a compact region.
+//
 // Three CTAs an SM (80 registers): measured 18% faster than the 114-register build at two
 // CTAs an SM (16.8 M photons of a 1024^2 field: 2.24 vs 2.73 ms).
 //
@@ -412,24 +539,7 @@ __global__ __launch_bounds__(256, 3) void refract_bwd_kernel(RefractArgs a) {
         Bilin b = {0, 0, 0.f, 0.f};
         float c[K];
         float texel = a.P.texel;
-        if (active) {
-            const float px = a.px[i], py = a.py[i];
-            const PlateParams P = photon_params(a, i);
-            texel = P.texel;
-            b = bilin(px, py, P.texel, a.H, a.W);
-            float s[K];
-            surface_scalars(a.h, a.H, a.W, P.texel, b, s);
-            if (REC) {
-                float gE, gx, gy, g0, g1, g3, g4;
-                active = photon_grads(a, i, n_tile, gE, gx, gy, g0, g1, g3, g4) &&
-                         plate_chain_adjoint(s, px, py, P, gx, gy, g0, g1, g3, g4,
-                                             4.f * a.flux[i] * gE, c);
-            } else {
-                active = plate_chain_adjoint(s, px, py, P, a.gX[i], a.gX[n + i], a.gM[i],
-                                             a.gM[n + i], a.gM[3 * n + i], a.gM[4 * n + i],
-                                             4.f * a.flux[i] * a.gE[i], c);
-            }
-        }
+        if (active) active = photon_adjoint<REC>(a, i, n_tile, texel, b, c);
         int* bb = bbs[p];
         region_bounds(bb, active, b.x0, b.y0);
         __syncthreads();
@@ -669,7 +779,13 @@ cudaError_t launch_refract(bool backward, const float* h, int H, int W, const pd
     a.rec_stage = rec ? reinterpret_cast<const float4*>(rec->stage) : nullptr;
     a.rec_counters = rec ? rec->counters : nullptr;
     a.gh = gh;
-    if (backward && rec)
+    const bool spread = int64_t(H) * W >= kSpreadTexels;
+    const unsigned sgrid = unsigned((n + kSpreadThreads - 1) / kSpreadThreads);
+    if (backward && spread && rec)
+        refract_bwd_spread_kernel<true><<<sgrid, kSpreadThreads, 0, st>>>(a);
+    else if (backward && spread)
+        refract_bwd_spread_kernel<false><<<sgrid, kSpreadThreads, 0, st>>>(a);
+    else if (backward && rec)
         refract_bwd_kernel<true><<<grid_for<refract_bwd_kernel<true>>(n), 256, 0, st>>>(a);
     else if (backward)
         refract_bwd_kernel<false><<<grid_for<refract_bwd_kernel<false>>(n), 256, 0, st>>>(a);
