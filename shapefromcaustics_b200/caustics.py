@@ -18,7 +18,7 @@ import torch
 from . import photon_differential
 from ._lib import check, lib
 from .photon_differential import PDS
-from .splatting import SplatPlan, _cfg_ref, _ptr, _stream
+from .splatting import SplatPlan, _cfg_ref, _on, _ptr, _stream
 
 __all__ = ["change_of_basis_matrix", "splat_inputs", "splat_photons"]
 
@@ -57,12 +57,11 @@ class _SplatPhotons(torch.autograd.Function):
         Ep, radius = torch.empty_like(flux), torch.empty_like(flux)
         Mp = torch.empty((2, 3, n), dtype=torch.float32, device=dev)
         cp = torch.empty((1, n), dtype=torch.int64, device=dev)
-        with torch.cuda.device(dev):
+        with _on(dev):
             check(lib().pds_splat_inputs_f32(_ptr(Du), _ptr(Dv), _ptr(normal), _ptr(flux),
                                              _ptr(channel), n, _ptr(Ep), _ptr(Mp), _ptr(cp),
                                              _ptr(radius), _stream(dev)))
-        plan = SplatPlan(Ep, xy, Mp, cp, radius, output_size, max_pixel_radius)
-        out = plan.forward()
+        plan, out = SplatPlan.splat((Ep, xy, Mp, cp, radius), output_size, max_pixel_radius)
         ctx.save_for_backward(Du, Dv, normal, flux, xy, channel, Ep, Mp, cp, radius)
         ctx.shape = (plan.C, plan.H, plan.W)
         ctx.mpr = plan.mpr
@@ -87,7 +86,7 @@ class _SplatPhotons(torch.autograd.Function):
         gX = torch.empty_like(xy)
         grads = [torch.empty_like(t) if w else None
                  for t, w in zip((Du, Dv, normal, flux), ctx.needs_input_grad)]
-        with torch.cuda.device(flux.device):
+        with _on(flux.device):
             check(lib().pds_splat_inputs_backward_planned_f32(
                 _ptr(Du), _ptr(Dv), _ptr(normal), _ptr(flux), flux.numel(), *ctx.shape,
                 _ptr(plan.ws), plan.ws.numel(), _cfg_ref(ctx.cfg), _ptr(gX),

@@ -14,7 +14,7 @@ import torch
 
 from . import _lib
 from ._lib import check, lib
-from .splatting import _ptr, _stream
+from .splatting import _on, _ptr, _stream
 
 __all__ = ["LandweberParams", "landweber_update", "reconstruct"]
 
@@ -53,7 +53,7 @@ def landweber_update(d, grad, mask, params, workspace=None):
     if workspace is None or workspace.numel() < nbytes:
         workspace = torch.empty(int(nbytes), dtype=torch.uint8, device=d.device)
     p = params.c_struct()
-    with torch.cuda.device(d.device):
+    with _on(d.device):
         check(lib().pds_landweber_update_f32(_ptr(d), _ptr(grad), _ptr(mask), rows, cols,
                                              ctypes.byref(p), _ptr(workspace), workspace.numel(),
                                              _stream(d.device)))
@@ -81,7 +81,7 @@ def photon_source(H, W, per_texel, texel, seed, offset, device, out=None):
     else:
         px = torch.empty(n, dtype=torch.float32, device=device)
         py = torch.empty(n, dtype=torch.float32, device=device)
-    with torch.cuda.device(px.device):
+    with _on(px.device):
         check(lib().pds_photon_source_f32(H, W, per_texel, float(texel), int(seed) & (2 ** 64 - 1),
                                           int(offset), _ptr(px), _ptr(py), _stream(px.device)))
     return px, py, int(offset) + (n + 1) // 2

@@ -11,7 +11,7 @@ bytes per photon) held between the passes.
 """
 import torch
 
-from .splatting import SplatPlan
+from .splatting import SplatPlan, _check_photons
 
 _keep_plan = True
 
@@ -24,11 +24,11 @@ def set_keep_plan(keep: bool):
 class PDS(torch.autograd.Function):
     @staticmethod
     def forward(ctx, Ep, xp, Mp, cp, radius, output_size, max_pixel_radius):
-        plan = SplatPlan(Ep, xp, Mp, cp, radius, output_size, max_pixel_radius)
-        out = plan.forward()
+        _check_photons(Ep, xp, Mp, cp, radius)
+        plan, out = SplatPlan.splat((Ep, xp, Mp, cp, radius), output_size, max_pixel_radius)
         ctx.save_for_backward(Ep, xp, Mp, cp, radius)
-        ctx.output_size = tuple(int(v) for v in output_size)
-        ctx.max_pixel_radius = int(max_pixel_radius)
+        ctx.output_size = (plan.C, plan.H, plan.W)
+        ctx.max_pixel_radius = plan.mpr
         ctx.plan_ws = plan.ws if _keep_plan else None
         ctx.cfg = plan.cfg
         return out

@@ -19,7 +19,7 @@ import torch
 
 from . import _lib
 from ._lib import check, lib
-from .splatting import SplatPlan, _ptr, _stream
+from .splatting import FlatInputs, SplatPlan, _on, _ptr, _stream
 
 __all__ = ["PlateParams", "plate_params", "refract_forward", "refract_backward", "PlateSplat",
            "PointLight", "point_light", "point_light_source", "refract_point_forward",
@@ -62,7 +62,7 @@ def refract_forward(height, px, py, flux, params, channel=None):
     Mp = torch.empty((2, 3, n), device=dev)
     cp = torch.empty((1, n), dtype=torch.int64, device=dev)
     radius = torch.empty(n, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(_fn("pds_refract_forward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params), _ptr(px),
             _ptr(py), _ptr(flux), _ptr(channel) if channel is not None else None, n, _ptr(Ep),
@@ -70,12 +70,24 @@ def refract_forward(height, px, py, flux, params, channel=None):
     return Ep, xp, Mp, cp, radius
 
 
+def _refract_flat(height, px, py, flux, params):
+    """``refract_forward`` into ``FlatInputs``."""
+    for t, nm in ((height, "height"), (px, "px"), (py, "py"), (flux, "flux")):
+        _check_f32(t, nm)
+    flat = FlatInputs(px.numel(), height.device)
+    with _on(flat.device):
+        check(lib().pds_refract_forward_f32(
+            height.data_ptr(), *height.shape, ctypes.byref(params), _ptr(px), _ptr(py), _ptr(flux),
+            None, flat.n, *flat.ptrs(), _stream(flat.device)))
+    return flat
+
+
 def refract_backward(height, px, py, flux, params, gE, gX, gM, grad_height=None):
     """Adds d L / d height for splat-input gradients (``pds_refract_backward_f32``)."""
     n = px.numel()
     if grad_height is None:
         grad_height = torch.zeros_like(height)
-    with torch.cuda.device(height.device):
+    with _on(height.device):
         check(_fn("pds_refract_backward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params), _ptr(px),
             _ptr(py), _ptr(flux), n, _ptr(gE.contiguous()), _ptr(gX.contiguous()),
@@ -91,7 +103,7 @@ def refract_backward_planned(height, px, py, flux, params, plan, grad_height=Non
     n = px.numel()
     if grad_height is None:
         grad_height = torch.zeros_like(height)
-    with torch.cuda.device(height.device):
+    with _on(height.device):
         check(_fn("pds_refract_backward_planned_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params), _ptr(px),
             _ptr(py), _ptr(flux), n, plan.C, plan.H, plan.W, _ptr(plan.ws), plan.ws.numel(),
@@ -105,29 +117,27 @@ class PlateSplat(torch.autograd.Function):
     @staticmethod
     def forward(ctx, height, px, py, flux, params, output_size, max_pixel_radius, keep_plan=True):
         h = height.detach().contiguous()
-        Ep, xp, Mp, cp, radius = refract_forward(h, px, py, flux, params)
-        plan = SplatPlan(Ep, xp, Mp, cp, radius, output_size, max_pixel_radius)
-        img = plan.forward()
+        inputs = _refract_flat(h, px, py, flux, params)
+        plan, img = SplatPlan.splat(inputs, output_size, max_pixel_radius)
         ctx.save_for_backward(h, px, py, flux)
         ctx.params = params
-        ctx.shape = tuple(int(v) for v in output_size)
-        ctx.mpr = int(max_pixel_radius)
+        ctx.shape = (plan.C, plan.H, plan.W)
+        ctx.mpr = plan.mpr
         # keep_plan: the plan and the refracted splat inputs are kept for the backward (the
         # reference's PDS saves its inputs, model/photon_differential.py:10); otherwise both
         # are recomputed there (less memory: 12 B per photon held instead of about 120 B)
         ctx.plan_ws = plan.ws if keep_plan else None
-        ctx.inputs = (Ep, xp, Mp, cp, radius) if keep_plan else None
+        ctx.inputs = inputs if keep_plan else None
         ctx.cfg = plan.cfg
         return img
 
     @staticmethod
     def backward(ctx, grad_img):
         h, px, py, flux = ctx.saved_tensors
-        if ctx.inputs is not None:
-            Ep, xp, Mp, cp, radius = ctx.inputs
-        else:
-            Ep, xp, Mp, cp, radius = refract_forward(h, px, py, flux, ctx.params)
-        plan = SplatPlan.planned((Ep, xp, Mp, cp, radius), ctx.shape, ctx.mpr, ctx.cfg, ctx.plan_ws)
+        inputs = ctx.inputs
+        if inputs is None:
+            inputs = _refract_flat(h, px, py, flux, ctx.params)
+        plan = SplatPlan.planned(inputs, ctx.shape, ctx.mpr, ctx.cfg, ctx.plan_ws)
         # the splat gradients stay in the plan's workspace as records, read there by the
         # refraction backward
         plan.backward(grad_img.contiguous(), records=True)
@@ -172,7 +182,7 @@ def point_light_source(light, n_directions, device, seed=0, offset=0, coeffs=Non
         _check_f32(coeffs, "coeffs")
         if tuple(coeffs.shape) != (2, int(n_directions)):
             raise RuntimeError("coeffs must be [2, n_directions]")
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(_fn("pds_point_light_source_f32")(
             ctypes.byref(light), int(n_directions), int(seed) & (2 ** 64 - 1), int(offset),
             _ptr(coeffs) if coeffs is not None else None, *(_ptr(t) for t in out), _stream(dev)))
@@ -192,7 +202,7 @@ def refract_point_forward(height, light, params, direction, dtheta, dphi, flux, 
     Mp = torch.empty((2, 3, n), device=dev)
     cp = torch.empty((1, n), dtype=torch.int64, device=dev)
     radius = torch.empty(n, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(_fn("pds_refract_point_forward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params),
             ctypes.byref(light), _ptr(direction), _ptr(dtheta), _ptr(dphi), _ptr(flux),
@@ -207,7 +217,7 @@ def refract_point_backward(height, light, params, direction, dtheta, dphi, flux,
     n = flux.numel()
     if grad_height is None:
         grad_height = torch.zeros_like(height)
-    with torch.cuda.device(height.device):
+    with _on(height.device):
         check(_fn("pds_refract_point_backward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params),
             ctypes.byref(light), _ptr(direction), _ptr(dtheta), _ptr(dphi), _ptr(flux), n,
@@ -296,7 +306,7 @@ class BatchedPlate:
         Mp = torch.empty((2, 3, n), device=dev)
         cp = torch.empty((1, n), dtype=torch.int64, device=dev)
         radius = torch.empty(n, device=dev)
-        with torch.cuda.device(dev):
+        with _on(dev):
             check(_fn("pds_batch_refract_forward_f32")(
                 _ptr(height), height.shape[0], height.shape[1], _ptr(self.plates_dev),
                 _ptr(self.begins_dev), self.n_sims, _ptr(px), _ptr(py), _ptr(flux), None, n,
@@ -325,7 +335,7 @@ class BatchedPlate:
         if grad_height is None:
             grad_height = torch.zeros_like(height)
         sp = self.splat
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(_fn("pds_batch_refract_backward_planned_f32")(
                 _ptr(height), height.shape[0], height.shape[1], _ptr(self.plates_dev),
                 _ptr(self.begins_dev), self.n_sims, _ptr(px), _ptr(py), _ptr(flux),

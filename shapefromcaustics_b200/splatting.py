@@ -14,6 +14,7 @@ device, like the reference's ``th::zeros`` / ``th::empty_like``
 runs many simulations of uneven sizes through one plan and one persistent launch per
 direction.
 """
+import contextlib
 import ctypes
 
 import torch
@@ -47,6 +48,16 @@ def _check_input(t, name):
 
 
 def _check_photons(Ep, xp, Mp, cp, radius, op="pds_forward"):
+    n = Ep.size(0) if Ep.dim() == 1 else -1
+    dev = Ep.device
+    f32 = torch.float32
+    # everything in order in one go; what is not is named below
+    if (Ep.is_cuda and Ep.dtype == xp.dtype == Mp.dtype == radius.dtype == f32 and
+            cp.dtype == torch.int64 and xp.device == Mp.device == cp.device == radius.device == dev
+            and xp.shape == (2, n) and Mp.shape == (2, 3, n) and cp.shape == (1, n) and
+            radius.shape == (n,) and Ep.is_contiguous() and xp.is_contiguous() and
+            Mp.is_contiguous() and cp.is_contiguous() and radius.is_contiguous()):
+        return n
     for t, n in ((Ep, "Ep"), (xp, "xp"), (Mp, "Mp"), (cp, "cp"), (radius, "radius")):
         _check_input(t, n)
     # PhotonDifferentialSplattig.cpp:19-22
@@ -67,19 +78,36 @@ def _check_photons(Ep, xp, Mp, cp, radius, op="pds_forward"):
         if t.dtype != torch.float32:
             raise RuntimeError(
                 f"pds_b200 computes in float32; {nm} has dtype {t.dtype}")
-    dev = Ep.device
     for t in (xp, Mp, cp, radius):
         if t.device != dev:
             raise RuntimeError(f"all inputs of {op} must be on the same device")
     return n
 
 
+# What every call needs of torch, without its wrappers' layers (a call of a few microseconds of
+# device time is bound by its host side; the device guard, the stream object and the pointer
+# objects were a third of it).
+_HERE = contextlib.nullcontext()
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() > 0 else ctypes.c_void_p(0)
+    """The tensor's address as ctypes takes it (null for None and for empty tensors)."""
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream of a CUDA device (with an index, as tensors' devices have)."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+def _on(device):
+    """Context with the device current: nothing to do where it is."""
+    if device.index is not None and torch.cuda.current_device() == device.index:
+        return _HERE
+    return torch.cuda.device(device)
 
 
 _cfg_ref = ctypes.byref
@@ -97,6 +125,25 @@ def _workspace(n, C, H, W, cfg, device):
     return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
+class FlatInputs:
+    """Splat inputs in one buffer (cp, Ep, xp, Mp, radius; 48 bytes a photon), for photons that
+    never leave the library: one allocation instead of five."""
+
+    def __init__(self, n, device):
+        self.n = n
+        self.buf = torch.empty(48 * n, dtype=torch.uint8, device=device)
+        self.device = self.buf.device
+
+    def ptrs(self):
+        """Addresses of Ep, xp, Mp, cp, radius."""
+        p, n = self.buf.data_ptr(), self.n
+        return (p + 8 * n, p + 12 * n, p + 20 * n, p, p + 44 * n) if n else (None,) * 5
+
+
+def _input_ptrs(inputs):
+    return inputs.ptrs() if type(inputs) is FlatInputs else tuple(t.data_ptr() for t in inputs)
+
+
 class SplatPlan:
     """One binning + sort of a photon set, shared by its forward and backward.
 
@@ -112,33 +159,56 @@ class SplatPlan:
         self.cfg = config if config is not None else _default_cfg
         self.device = Ep.device
         self.inputs = (Ep, xp, Mp, cp, radius)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             self.ws = _workspace(n, self.C, self.H, self.W, self.cfg, self.device)
-            check(lib().pds_plan_f32(*(_ptr(t) for t in self.inputs), n, self.C, self.H,
+            check(lib().pds_plan_f32(*_input_ptrs(self.inputs), n, self.C, self.H,
                                      self.W, self.mpr, _ptr(self.ws), self.ws.numel(),
                                      ctypes.byref(self.cfg), _stream(self.device)))
 
     @classmethod
     def planned(cls, inputs, output_size, max_pixel_radius, config, ws):
-        """The plan that another object built in the workspace ``ws`` from the same photon
-        tensors (a forward's, for its backward); with ``ws`` None it is built again."""
-        if ws is None:
-            return cls(*inputs, output_size, max_pixel_radius, config=config)
+        """The plan that another object built in the workspace ``ws`` from the same photons (a
+        forward's, for its backward); with ``ws`` None it is built again."""
         plan = cls.__new__(cls)
-        plan.n = inputs[0].size(0)
+        flat = type(inputs) is FlatInputs
+        plan.n = inputs.n if flat else inputs[0].size(0)
         plan.C, plan.H, plan.W = output_size
         plan.mpr = max_pixel_radius
         plan.cfg = config
-        plan.device = inputs[0].device
+        plan.device = inputs.device if flat else inputs[0].device
         plan.inputs = inputs
         plan.ws = ws
+        if ws is None:
+            plan.ws = _workspace(plan.n, plan.C, plan.H, plan.W, config, plan.device)
+            with _on(plan.device):
+                check(lib().pds_plan_f32(*_input_ptrs(inputs), plan.n, plan.C, plan.H, plan.W,
+                                         plan.mpr, _ptr(plan.ws), plan.ws.numel(),
+                                         ctypes.byref(config), _stream(plan.device)))
         return plan
+
+    @classmethod
+    def splat(cls, inputs, output_size, max_pixel_radius):
+        """(plan, image) of checked photon tensors, or of ``FlatInputs``, in one library call."""
+        plan = cls.__new__(cls)
+        flat = type(inputs) is FlatInputs
+        plan.n = inputs.n if flat else inputs[0].size(0)
+        C, H, W = plan.C, plan.H, plan.W = _output_size(output_size)
+        plan.mpr = int(max_pixel_radius)
+        cfg = plan.cfg = _default_cfg
+        dev = plan.device = inputs.device if flat else inputs[0].device
+        plan.inputs = inputs
+        with _on(dev):
+            out = torch.empty((C, H, W), dtype=torch.float32, device=dev)
+            ws = plan.ws = _workspace(plan.n, C, H, W, cfg, dev)
+            check(lib().pds_forward_f32(*_input_ptrs(inputs), plan.n, C, H, W, plan.mpr, _ptr(out),
+                                        _ptr(ws), ws.numel(), ctypes.byref(cfg), _stream(dev)))
+        return plan, out
 
     def forward(self, out=None):
         if out is None:
             out = torch.empty((self.C, self.H, self.W), dtype=torch.float32, device=self.device)
-        with torch.cuda.device(self.device):
-            check(lib().pds_forward_planned_f32(*(_ptr(t) for t in self.inputs), self.n, self.C,
+        with _on(self.device):
+            check(lib().pds_forward_planned_f32(*_input_ptrs(self.inputs), self.n, self.C,
                                                 self.H, self.W, self.mpr, _ptr(out),
                                                 _ptr(self.ws), self.ws.numel(),
                                                 ctypes.byref(self.cfg), _stream(self.device)))
@@ -151,15 +221,15 @@ class SplatPlan:
         _check_input(grad_pds, "grad_pds")
         if tuple(grad_pds.shape) != (self.C, self.H, self.W) or grad_pds.dtype != torch.float32:
             raise RuntimeError("grad_pds must be a float32 tensor of the forward's output_size")
-        Ep, xp, Mp = self.inputs[:3]
         if records:
             gE = gx = gM = None
         else:
             if out is None:
+                Ep, xp, Mp = self.inputs[:3]
                 out = (torch.empty_like(Ep), torch.empty_like(xp), torch.empty_like(Mp))
             gE, gx, gM = out
-        with torch.cuda.device(self.device):
-            check(lib().pds_backward_planned_f32(_ptr(grad_pds), *(_ptr(t) for t in self.inputs),
+        with _on(self.device):
+            check(lib().pds_backward_planned_f32(_ptr(grad_pds), *_input_ptrs(self.inputs),
                                                  self.n, self.C, self.H, self.W, self.mpr,
                                                  _ptr(gE), _ptr(gx), _ptr(gM), _ptr(self.ws),
                                                  self.ws.numel(), ctypes.byref(self.cfg),
@@ -173,7 +243,7 @@ def pds_forward(Ep, xp, Mp, cp, radius, output_size, max_pixel_radius):
     n = _check_photons(Ep, xp, Mp, cp, radius)
     C, H, W = _output_size(output_size)
     cfg = _default_cfg
-    with torch.cuda.device(Ep.device):
+    with _on(Ep.device):
         out = torch.empty((C, H, W), dtype=Ep.dtype, device=Ep.device)
         ws = _workspace(n, C, H, W, cfg, Ep.device)
         check(lib().pds_forward_f32(_ptr(Ep), _ptr(xp), _ptr(Mp), _ptr(cp), _ptr(radius), n, C,
@@ -191,7 +261,7 @@ def pds_backward(grad_pds, Ep, xp, Mp, cp, radius, max_pixel_radius):
         raise RuntimeError("grad_pds must be a float32 [C,H,W] tensor on the inputs' device")
     C, H, W = (int(v) for v in grad_pds.shape)
     cfg = _default_cfg
-    with torch.cuda.device(Ep.device):
+    with _on(Ep.device):
         gE, gx, gM = torch.empty_like(Ep), torch.empty_like(xp), torch.empty_like(Mp)
         ws = _workspace(n, C, H, W, cfg, Ep.device)
         check(lib().pds_backward_f32(_ptr(grad_pds), _ptr(Ep), _ptr(xp), _ptr(Mp), _ptr(cp),
@@ -252,7 +322,7 @@ class BatchedSplat:
         if n != self.n_total:
             raise RuntimeError(f"batch expects {self.n_total} photons, got {n}")
         self.inputs = (Ep, xp, Mp, cp, radius)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib().pds_batch_plan_f32(*(_ptr(t) for t in self.inputs), *self._common(),
                                            self.mpr, _ptr(self.ws), self.ws.numel(),
                                            ctypes.byref(self.cfg), _stream(self.device)))
@@ -275,7 +345,7 @@ class BatchedSplat:
         if out is None:
             out = torch.empty(self.image_elems, dtype=torch.float32, device=self.device)
         self._check_flat(out, "out")
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib().pds_batch_forward_planned_f32(*(_ptr(t) for t in self.inputs),
                                                       *self._common(), self.image_elems,
                                                       self.mpr, _ptr(out), _ptr(self.ws),
@@ -296,7 +366,7 @@ class BatchedSplat:
             if out is None:
                 out = (torch.empty_like(Ep), torch.empty_like(xp), torch.empty_like(Mp))
             gE, gx, gM = out
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(lib().pds_batch_backward_planned_f32(_ptr(grad_flat),
                                                        *(_ptr(t) for t in self.inputs),
                                                        *self._common(), self.image_elems,
