@@ -241,8 +241,11 @@ pds::SimTable table_dev(const pds_sim* dev, int32_t n) {
 
 // ---- shared implementations -------------------------------------------------------
 
+// image (n photons > 0): the image of image_elems elements that a forward adds to next, cleared by
+// the plan's kernels
 int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, int32_t mpr,
-              const pds_config* cfg, void* ws, size_t ws_bytes, cudaStream_t s) {
+              const pds_config* cfg, void* ws, size_t ws_bytes, cudaStream_t s,
+              float* image = nullptr, int64_t image_elems = 0) {
     Resolved r;
     int rc = resolve(cfg, mpr, n_tiles, ph.n, r);
     if (rc) return rc;
@@ -278,6 +281,8 @@ int plan_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
     a.tile_r = b.tile_r;
     a.start = b.start;
     a.chunk_tile = b.chunk_tile;
+    a.image = image;
+    a.image_elems = image_elems;
     a.fused = fused ? 1 : 0;
     pds::plan_shape(ph.n, r.n_buckets, &a.window, &a.range);
     a.window_tiles = pds::plan_window_tiles(a.window, r.cfg.class_bits);
@@ -326,7 +331,7 @@ int tile_args(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles, 
 
 int forward_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tiles,
                  int64_t image_elems, int32_t mpr, float* out, const pds_config* cfg, void* ws,
-                 size_t ws_bytes, cudaStream_t s) {
+                 size_t ws_bytes, cudaStream_t s, bool cleared = false) {
     if (!out) return fail(PDS_ERR_INVALID_ARGUMENT, "null output image");
     pds::TileArgs a;
     int rc = tile_args(ph, st, n_tiles, mpr, cfg, ws, ws_bytes, a);
@@ -334,7 +339,8 @@ int forward_impl(const pds::Photons& ph, const pds::SimTable& st, int64_t n_tile
     a.out = out;
     a.image_elems = image_elems;
     a.queue = const_cast<uint32_t*>(a.counters) + 4;  // [0..3) plan counters; [4], [5]
-    cudaError_t e = cudaMemsetAsync(out, 0, size_t(image_elems) * sizeof(float), s);
+    cudaError_t e = cudaSuccess;
+    if (!cleared) e = cudaMemsetAsync(out, 0, size_t(image_elems) * sizeof(float), s);
     if (e != cudaSuccess) return cuda_fail(e, "forward: output reset");
     if (ph.n == 0) return PDS_OK;
     e = pds::launch_forward(a, s);
@@ -446,10 +452,20 @@ int pds_backward_planned_f32(const float* G, const float* E, const float* X, con
 int pds_forward_f32(const float* E, const float* X, const float* M, const int64_t* cp,
                     const float* R, int64_t n, int64_t C, int64_t H, int64_t W, int32_t mpr,
                     float* out, void* ws, size_t ws_bytes, const pds_config* cfg, void* stream) {
-    int rc = pds_plan_f32(E, X, M, cp, R, n, C, H, W, mpr, ws, ws_bytes, cfg, stream);
+    int rc = check_photons(E, X, M, cp, R, n);
     if (rc) return rc;
-    return pds_forward_planned_f32(E, X, M, cp, R, n, C, H, W, mpr, out, ws, ws_bytes, cfg,
-                                   stream);
+    pds_sim sim;
+    int64_t nt;
+    rc = single_tiles(cfg, C, H, W, &nt, &sim, n);
+    if (rc) return rc;
+    if (!out) return fail(PDS_ERR_INVALID_ARGUMENT, "null output image");
+    const pds::Photons ph = photons(E, X, M, cp, R, n);
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const bool clear = n > 0;  // (no photons: no plan kernels)
+    rc = plan_impl(ph, table_one(sim), nt, mpr, cfg, ws, ws_bytes, s, clear ? out : nullptr,
+                   C * H * W);
+    if (rc) return rc;
+    return forward_impl(ph, table_one(sim), nt, C * H * W, mpr, out, cfg, ws, ws_bytes, s, clear);
 }
 
 int pds_backward_f32(const float* G, const float* E, const float* X, const float* M,

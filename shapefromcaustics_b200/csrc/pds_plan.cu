@@ -87,6 +87,18 @@ __device__ __forceinline__ void zero_window(uint32_t* hist, int window) {
     for (int j = threadIdx.x; j < window; j += blockDim.x) hist[j] = 0u;
 }
 
+// Clears a buffer by all CTAs of the grid: 16 bytes a store from its first 16-byte boundary on.
+__device__ __forceinline__ void clear_image(float* p, int64_t n) {
+    const int64_t head = min(int64_t((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4, n);
+    const int64_t quads = (n - head) >> 2, tail = head + 4 * quads;
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    float4* q = reinterpret_cast<float4*>(p + head);
+    for (int64_t k = t; k < quads; k += int64_t(gridDim.x) * blockDim.x)
+        q[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < head) p[t] = 0.f;
+    if (tail + t < n) p[tail + t] = 0.f;
+}
+
 // What binning needs of a simulation, kept by each thread along its photons.
 struct SimGeo {
     int32_t W, H, tiles_x, tiles_y, channels;
@@ -272,6 +284,9 @@ __global__ __launch_bounds__(kPlanKernelThreads) void plan_pass_kernel(PlanArgs 
         }
     } else {
         zero_window(hist, a.window + a.window_tiles);
+        // the image that the forward after this plan adds to: its stores ride along with the
+        // pass, a memset of its own is a launch more (3 us of the host, 2 of the device)
+        if (a.image) clear_image(a.image, a.image_elems);
     }
     __syncthreads();
     // the window's tiles' largest radii (kb0 is a tile's first bucket)

@@ -39,6 +39,8 @@ struct PlanArgs {
     Rec* srecs;          // [n] out: records in sorted order (place pass)
     uint32_t* tile_r;    // [tiles] out: the largest box radius max(rx, ry) of each tile's
                          // tile-path photons (count pass); zeroed by the caller
+    float* image;        // the forward's image to clear in the count pass, or null
+    int64_t image_elems;
     int64_t range;       // photons per CTA (plan_shape)
     int32_t window;      // buckets of each CTA's shared histogram (plan_shape)
     int32_t window_tiles;  // tiles of the window whose radii are kept there too (count pass)
