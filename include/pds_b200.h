@@ -358,6 +358,16 @@ int pds_refract_point_backward_f32(const float* height, int32_t rows, int32_t co
                                    const float* grad_Ep, const float* grad_xp,
                                    const float* grad_Mp, float* grad_height, void* stream);
 
+/* pds_refract_point_backward_f32 with the splat-input gradients read from the records that a
+ * backward of the plan in `workspace` left there (as pds_refract_backward_planned_f32). */
+int pds_refract_point_backward_planned_f32(const float* height, int32_t rows, int32_t cols,
+                                           const pds_plate* plate, const pds_point_light* light,
+                                           const float* direction, const float* dtheta,
+                                           const float* dphi, const float* flux, int64_t n_photons,
+                                           int64_t C, int64_t H, int64_t W, const void* workspace,
+                                           size_t workspace_bytes, const pds_config* cfg,
+                                           float* grad_height, void* stream);
+
 /* ---- projected Landweber update of the height field ------------------------------- */
 /* One update of the reference's pixel-basis Landweber loop (shape_from_caustics.py:386-398):
  * d <- VconsHeur(mask * extShrink(d - tau * grad, shrink, lower, upper)), with extShrink

@@ -116,6 +116,11 @@ SIGNATURES = {
     "pds_refract_point_backward_f32": (ctypes.c_int, [_P, _I32, _I32, ctypes.POINTER(PdsPlate),
                                                       ctypes.POINTER(PdsPointLight), _P, _P, _P,
                                                       _P, _I64, _P, _P, _P, _P, _P]),
+    "pds_refract_point_backward_planned_f32": (ctypes.c_int, [_P, _I32, _I32,
+                                                              ctypes.POINTER(PdsPlate),
+                                                              ctypes.POINTER(PdsPointLight), _P,
+                                                              _P, _P, _P, _I64, _I64, _I64, _I64,
+                                                              _P, _SZ, _CFG, _P, _P]),
     "pds_photon_source_f32": (ctypes.c_int, [_I32, _I32, _I32, ctypes.c_float, ctypes.c_uint64,
                                              ctypes.c_uint64, _P, _P, _P]),
     "pds_point_light_source_f32": (ctypes.c_int, [ctypes.POINTER(PdsPointLight), _I64,

@@ -828,6 +828,32 @@ int pds_refract_point_backward_f32(const float* h, int32_t rows, int32_t cols,
     return PDS_OK;
 }
 
+int pds_refract_point_backward_planned_f32(const float* h, int32_t rows, int32_t cols,
+                                           const pds_plate* plate, const pds_point_light* light,
+                                           const float* dir, const float* dth, const float* dph,
+                                           const float* flux, int64_t n, int64_t C, int64_t H,
+                                           int64_t W, const void* ws, size_t ws_bytes,
+                                           const pds_config* cfg, float* gh, void* stream) {
+    int rc = check_plate(h, rows, cols, plate, dir, dir, flux, n);
+    if (rc) return rc;
+    rc = check_point(light, dir, dth, dph, n);
+    if (rc) return rc;
+    if (n > 0 && !gh) return fail(PDS_ERR_INVALID_ARGUMENT, "null gradient array");
+    pds_sim sim;
+    int64_t nt;
+    rc = single_tiles(cfg, C, H, W, &nt, &sim, n);
+    if (rc) return rc;
+    pds::GradRecords rec;
+    rc = plan_records(ws, ws_bytes, n, nt, cfg, &rec);
+    if (rc) return rc;
+    cudaError_t e = pds::launch_refract_point(true, h, rows, cols, *plate, *light, dir, dth, dph,
+                                              flux, nullptr, n, nullptr, nullptr, nullptr, nullptr,
+                                              nullptr, nullptr, nullptr, nullptr, gh,
+                                              static_cast<cudaStream_t>(stream), &rec);
+    if (e != cudaSuccess) return cuda_fail(e, "point_bwd_kernel (records)");
+    return PDS_OK;
+}
+
 int pds_photon_source_f32(int32_t rows, int32_t cols, int32_t per_texel, float texel,
                           uint64_t seed, uint64_t offset, float* px, float* py, void* stream) {
     if (rows < 1 || cols < 1 || per_texel < 1)

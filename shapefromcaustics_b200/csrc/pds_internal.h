@@ -100,7 +100,7 @@ cudaError_t launch_refract_point(bool backward, const float* h, int H, int W,
                                  const float* flux, const int64_t* channel, int64_t n, float* Ep,
                                  float* xp, float* Mp, int64_t* cp, float* radius,
                                  const float* gE, const float* gX, const float* gM, float* gh,
-                                 cudaStream_t st);
+                                 cudaStream_t st, const GradRecords* rec = nullptr);
 
 // splat inputs of traced photons (pds_basis.cu); vectors [3][n]
 struct BasisArgs {

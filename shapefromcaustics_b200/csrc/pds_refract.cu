@@ -161,9 +161,10 @@ struct RefractArgs {
 // The splat gradients of photon i (d L / d Ep, xp, Mp[0,0..1], Mp[1,0..1]) from the plan's
 // gradient records: the values the gradient spread would write, without the spread and its
 // re-read. False for a photon that touches no pixel (zero gradients).
-__device__ __forceinline__ bool photon_grads(const RefractArgs& a, int64_t i, int64_t n_tile,
-                                             float& gE, float& gx, float& gy, float& g0,
-                                             float& g1, float& g3, float& g4) {
+template <class Args>
+__device__ __forceinline__ bool photon_grads(const Args& a, int64_t i, int64_t n_tile, float& gE,
+                                             float& gx, float& gy, float& g0, float& g1, float& g3,
+                                             float& g4) {
     const int64_t n = a.n;
     const uint32_t v = __ldg(a.rec_inv + i);
     const int64_t slot = (v & kWideBit) ? n_tile + int64_t(v & ~kWideBit) : int64_t(v);
@@ -607,8 +608,13 @@ struct PointArgs {
     const float* gE;
     const float* gX;
     const float* gM;
+    const uint32_t* rec_inv;   // non-null: the gradients are a plan's records
+    const float4* rec_stage;
+    const uint32_t* rec_counters;
     float* gh;
 };
+
+constexpr int kPointThreads = 64;
 
 __device__ __forceinline__ Ray photon_ray(const PointArgs& a, int64_t i) {
     Ray r;
@@ -617,75 +623,117 @@ __device__ __forceinline__ Ray photon_ray(const PointArgs& a, int64_t i) {
     return r;
 }
 
-__global__ __launch_bounds__(256) void point_fwd_kernel(PointArgs a) {
+__global__ __launch_bounds__(kPointThreads, 20) void point_fwd_kernel(PointArgs a) {
     const int64_t n = a.n;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const Ray r = photon_ray(a, i);
-        float t, fp, s[K];
-        Bilin b;
-        SurfGeo geo;
-        const bool hit = trace_hit(a.h, a.H, a.W, a.P.texel, a.plane_z, r, t, b, s, geo, fp);
-        float xr = 0.f, yr = 0.f, Dux = 0.f, Duy = 0.f, Dvx = 0.f, Dvy = 0.f;
-        if (hit) {
-            const V3<float> Dt = {a.dth[i], a.dth[n + i], a.dth[2 * n + i]};
-            const V3<float> Dp = {a.dph[i], a.dph[n + i], a.dph[2 * n + i]};
-            point_chain<float>(t, s[1], s[2], s[3], s[4], s[5], s[6], r, Dt, Dp, a.P, xr, yr, Dux,
-                               Duy, Dvx, Dvy);
-        }
-        const float den = Dux * Dvy - Duy * Dvx;
-        const bool good = hit && den != 0.f;
-        const float f = qdiv(2.f, good ? den : 1.f);
-        a.Mp[i] = f * Dvy;
-        a.Mp[n + i] = -f * Dvx;
-        a.Mp[2 * n + i] = 0.f;
-        a.Mp[3 * n + i] = -f * Duy;
-        a.Mp[4 * n + i] = f * Dux;
-        a.Mp[5 * n + i] = 0.f;
-        a.xp[i] = xr;
-        a.xp[n + i] = yr;
-        a.radius[i] = 0.5f * fmaxf(sqrtf(Dux * Dux + Duy * Duy), sqrtf(Dvx * Dvx + Dvy * Dvy));
-        a.Ep[i] = qdiv(4.f * a.flux[i], good ? fabsf(den) : 1.f);
-        const int64_t ch = a.channel ? a.channel[i] : 0;
-        a.cp[i] = good ? ch : -1;
-    }
-}
-
-__global__ __launch_bounds__(256) void point_bwd_kernel(PointArgs a) {
-    const int64_t n = a.n;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const Ray r = photon_ray(a, i);
-        float t, fp, s[K];
-        Bilin b;
-        SurfGeo geo;
-        if (!trace_hit(a.h, a.H, a.W, a.P.texel, a.plane_z, r, t, b, s, geo, fp)) continue;
+    const int64_t i = int64_t(blockIdx.x) * kPointThreads + threadIdx.x;
+    if (i >= n) return;
+    const Ray r = photon_ray(a, i);
+    float t, fp, s[K];
+    Bilin b;
+    SurfGeo geo;
+    const bool hit = trace_hit(a.h, a.H, a.W, a.P.texel, a.plane_z, r, t, b, s, geo, fp);
+    float xr = 0.f, yr = 0.f, Dux = 0.f, Duy = 0.f, Dvx = 0.f, Dvy = 0.f;
+    if (hit) {
         const V3<float> Dt = {a.dth[i], a.dth[n + i], a.dth[2 * n + i]};
         const V3<float> Dp = {a.dph[i], a.dph[n + i], a.dph[2 * n + i]};
-        float tb, Sb[K];
-        if (!point_chain_adjoint(t, s, r, Dt, Dp, a.P, a.gX[i], a.gX[n + i], a.gM[i],
-                                 a.gM[n + i], a.gM[3 * n + i], a.gM[4 * n + i],
-                                 4.f * a.flux[i] * a.gE[i], tb, Sb))
-            continue;
-        // d L / d t along the ray: t itself, and the normal scalars following the hit (their
-        // position derivatives times d); the hit moves with the heights, dt / dh_j = w_j / f'(t)
-        // for the bilinear weights w_j of the hit's cell
-        const float Lt = tb + Sb[1] * (s[3] * r.dx + s[5] * r.dy) +
-                         Sb[2] * (s[4] * r.dx + s[6] * r.dy) +
-                         (Sb[3] * geo.tw_nx + Sb[4] * geo.tw_ny) * r.dy +
-                         (Sb[5] * geo.tw_nx + Sb[6] * geo.tw_ny) * r.dx;
-        float c[K];
-        c[0] = qdiv(Lt, fp);
+        point_chain<float>(t, s[1], s[2], s[3], s[4], s[5], s[6], r, Dt, Dp, a.P, xr, yr, Dux,
+                           Duy, Dvx, Dvy);
+    }
+    const float den = Dux * Dvy - Duy * Dvx;
+    const bool good = hit && den != 0.f;
+    const float f = qdiv(2.f, good ? den : 1.f);
+    a.Mp[i] = f * Dvy;
+    a.Mp[n + i] = -f * Dvx;
+    a.Mp[2 * n + i] = 0.f;
+    a.Mp[3 * n + i] = -f * Duy;
+    a.Mp[4 * n + i] = f * Dux;
+    a.Mp[5 * n + i] = 0.f;
+    a.xp[i] = xr;
+    a.xp[n + i] = yr;
+    a.radius[i] = 0.5f * fmaxf(sqrtf(Dux * Dux + Duy * Duy), sqrtf(Dvx * Dvx + Dvy * Dvy));
+    a.Ep[i] = qdiv(4.f * a.flux[i], good ? fabsf(den) : 1.f);
+    const int64_t ch = a.channel ? a.channel[i] : 0;
+    a.cp[i] = good ? ch : -1;
+}
+
+// Adds a row of a patch (four texels from column x0 - 1 on, none outside the field) by one or two
+// 16-byte reductions: the row is moved to its place in the aligned quads it lies in, the rest of
+// which gets zeros. False where a quad would leave the field's memory.
+__device__ __forceinline__ bool add_row4(float* gh, int64_t texels, int64_t at, const float* v) {
+    float* const row = gh + at;
+    const int s = int(reinterpret_cast<uintptr_t>(row) >> 2) & 3;
+    if (at < s || at - s + (s ? 8 : 4) > texels) return false;
+    float q[8];
 #pragma unroll
-        for (int k = 1; k < K; ++k) c[k] = Sb[k];
-        // traced hits follow the photons' random directions, not the field's texel order:
-        // global adds
-        PatchAcc acc;
-        acc.buf = nullptr;
-        acc.x0 = acc.y0 = acc.rw = 0;
-        acc.gh = a.gh;
-        acc.W = a.W;
-        scatter_patch(a.H, a.W, a.P.texel, b, c, acc);
+    for (int k = 0; k < 8; ++k) {
+        const float v0 = k < 4 ? v[k] : 0.f, v1 = k >= 1 && k < 5 ? v[k - 1] : 0.f;
+        const float v2 = k >= 2 && k < 6 ? v[k - 2] : 0.f, v3 = k >= 3 && k < 7 ? v[k - 3] : 0.f;
+        const float even = s & 2 ? v2 : v0, odd = s & 2 ? v3 : v1;
+        q[k] = s & 1 ? odd : even;
+    }
+    float4* const quad = reinterpret_cast<float4*>(row - s);
+    atomicAdd(quad, make_float4(q[0], q[1], q[2], q[3]));
+    if (s) atomicAdd(quad + 1, make_float4(q[4], q[5], q[6], q[7]));
+    return true;
+}
+
+// The hits follow the photons' random directions, not the field's texel order: a warp's 32 patches
+// rarely share a sector, and every reduction of a warp is 32 sectors' work for the L2. Rows of a
+// patch inside the field go as 16-byte reductions, 7 a photon on average instead of 16 (2^20
+// photons on a 256^2 field: 150 -> 100 us). (The photons of a collimated source come in texel
+// order, where 32 lanes' 4-byte reductions fall on four or five sectors: the kernels above.)
+template <bool REC>
+__global__ __launch_bounds__(kPointThreads, 11) void point_bwd_kernel(PointArgs a) {
+    const int64_t n = a.n;
+    const int64_t i = int64_t(blockIdx.x) * kPointThreads + threadIdx.x;
+    if (i >= n) return;
+    float gE = 0.f, gx, gy, g0, g1, g3, g4;
+    if (REC) {
+        // tile-path photons of the plan whose gradient records are read
+        const int64_t n_tile = min(int64_t(__ldg(a.rec_counters)), n);
+        if (!photon_grads(a, i, n_tile, gE, gx, gy, g0, g1, g3, g4)) return;
+    }
+    const Ray r = photon_ray(a, i);
+    float t, fp, s[K];
+    Bilin b;
+    SurfGeo geo;
+    if (!trace_hit(a.h, a.H, a.W, a.P.texel, a.plane_z, r, t, b, s, geo, fp)) return;
+    const V3<float> Dt = {a.dth[i], a.dth[n + i], a.dth[2 * n + i]};
+    const V3<float> Dp = {a.dph[i], a.dph[n + i], a.dph[2 * n + i]};
+    if (!REC) {
+        gE = a.gE[i]; gx = a.gX[i]; gy = a.gX[n + i];
+        g0 = a.gM[i]; g1 = a.gM[n + i]; g3 = a.gM[3 * n + i]; g4 = a.gM[4 * n + i];
+    }
+    float tb, Sb[K];
+    if (!point_chain_adjoint(t, s, r, Dt, Dp, a.P, gx, gy, g0, g1, g3, g4, 4.f * a.flux[i] * gE, tb,
+                             Sb))
+        return;
+    // d L / d t along the ray: t itself, and the normal scalars following the hit (their
+    // position derivatives times d); the hit moves with the heights, dt / dh_j = w_j / f'(t)
+    // for the bilinear weights w_j of the hit's cell
+    const float Lt = tb + Sb[1] * (s[3] * r.dx + s[5] * r.dy) +
+                     Sb[2] * (s[4] * r.dx + s[6] * r.dy) +
+                     (Sb[3] * geo.tw_nx + Sb[4] * geo.tw_ny) * r.dy +
+                     (Sb[5] * geo.tw_nx + Sb[6] * geo.tw_ny) * r.dx;
+    float c[K];
+    c[0] = qdiv(Lt, fp);
+#pragma unroll
+    for (int k = 1; k < K; ++k) c[k] = Sb[k];
+    float patch[4][4];
+    patch_values(a.P.texel, b, c, patch);
+    const auto add = [&](int ii, int jj, float v) {
+        if (v != 0.f) atomicAdd(a.gh + int64_t(ii) * a.W + jj, v);
+    };
+    if (b.x0 < 1 || b.x0 + 2 >= a.W) {
+        for_patch(a.H, a.W, b, patch, add);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int ii = min(max(b.y0 - 1 + k, 0), a.H - 1);
+        if (!add_row4(a.gh, int64_t(a.H) * a.W, int64_t(ii) * a.W + b.x0 - 1, patch[k]))
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add(ii, b.x0 - 1 + q, patch[k][q]);
     }
 }
 
@@ -709,7 +757,7 @@ cudaError_t launch_refract_point(bool backward, const float* h, int H, int W,
                                  const float* flux, const int64_t* channel, int64_t n, float* Ep,
                                  float* xp, float* Mp, int64_t* cp, float* radius,
                                  const float* gE, const float* gX, const float* gM, float* gh,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, const GradRecords* rec) {
     if (n <= 0) return cudaSuccess;
     PointArgs a;
     a.h = h;
@@ -739,11 +787,17 @@ cudaError_t launch_refract_point(bool backward, const float* h, int H, int W,
     a.gE = gE;
     a.gX = gX;
     a.gM = gM;
+    a.rec_inv = rec ? rec->inv : nullptr;
+    a.rec_stage = rec ? reinterpret_cast<const float4*>(rec->stage) : nullptr;
+    a.rec_counters = rec ? rec->counters : nullptr;
     a.gh = gh;
-    if (backward)
-        point_bwd_kernel<<<grid_for<point_bwd_kernel>(n), 256, 0, st>>>(a);
+    const unsigned int ctas = static_cast<unsigned int>((n + kPointThreads - 1) / kPointThreads);
+    if (backward && rec)
+        point_bwd_kernel<true><<<ctas, kPointThreads, 0, st>>>(a);
+    else if (backward)
+        point_bwd_kernel<false><<<ctas, kPointThreads, 0, st>>>(a);
     else
-        point_fwd_kernel<<<grid_for<point_fwd_kernel>(n), 256, 0, st>>>(a);
+        point_fwd_kernel<<<ctas, kPointThreads, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -82,6 +82,20 @@ def _refract_flat(height, px, py, flux, params):
     return flat
 
 
+def _refract_point_flat(height, light, params, direction, dtheta, dphi, flux):
+    """``refract_point_forward`` into ``FlatInputs``."""
+    for t, nm in ((height, "height"), (direction, "direction"), (dtheta, "dtheta"),
+                  (dphi, "dphi"), (flux, "flux")):
+        _check_f32(t, nm)
+    flat = FlatInputs(flux.numel(), height.device)
+    with _on(flat.device):
+        check(lib().pds_refract_point_forward_f32(
+            height.data_ptr(), *height.shape, ctypes.byref(params), ctypes.byref(light),
+            _ptr(direction), _ptr(dtheta), _ptr(dphi), _ptr(flux), None, flat.n, *flat.ptrs(),
+            _stream(flat.device)))
+    return flat
+
+
 def refract_backward(height, px, py, flux, params, gE, gX, gM, grad_height=None):
     """Adds d L / d height for splat-input gradients (``pds_refract_backward_f32``)."""
     n = px.numel()
@@ -226,34 +240,52 @@ def refract_point_backward(height, light, params, direction, dtheta, dphi, flux,
     return grad_height
 
 
+def _refract_point_backward_planned(height, light, params, direction, dtheta, dphi, flux, plan):
+    """d L / d height from the gradient records that ``plan.backward(g, records=True)`` left in
+    the plan's workspace (``pds_refract_point_backward_planned_f32``)."""
+    grad_height = torch.zeros_like(height)
+    with _on(height.device):
+        check(lib().pds_refract_point_backward_planned_f32(
+            _ptr(height), *height.shape, ctypes.byref(params), ctypes.byref(light),
+            _ptr(direction), _ptr(dtheta), _ptr(dphi), _ptr(flux), flux.numel(), plan.C, plan.H,
+            plan.W, _ptr(plan.ws), plan.ws.numel(), ctypes.byref(plan.cfg), _ptr(grad_height),
+            _stream(height.device)))
+    return grad_height
+
+
 class PointPlateSplat(torch.autograd.Function):
     """Caustic image of the plate lit by a point light (photons traced onto the height-field
     surface); differentiable in the height field. ``photons`` = ``(direction, dtheta, dphi,
-    flux)`` as from ``point_light_source``."""
+    flux)`` as from ``point_light_source``. ``keep_plan`` as in ``PlateSplat``."""
 
     @staticmethod
     def forward(ctx, height, direction, dtheta, dphi, flux, light, params, output_size,
-                max_pixel_radius):
+                max_pixel_radius, keep_plan=True):
         h = height.detach().contiguous()
-        inputs = refract_point_forward(h, light, params, direction, dtheta, dphi, flux)
-        plan = SplatPlan(*inputs, output_size, max_pixel_radius)
-        img = plan.forward()
+        inputs = _refract_point_flat(h, light, params, direction, dtheta, dphi, flux)
+        plan, img = SplatPlan.splat(inputs, output_size, max_pixel_radius)
         ctx.save_for_backward(h, direction, dtheta, dphi, flux)
         ctx.light, ctx.params = light, params
-        ctx.shape = tuple(int(v) for v in output_size)
-        ctx.mpr = int(max_pixel_radius)
+        ctx.shape = (plan.C, plan.H, plan.W)
+        ctx.mpr = plan.mpr
+        ctx.plan_ws = plan.ws if keep_plan else None
+        ctx.inputs = inputs if keep_plan else None
         ctx.cfg = plan.cfg
         return img
 
     @staticmethod
     def backward(ctx, grad_img):
         h, direction, dtheta, dphi, flux = ctx.saved_tensors
-        inputs = refract_point_forward(h, ctx.light, ctx.params, direction, dtheta, dphi, flux)
-        plan = SplatPlan(*inputs, ctx.shape, ctx.mpr, config=ctx.cfg)
-        gE, gX, gM = plan.backward(grad_img.contiguous())
-        gh = refract_point_backward(h, ctx.light, ctx.params, direction, dtheta, dphi, flux, gE,
-                                    gX, gM)
-        return gh, None, None, None, None, None, None, None, None
+        inputs = ctx.inputs
+        if inputs is None:
+            inputs = _refract_point_flat(h, ctx.light, ctx.params, direction, dtheta, dphi, flux)
+        plan = SplatPlan.planned(inputs, ctx.shape, ctx.mpr, ctx.cfg, ctx.plan_ws)
+        plan.backward(grad_img.contiguous(), records=True)
+        gh = _refract_point_backward_planned(h, ctx.light, ctx.params, direction, dtheta, dphi,
+                                             flux, plan)
+        ctx.plan_ws = None
+        ctx.inputs = None
+        return gh, None, None, None, None, None, None, None, None, None
 
 
 class BatchedPlate:
