@@ -48,8 +48,8 @@ sys.path.insert(0, ROOT)
 from shapefromcaustics_b200 import synthetic as S  # noqa: E402
 
 METRIC = "photon fwd+bwd splats/s"
-PHASE_KERNELS = {"forward": "fwd_tiles_kernel + tail_fwd_kernel",
-                 "backward": "bwd_tiles_kernel + tail_bwd_kernel + grad_scatter"}
+PHASE_KERNELS = {"forward": "fwd_tiles_kernel",
+                 "backward": "bwd_tiles_kernel + grad_scatter4_kernel"}
 UNIT = "photons/s"
 MPR = 20
 FP32_SIMT_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # 74.4, nominal (no measured figure)
@@ -270,11 +270,11 @@ def support_pixels(specs, photons, mpr):
 # Measured DRAM traffic per photon of each phase's kernels (ncu dram__bytes_read.sum +
 # dram__bytes_write.sum on the 2^23-photon 1024^2 workload, profiles/*__medium.md), scaled to
 # a workload by its photon count.
-TRAFFIC_PER_PHOTON = {"plan": (309.602816e6 + 11.343360e6 + 349.815040e6 +
-                               255.564032e6) / 2 ** 23,
-                      "forward": (261.056000e6 + 6.905344e6) / 2 ** 23,
-                      "backward": (262.672896e6 + 216.617984e6 + 327.180800e6 +
-                                   263.077888e6) / 2 ** 23}
+TRAFFIC_PER_PHOTON = {"plan": (309.597696e6 + 11.014912e6 + 349.501440e6 +
+                               259.034112e6) / 2 ** 23,
+                      "forward": (260.916992e6 + 5.792768e6) / 2 ** 23,
+                      "backward": (264.973568e6 + 223.695616e6 + 326.829568e6 +
+                                   259.598592e6) / 2 ** 23}
 
 
 # ------------------------------------------------------------------ our arm --------------
@@ -501,10 +501,11 @@ def run_ours(args, rank, world, device):
                      "traffic": sum(TRAFFIC_PER_PHOTON.values()) * n_total}
     achieved = alg[dom] / (ph_ms[dom] / 1e3) / 1e9
     simt = flops[dom] / (ph_ms[dom] / 1e3) / 1e12
-    # plan: plan_pass_kernel<0> (count), bucket_reduce/top/down, plan_pass_kernel<1> (place),
-    # chunk_tile_kernel; forward: fwd_tiles_kernel, tail_fwd_kernel; backward:
-    # bwd_tiles_kernel, tail_bwd_kernel, grad_scatter4_kernel
-    launches_per_step = 6 + 2 + 3
+    # plan: plan_pass_kernel<false> (count), the bucket scan (inside the place pass up to 4608
+    # buckets, bucket_down up to 131072, else bucket_reduce/top/down), plan_pass_kernel<true>
+    # (place); forward: fwd_tiles_kernel; backward: bwd_tiles_kernel, grad_scatter4_kernel
+    buckets = batch.n_tiles << max((tuned or {}).get("class_bits", 5), 0)
+    launches_per_step = 5 + (0 if buckets <= 4608 else 1 if buckets <= 131072 else 3)
     result = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
