@@ -20,9 +20,10 @@
 // point light the hit parameter in place of the height) by a hand-written reverse-mode sweep,
 // and maps them back onto the photon's 4x4 texel patch through the transposed bilinear and
 // Sobel stencils (the chain and its sweeps: pds_chain.cuh, checked on the host against the
-// chain instantiated with forward-mode dual numbers by tests/chain_adjoint_check.cu). A CTA's
-// patches are summed in shared memory where its photons share a compact region of the field,
-// else added with global float atomics.
+// chain instantiated with forward-mode dual numbers by tests/chain_adjoint_check.cu). On large
+// fields every photon adds its patch by global float reductions (summed over its warp first where
+// that lies in a 2 x 2 block of cells); on small ones a CTA's patches are summed in shared memory
+// where its photons share a compact region of the field.
 #include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -435,17 +436,16 @@ constexpr int kSpreadThreads = 64;
 
 // The patches of a warp whose cells lie in the 2 x 2 block at (x0, y0), summed over the warp: the
 // 5 x 5 texels they cover as 32 values a lane, halved in every exchange, so that lane k is left
-// with texel k's sum and adds it to the field. (Out of line: its registers would be spilled in
-// every photon's sweep.)
+// with texel k's sum and adds it to the field. A lane without an active photon gives zeros by
+// selection, not by a factor: its texel may be zero (a lane past the photons of a batch), its patch
+// then no number. (Out of line: its registers would be spilled in every photon's sweep.)
 struct Scalars {
     float c[K];
 };
 __device__ __noinline__ void spread_block(float* gh, int H, int W, bool active, float texel, Bilin b,
                                           Scalars sc, int x0, int y0) {
-    float patch[4][4], c[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) c[k] = active ? sc.c[k] : 0.f;
-    patch_values(texel, b, c, patch);
+    float patch[4][4];
+    patch_values(texel, b, sc.c, patch);
     const bool dx = b.x0 > x0, dy = b.y0 > y0;
     float v[32];
 #pragma unroll
@@ -456,7 +456,7 @@ __device__ __noinline__ void spread_block(float* gh, int H, int W, bool active, 
             const float moved = q > 0 ? patch[pr][q - 1] : 0.f, own = q < 4 ? patch[pr][q] : 0.f;
             return dx ? moved : own;
         };
-        v[k] = k < 25 ? (dy ? at(r - 1) : at(r)) : 0.f;
+        v[k] = active && k < 25 ? (dy ? at(r - 1) : at(r)) : 0.f;
     }
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -484,7 +484,11 @@ __global__ __launch_bounds__(kSpreadThreads, 11) void refract_bwd_spread_kernel(
     Bilin b = {0, 0, 0.f, 0.f};
     float c[K], texel = a.P.texel;
     const bool active = i < n && photon_adjoint<REC>(a, i, n_tile, texel, b, c);
-    // all cells next to the first lane's (which always has a photon), and then in a 2 x 2 block?
+    // nothing to add, or a warp past the last photon (every second one of a last CTA whose photons
+    // fill one warp)
+    if (!__any_sync(0xFFFFFFFFu, active)) return;
+    // all cells next to the first lane's (which has a photon where any lane has), and then in a
+    // 2 x 2 block?
     const int fx = __shfl_sync(0xFFFFFFFFu, b.x0, 0), fy = __shfl_sync(0xFFFFFFFFu, b.y0, 0);
     bool block = __all_sync(0xFFFFFFFFu, i >= n || (abs(b.x0 - fx) <= 1 && abs(b.y0 - fy) <= 1));
     int x0 = 0, y0 = 0;
@@ -502,7 +506,7 @@ __global__ __launch_bounds__(kSpreadThreads, 11) void refract_bwd_spread_kernel(
     }
     Scalars sc;
 #pragma unroll
-    for (int k = 0; k < K; ++k) sc.c[k] = c[k];
+    for (int k = 0; k < K; ++k) sc.c[k] = active ? c[k] : 0.f;
     spread_block(a.gh, a.H, a.W, active, texel, b, sc, x0, y0);
 }
 
