@@ -101,11 +101,13 @@ def refract_backward(height, px, py, flux, params, gE, gX, gM, grad_height=None)
     n = px.numel()
     if grad_height is None:
         grad_height = torch.zeros_like(height)
+    # held until the launch: a copy let go earlier may be given to the next one
+    gE, gX, gM = gE.contiguous(), gX.contiguous(), gM.contiguous()
     with _on(height.device):
         check(_fn("pds_refract_backward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params), _ptr(px),
-            _ptr(py), _ptr(flux), n, _ptr(gE.contiguous()), _ptr(gX.contiguous()),
-            _ptr(gM.contiguous()), _ptr(grad_height), _stream(height.device)))
+            _ptr(py), _ptr(flux), n, _ptr(gE), _ptr(gX), _ptr(gM), _ptr(grad_height),
+            _stream(height.device)))
     return grad_height
 
 
@@ -231,12 +233,12 @@ def refract_point_backward(height, light, params, direction, dtheta, dphi, flux,
     n = flux.numel()
     if grad_height is None:
         grad_height = torch.zeros_like(height)
+    gE, gX, gM = gE.contiguous(), gX.contiguous(), gM.contiguous()  # (held, as above)
     with _on(height.device):
         check(_fn("pds_refract_point_backward_f32")(
             _ptr(height), height.shape[0], height.shape[1], ctypes.byref(params),
             ctypes.byref(light), _ptr(direction), _ptr(dtheta), _ptr(dphi), _ptr(flux), n,
-            _ptr(gE.contiguous()), _ptr(gX.contiguous()), _ptr(gM.contiguous()),
-            _ptr(grad_height), _stream(height.device)))
+            _ptr(gE), _ptr(gX), _ptr(gM), _ptr(grad_height), _stream(height.device)))
     return grad_height
 
 
