@@ -157,9 +157,11 @@ __device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, T
 // add is rounded to half a count, so a pixel's sum is off by about 7e-9 sqrt(c) of it where
 // the photons are spread out; a float sum of c adds is off by 1.4e-8 sqrt(c).
 // - A pixel whose count wraps (photons gathered on few pixels) is seen by the lane that causes
-//   it, from the old count that the add returns. The band walk only marks the segment, without
-//   a branch per pixel, and a marked segment is summed again by redo_segment; the other walks
-//   add the 2^32 counts to the image pixel on the spot (add_pixel).
+//   it, from the old count that the add returns. Every walk only marks the segment, and a marked
+//   segment is summed again from zero by redo_segment, whose adds put each wrap's 2^32 counts into
+//   the image pixel (carry_pixel). (Carried on the spot, the band walk has a branch a step that
+//   its lanes leave apart: 2^22 photons on caustic curves 600 against 402 us. And no walk may
+//   carry where another one marks: what it carried would be added again.)
 // - A photon whose peak reaches 2^31 counts (at least 2^6 typical ones), or any photon where no
 //   power of two in float range fits, is added to the image directly, in float (deposit_direct).
 constexpr int kMaxCountBits = 25;  // counts of a typical peak at most, leaving the 2^6 above
@@ -218,15 +220,21 @@ __device__ __forceinline__ void carry_pixel(const TileArgs& a, const TileState& 
 }
 
 // One pixel of a deposit: s = |u|^2 and the photon's peak in counts; adds peak (1 - s)^2 where
-// s < 1 and in (the reference's value > 0, photon_differentials.cu:105-106).
+// s < 1 and in (the reference's value > 0, photon_differentials.cu:105-106). A wrap is carried on
+// (CARRY: when the segment is summed again) or recorded in wraps.
+template <bool CARRY>
 __device__ __forceinline__ void add_pixel(const TileArgs& a, const TileState& t, uint32_t acc_base,
-                                          uint32_t at, float s, float peak, bool in = true) {
+                                          uint32_t at, float s, float peak, bool& wraps,
+                                          bool in = true) {
     if (!(in && s < 1.f)) return;
     const float d = 1.f - s;
     const uint32_t v = __float2uint_rn((d * peak) * d);
     uint32_t old;
     asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
-    if (old + v < v) carry_pixel(a, t, acc_base, at);
+    if (!CARRY)
+        wraps |= old + v < v;
+    else if (old + v < v)
+        carry_pixel(a, t, acc_base, at);
 }
 
 // Adds the counts v0, v1 to the pixels at shared byte addresses at, at + 4 and counts the wraps.
@@ -242,12 +250,13 @@ __device__ __forceinline__ void add_pair(uint32_t at, uint32_t v0, uint32_t v1, 
 
 // One row of a forward deposit: n pixels from shared byte address `at`, with
 // u = (k M00 sx + b0, k M10 sx + b1) at the k-th pixel.
+template <bool CARRY>
 __device__ __forceinline__ void fwd_row(const TileArgs& a, const TileState& t, uint32_t acc_base,
                                         int n, uint32_t at, float b0, float b1, float a00,
-                                        float a10, float peak) {
+                                        float a10, float peak, bool& wraps) {
     for (int k = 0; k < n; ++k, at += 4u) {
         const float u0 = fmaf(float(k), a00, b0), u1 = fmaf(float(k), a10, b1);
-        add_pixel(a, t, acc_base, at, fmaf(u0, u0, u1 * u1), peak);
+        add_pixel<CARRY>(a, t, acc_base, at, fmaf(u0, u0, u1 * u1), peak, wraps);
     }
 }
 
@@ -431,8 +440,10 @@ __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, i
 // image-half-size ellipse test somewhere in their box (tiny images only) take the per-pixel test
 // path. Out of line: with the band walk on, hardly any photon comes here, and inlined its
 // registers were spilled around every photon's band walk.
-__device__ __noinline__ void deposit_generic(const TileArgs& a, const TileState* tp, const Rec* rp,
+template <bool CARRY>
+__device__ __noinline__ void deposit_generic(const TileArgs& a, TileState* tp, const Rec* rp,
                                              float peak, uint32_t acc_base) {
+    bool wraps = false;
     const Rec r = *rp;
     const TileState& t = *tp;
     const TileInfo ti = t.ti;
@@ -454,18 +465,22 @@ __device__ __noinline__ void deposit_generic(const TileArgs& a, const TileState*
         const uint32_t at = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc + kx0 - ti.ox));
         if (all) {
             const float kf = float(kx0);
-            fwd_row(a, t, acc_base, kx1 - kx0 + 1, at, fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
-                    fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak);
+            fwd_row<CARRY>(a, t, acc_base, kx1 - kx0 + 1, at,
+                           fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
+                           fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak,
+                           wraps);
         } else {
             const float c0 = fmaf(r.m00, r.dx0, r.m01 * dy);
             const float c1 = fmaf(r.m10, r.dx0, r.m11 * dy);
             for (int kx = kx0; kx <= kx1; ++kx) {
                 if (!ellipse_ok(kx, ky, img_wd(ti), img_hd(ti))) continue;
                 const float u0 = fmaf(float(kx), a00, c0), u1 = fmaf(float(kx), a10, c1);
-                add_pixel(a, t, acc_base, at + 4u * uint32_t(kx - kx0), fmaf(u0, u0, u1 * u1), peak);
+                add_pixel<CARRY>(a, t, acc_base, at + 4u * uint32_t(kx - kx0),
+                                 fmaf(u0, u0, u1 * u1), peak, wraps);
             }
         }
     }
+    if (wraps) tp->wrapped = 1u;
 }
 
 // ---- the padded-row walk (walk 4) -------------------------------------------------------
@@ -541,10 +556,11 @@ __device__ __forceinline__ float lds_row(uint32_t a, int c, int w) {
 
 // Forward deposit of the warp's photons by padded rows. rows = 0 for lanes with nothing to
 // walk (their g is not read). Every lane of the warp calls it.
-__device__ __forceinline__ void deposit_rows(const TileArgs& a, const TileState& t, const RowGeo& g,
+__device__ __forceinline__ void deposit_rows(const TileArgs& a, TileState& t, const RowGeo& g,
                                              int rows, float peak, uint32_t acc_base) {
     const int rm = __reduce_max_sync(0xFFFFFFFFu, rows);
     if (rm == 0) return;
+    bool wraps = false;
     const int wm = __reduce_max_sync(0xFFFFFFFFu, rows > 0 ? g.w : 0);
     const float dd = 2.f * g.A;
     for (int j = 0; j < rm; ++j) {
@@ -554,11 +570,12 @@ __device__ __forceinline__ void deposit_rows(const TileArgs& a, const TileState&
         const int xs = row_begin(g, ky, s, d);
         uint32_t at = acc_base + 4u * uint32_t(g.off + ky * a.cfg.sw + xs);
         for (int c = 0; c < wm; ++c, at += 4u) {
-            add_pixel(a, t, acc_base, at, s, peak, c < wl);
+            add_pixel<false>(a, t, acc_base, at, s, peak, wraps, c < wl);
             s += d;
             d += dd;
         }
     }
+    if (wraps) t.wrapped = 1u;
 }
 
 // Backward moments of the warp's photons by padded rows (no rotation: the gathers read).
@@ -647,7 +664,7 @@ __device__ __forceinline__ bool use_coop(const Rec& r, int coop_r) {
 }
 
 // Forward deposit of one photon by the whole warp (see use_coop).
-__device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp, const Rec* rp,
+__device__ __noinline__ void deposit_coop(const TileArgs& a, TileState* tp, const Rec* rp,
                                           uint32_t acc_base) {
     const Rec r = *rp;
     const TileState& t = *tp;
@@ -663,6 +680,7 @@ __device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp
     const float m01sy = r.m01 * ti.sy, m11sy = r.m11 * ti.sy;
     const float c00 = fmaf(r.m00, r.dx0, r.m01 * r.dy0), c10 = fmaf(r.m10, r.dx0, r.m11 * r.dy0);
     const Support sup = make_support(r.m00, r.m01, r.m10, r.m11, true);
+    bool wraps = false;
     int ky0 = y0 - pyc, ky1 = y1 - pyc;
     support_rows(sup, r.dy0, ti.isy, ky0, ky1);
     for (int ky = ky0 + int(threadIdx.x & 31); ky <= ky1; ky += 32) {
@@ -670,11 +688,13 @@ __device__ __noinline__ void deposit_coop(const TileArgs& a, const TileState* tp
         int kx0 = x0 - pxc, kx1 = x1 - pxc;
         if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
         const float kf = float(kx0);
-        fwd_row(a, t, acc_base, kx1 - kx0 + 1,
-                acc_base + 4u * uint32_t((pyc + ky - ti.oy) * a.cfg.sw + (pxc + kx0 - ti.ox)),
-                fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
-                fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak);
+        fwd_row<false>(
+            a, t, acc_base, kx1 - kx0 + 1,
+            acc_base + 4u * uint32_t((pyc + ky - ti.oy) * a.cfg.sw + (pxc + kx0 - ti.ox)),
+            fmaf(kf, a00, fmaf(float(ky), m01sy, c00)), fmaf(kf, a10, fmaf(float(ky), m11sy, c10)),
+            a00, a10, peak, wraps);
     }
+    if (wraps) tp->wrapped = 1u;
 }
 
 // Next chunk of sorted photons for this CTA (the whole warp calls it): a shared work counter
@@ -866,7 +886,7 @@ __device__ __forceinline__ void start_segment(const TileArgs& a, const Segment& 
 // Sums the segment's photons [begin, end) again where a pixel's count has wrapped: from zero, by
 // the walk whose adds carry a wrap on (the photons that went to the image directly stay there).
 // All threads call it, between barriers.
-__device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, const TileState* t,
+__device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, TileState* t,
                                           uint32_t begin, uint32_t end) {
     const int sw = a.cfg.sw;
     for (int k = threadIdx.x; k < sw * sw; k += blockDim.x) acc[k] = 0u;
@@ -875,7 +895,7 @@ __device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, cons
     for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
         const float peak = count_peak(*t, a.srecs[i].e);
         if (!(rec_flags(a.srecs[i].packed) & kFlagFwdSkip) && peak > 0.f)
-            deposit_generic(a, t, a.srecs + i, peak, acc_base);
+            deposit_generic<true>(a, t, a.srecs + i, peak, acc_base);
     }
     __syncthreads();
 }
@@ -947,7 +967,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
                 if (!(peak > 0.f))
                     deposit_direct(a, &t, a.srecs + i);
                 else if (!(a.cfg.band && deposit_band(r, t.ti, a.cfg.sw, peak, acc_base, &t.wrapped)))
-                    deposit_generic(a, &t, a.srecs + i, peak, acc_base);
+                    deposit_generic<false>(a, &t, a.srecs + i, peak, acc_base);
             }
         }
         if (a.cfg.coop_r > 0) {
@@ -1398,7 +1418,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
         }
         __syncwarp();
         deposit_rows(a, t, g, rows, peak, acc_base);
-        if (generic) deposit_generic(a, &t, a.srecs + i, peak, acc_base);
+        if (generic) deposit_generic<false>(a, &t, a.srecs + i, peak, acc_base);
         __syncwarp();
         for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
             deposit_coop(a, &t, a.srecs + __shfl_sync(0xFFFFFFFFu, i, __ffs(cm) - 1), acc_base);
