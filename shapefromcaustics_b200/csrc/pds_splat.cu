@@ -128,7 +128,8 @@ struct TileState {
     int x0, x1, y0, y1;  // pixels its photons can touch: the tile and the plan's largest radius
                          // around it, inside the image
     float scale, unit;   // forward: accumulator counts per unit of energy density (a power of
-                         // two) and its inverse; scale 0: no photon is accumulated
+                         // two) and its inverse; both 0: the accumulator holds floats
+    uint32_t stop;       // forward: end of the photons that are summed together
     uint32_t wrapped;    // forward: non-zero where a pixel's count has wrapped
     uint32_t groups;     // groups of 32 photons that warps have taken
 };
@@ -151,25 +152,47 @@ __device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, T
 // of about eight (measured a warp and SM, random pixels of a tile: 3.1 against 8.9 cycles with
 // the loop around it; all lanes in 32 pixels, as in a focused caustic: 3.1 against 34).
 //
-// The count is a power of two chosen per segment from a sample of its photons (set_scale): with
-// c the photons' mean number of covers of a pixel if they were spread over the tile, 2^32
-// counts hold about 64 c typical peaks (at most all of the segment's photons on one pixel). An
-// add is rounded to half a count, so a pixel's sum is off by about 7e-9 sqrt(c) of it where
-// the photons are spread out; a float sum of c adds is off by 1.4e-8 sqrt(c).
+// What a count is worth is a power of two chosen per segment from a sample of its photons
+// (set_scale): with c the photons' mean number of covers of a pixel if they were spread over the
+// tile, 2^32 counts hold at least 64 c typical peaks (or all of the segment's photons on one
+// pixel). Where the peak of the sample's dimmest photon would then be below 2^kMinCountBits counts,
+// a large segment is summed in pieces (kPiece), which need less room, and what is still missing is
+// taken from the room.
+//
+// An add is rounded to half a count (0.29 in the mean square): at most 2^-20 of its photon's peak,
+// mostly 2^-22 and less, as far as a photon evaluated in float32 is off anyway. Measured against 64
+// bits, and with sums in float instead:
+// - single photons of 0.5 to 4 px: 6.3e-8 of their peak in the mean square, 6.9e-8;
+// - a pixel of 2^24 photons on caustic curves, in chunks of 8192: 3.6e-9 of the peaks that cover
+//   it, 9.1e-9; the whole image 4.9e-8, 3.0e-7;
+// - of 2^22 uniform photons: 4.9e-9, 4.5e-9; the whole image 1.06e-7, 1.01e-7 (mostly the float
+//   sums of the segments in the image).
+//
 // - A pixel whose count wraps (photons gathered on few pixels) is seen by the lane that causes
 //   it, from the old count that the add returns. Every walk only marks the segment, and a marked
 //   segment is summed again from zero by redo_segment, whose adds put each wrap's 2^32 counts into
 //   the image pixel (carry_pixel). (Carried on the spot, the band walk has a branch a step that
 //   its lanes leave apart: 2^22 photons on caustic curves 600 against 402 us. And no walk may
 //   carry where another one marks: what it carried would be added again.)
-// - A photon whose peak reaches 2^31 counts (at least 2^6 typical ones), or any photon where no
-//   power of two in float range fits, is added to the image directly, in float (deposit_direct).
+// - A photon with a peak below 2^kDimBits counts, or of 2^31 and more, is added to the image
+//   directly, in float (deposit_direct).
+// - Where no scale holds the sample's dimmest and brightest photons, or none is in float range,
+//   the whole segment is summed in float, in shared memory (scale 0, deposit_slow): 2^22 photons
+//   with energies over six decades 190 us, all those out of range sent to the image 765.
+// A floor of 23 bits for the dimmest photon instead of 21 makes dense segments wrap (2^22 photons on
+// caustic curves 1043 us against 402), and a quarter of the room does so where photons gather (2^22
+// of them within 2 px: 107 us, with 16 c peaks 191).
 constexpr int kMaxCountBits = 25;  // counts of a typical peak at most, leaving the 2^6 above
+constexpr int kMinCountBits = 21, kDimBits = 19;
 constexpr float kCountLimit = 2147483648.f;
+// Photons of a piece at least (each is added to the image by itself): 2^26 photons on caustic curves
+// in chunks of 8192 4.33 ms, 4.70 in pieces from 512 on, 4.58 to 4.77 from 2048 on (where some wrap),
+// 7.00 in whole segments; 4.31 with the typical peak at 18 bits.
+constexpr uint32_t kPiece = 1024;
 
-// Sets t's scale from at most 32 photons spread evenly over the sorted positions [begin, end),
-// one a lane (the whole warp calls it): the geometric mean of their energies as a power of two,
-// and their mean support pi / |det M|, at most their box.
+// Sets t's stop, and its scale, from at most 32 photons spread evenly over the sorted positions
+// [begin, end), one a lane (the whole warp calls it): the geometric mean, the least and the greatest
+// of their energies as powers of two, and their mean support pi / |det M|, at most their box.
 __device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uint32_t end,
                                           TileState* t) {
     const uint32_t lane = threadIdx.x & 31, n = end > begin ? end - begin : 0u;
@@ -182,7 +205,10 @@ __device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uin
         area = fminf(__fdividef(3.1415927f, det), box);  // (NaN, inf: the box)
     }
     const bool use = e > 0.f && e < __int_as_float(0x7F800000);
-    const int sum = __reduce_add_sync(0xFFFFFFFFu, use ? (__float_as_int(e) >> 23) - 127 : 0);
+    const int lg = (__float_as_int(e) >> 23) - 127;  // floor(log2 e)
+    const int sum = __reduce_add_sync(0xFFFFFFFFu, use ? lg : 0);
+    const int least = __reduce_min_sync(0xFFFFFFFFu, use ? lg : 128);
+    const int most = __reduce_max_sync(0xFFFFFFFFu, use ? lg : -127);
     const int count = __popc(__ballot_sync(0xFFFFFFFFu, use));
     const int area16 = __reduce_add_sync(0xFFFFFFFFu, int(area * 16.f));  // mean area * 512
     if (lane == 0) {
@@ -191,19 +217,23 @@ __device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uin
         const float peaks = 32.f * float(n) * (float(area16) * (1.f / 512.f)) / pixels;
         // ceil(log2) of min(peaks, n): the exponent of the next float below, plus one
         const int room = (__float_as_int(fmaxf(fminf(peaks, float(n)), 1.f) * 0.99999994f) >> 23) - 126;
-        const int bits = min(kMaxCountBits, 30 - room);
-        const int k = count > 0 ? bits - __float2int_rd(float(sum) / float(count)) : 127;
-        const bool fits = k <= 126;
+        const int mean = __float2int_rd(float(sum) / float(max(count, 1)));
+        const int lift = kMinCountBits - least + mean;  // bits of a typical peak that this takes
+        int halvings = 0;
+        while (lift > 30 - room + halvings && (n >> (halvings + 1)) >= kPiece) ++halvings;
+        t->stop = begin + ((n + (1u << halvings) - 1u) >> halvings);
+        const int k = max(min(kMaxCountBits, 30 - room + halvings), lift) - mean;
+        const bool fits = count > 0 && most + k <= 30 && k <= 126;
         t->scale = fits ? __int_as_float((k + 127) << 23) : 0.f;
         t->unit = fits ? __int_as_float((127 - k) << 23) : 0.f;
         t->wrapped = 0u;
     }
 }
 
-// The photon's peak E 3/pi in counts, or 0 for one that goes to the image directly.
+// The photon's peak E 3/pi in counts, or 0 for one that is not counted.
 __device__ __forceinline__ float count_peak(const TileState& t, float e) {
     const float p = (e * kThreeOverPi) * t.scale;
-    return p < kCountLimit ? p : 0.f;
+    return p >= float(1 << kDimBits) && p < kCountLimit ? p : 0.f;
 }
 
 // Adds the 2^32 counts that the pixel at shared byte address `at` has wrapped by to the image.
@@ -221,20 +251,33 @@ __device__ __forceinline__ void carry_pixel(const TileArgs& a, const TileState& 
 
 // One pixel of a deposit: s = |u|^2 and the photon's peak in counts; adds peak (1 - s)^2 where
 // s < 1 and in (the reference's value > 0, photon_differentials.cu:105-106). A wrap is carried on
-// (CARRY: when the segment is summed again) or recorded in wraps.
-template <bool CARRY>
+// (kCarry: when the segment is summed again) or recorded in wraps. kFloat: the peak is E 3/pi and
+// the sum is in float.
+enum AddMode { kMark, kCarry, kFloat };
+__device__ __forceinline__ bool add_count(uint32_t at, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+    return old + v < v;
+}
+__device__ __forceinline__ void add_carry(const TileArgs& a, const TileState& t, uint32_t acc_base,
+                                          uint32_t at, uint32_t v) {
+    if (add_count(at, v)) carry_pixel(a, t, acc_base, at);
+}
+__device__ __forceinline__ void add_shared(uint32_t at, float v) {
+    asm volatile("red.shared.add.f32 [%0], %1;" :: "r"(at), "f"(v) : "memory");
+}
+template <AddMode MODE>
 __device__ __forceinline__ void add_pixel(const TileArgs& a, const TileState& t, uint32_t acc_base,
                                           uint32_t at, float s, float peak, bool& wraps,
                                           bool in = true) {
     if (!(in && s < 1.f)) return;
     const float d = 1.f - s;
+    if (MODE == kFloat) return add_shared(at, (d * peak) * d);
     const uint32_t v = __float2uint_rn((d * peak) * d);
-    uint32_t old;
-    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
-    if (!CARRY)
-        wraps |= old + v < v;
-    else if (old + v < v)
-        carry_pixel(a, t, acc_base, at);
+    if (MODE == kCarry)
+        add_carry(a, t, acc_base, at, v);
+    else
+        wraps |= add_count(at, v);
 }
 
 // Adds the counts v0, v1 to the pixels at shared byte addresses at, at + 4 and counts the wraps.
@@ -250,13 +293,13 @@ __device__ __forceinline__ void add_pair(uint32_t at, uint32_t v0, uint32_t v1, 
 
 // One row of a forward deposit: n pixels from shared byte address `at`, with
 // u = (k M00 sx + b0, k M10 sx + b1) at the k-th pixel.
-template <bool CARRY>
+template <AddMode MODE>
 __device__ __forceinline__ void fwd_row(const TileArgs& a, const TileState& t, uint32_t acc_base,
                                         int n, uint32_t at, float b0, float b1, float a00,
                                         float a10, float peak, bool& wraps) {
     for (int k = 0; k < n; ++k, at += 4u) {
         const float u0 = fmaf(float(k), a00, b0), u1 = fmaf(float(k), a10, b1);
-        add_pixel<CARRY>(a, t, acc_base, at, fmaf(u0, u0, u1 * u1), peak, wraps);
+        add_pixel<MODE>(a, t, acc_base, at, fmaf(u0, u0, u1 * u1), peak, wraps);
     }
 }
 
@@ -273,8 +316,8 @@ __device__ __forceinline__ void rec_box(const Rec& r, const TileInfo& ti, int& p
     y1 = min(pyc + ry, ti.H - 1);
 }
 
-// Forward deposit of one photon straight into the image, in float: the photons that the counts
-// cannot hold (see kCountLimit). Rare, and out of line.
+// Forward deposit of one photon straight into the image, in float: the few photons that the
+// segment's counts cannot hold. Out of line.
 __device__ __noinline__ void deposit_direct(const TileArgs& a, const TileState* tp, const Rec* rp) {
     const Rec r = *rp;
     const TileInfo ti = tp->ti;
@@ -399,10 +442,12 @@ __device__ __forceinline__ float hsum(float2 v) { return v.x + v.y; }
 // Bound by instruction issue. A row change, which some lane of the warp makes on nearly every
 // step, is selected rather than branched to (2^22 photons on caustic curves 403 against 430 us;
 // the backward, with more to select, is faster with the branch).
-__device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, int sw, float peak,
-                                             uint32_t acc_base, uint32_t* wrapped) {
+template <AddMode MODE>
+__device__ __forceinline__ bool deposit_band(const TileArgs& a, TileState& t, const Rec& r,
+                                             float peak, uint32_t acc_base) {
+    const int sw = a.cfg.sw;
     PairWalk p;
-    if (!pair_walk(r, ti, sw, p)) return false;
+    if (!pair_walk(r, t.ti, sw, p)) return false;
     const float2 P = pair(peak);
     float ky = p.ky0;
     PairRow c = pair_row(p, ky);
@@ -418,7 +463,15 @@ __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, i
         const float t1 = rem == p.tail ? 0.f : fmaxf(fmaf(-p.A * e1, e1, c.d), 0.f);
         const float2 T = make_float2(t0, t1);
         const float2 V = __fmul2_rn(__fmul2_rn(T, P), T);
-        add_pair(at, __float2uint_rn(V.x), __float2uint_rn(V.y), wraps);
+        if (MODE == kFloat) {
+            if (V.x > 0.f) add_shared(at, V.x);
+            if (V.y > 0.f) add_shared(at + 4u, V.y);
+        } else if (MODE == kCarry) {
+            add_carry(a, t, acc_base, at, __float2uint_rn(V.x));
+            add_carry(a, t, acc_base, at + 4u, __float2uint_rn(V.y));
+        } else {
+            add_pair(at, __float2uint_rn(V.x), __float2uint_rn(V.y), wraps);
+        }
         // the next pair: two columns on, or the next row's start
         const bool wrap = --rem == 0;
         const PairRow n = pair_row(p, ky + 1.f);
@@ -430,7 +483,7 @@ __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, i
         row = wrap ? row1 : row;
         rem = wrap ? p.npairs : rem;
     }
-    if (wraps) *wrapped = 1u;
+    if (wraps) t.wrapped = 1u;
     return true;
 }
 
@@ -440,7 +493,7 @@ __device__ __forceinline__ bool deposit_band(const Rec& r, const TileInfo& ti, i
 // image-half-size ellipse test somewhere in their box (tiny images only) take the per-pixel test
 // path. Out of line: with the band walk on, hardly any photon comes here, and inlined its
 // registers were spilled around every photon's band walk.
-template <bool CARRY>
+template <AddMode MODE>
 __device__ __noinline__ void deposit_generic(const TileArgs& a, TileState* tp, const Rec* rp,
                                              float peak, uint32_t acc_base) {
     bool wraps = false;
@@ -465,7 +518,7 @@ __device__ __noinline__ void deposit_generic(const TileArgs& a, TileState* tp, c
         const uint32_t at = acc_base + 4u * uint32_t((pyc + ky - ti.oy) * sw + (pxc + kx0 - ti.ox));
         if (all) {
             const float kf = float(kx0);
-            fwd_row<CARRY>(a, t, acc_base, kx1 - kx0 + 1, at,
+            fwd_row<MODE>(a, t, acc_base, kx1 - kx0 + 1, at,
                            fmaf(kf, a00, fmaf(float(ky), m01sy, c00)),
                            fmaf(kf, a10, fmaf(float(ky), m11sy, c10)), a00, a10, peak,
                            wraps);
@@ -475,12 +528,31 @@ __device__ __noinline__ void deposit_generic(const TileArgs& a, TileState* tp, c
             for (int kx = kx0; kx <= kx1; ++kx) {
                 if (!ellipse_ok(kx, ky, img_wd(ti), img_hd(ti))) continue;
                 const float u0 = fmaf(float(kx), a00, c0), u1 = fmaf(float(kx), a10, c1);
-                add_pixel<CARRY>(a, t, acc_base, at + 4u * uint32_t(kx - kx0),
+                add_pixel<MODE>(a, t, acc_base, at + 4u * uint32_t(kx - kx0),
                                  fmaf(u0, u0, u1 * u1), peak, wraps);
             }
         }
     }
     if (wraps) tp->wrapped = 1u;
+}
+
+// Forward deposit of a photon of a segment that is summed again with carries, or in float. Out of
+// line.
+template <AddMode MODE>
+__device__ __noinline__ void deposit_slow(const TileArgs& a, TileState* t, const Rec* rp,
+                                          float peak, uint32_t acc_base) {
+    const Rec r = *rp;
+    if (!((a.cfg.band || a.cfg.rows) && deposit_band<MODE>(a, *t, r, peak, acc_base)))
+        deposit_generic<MODE>(a, t, rp, peak, acc_base);
+}
+
+// Forward deposit of a photon that is not counted.
+__device__ __forceinline__ void deposit_uncounted(const TileArgs& a, TileState* t, const Rec* rp,
+                                                  float e, uint32_t acc_base) {
+    if (t->scale > 0.f)
+        deposit_direct(a, t, rp);
+    else
+        deposit_slow<kFloat>(a, t, rp, e * kThreeOverPi, acc_base);
 }
 
 // ---- the padded-row walk (walk 4) -------------------------------------------------------
@@ -570,7 +642,7 @@ __device__ __forceinline__ void deposit_rows(const TileArgs& a, TileState& t, co
         const int xs = row_begin(g, ky, s, d);
         uint32_t at = acc_base + 4u * uint32_t(g.off + ky * a.cfg.sw + xs);
         for (int c = 0; c < wm; ++c, at += 4u) {
-            add_pixel<false>(a, t, acc_base, at, s, peak, wraps, c < wl);
+            add_pixel<kMark>(a, t, acc_base, at, s, peak, wraps, c < wl);
             s += d;
             d += dd;
         }
@@ -670,10 +742,6 @@ __device__ __noinline__ void deposit_coop(const TileArgs& a, TileState* tp, cons
     const TileState& t = *tp;
     const TileInfo ti = t.ti;
     const float peak = count_peak(t, r.e);
-    if (!(peak > 0.f)) {
-        if ((threadIdx.x & 31) == 0) deposit_direct(a, tp, rp);
-        return;
-    }
     int pxc, pyc, x0, x1, y0, y1;
     rec_box(r, ti, pxc, pyc, x0, x1, y0, y1);
     const float a00 = r.m00 * ti.sx, a10 = r.m10 * ti.sx;
@@ -688,7 +756,7 @@ __device__ __noinline__ void deposit_coop(const TileArgs& a, TileState* tp, cons
         int kx0 = x0 - pxc, kx1 = x1 - pxc;
         if (!support_cols(sup, dy, r.dx0, ti.isx, kx0, kx1)) continue;
         const float kf = float(kx0);
-        fwd_row<false>(
+        fwd_row<kMark>(
             a, t, acc_base, kx1 - kx0 + 1,
             acc_base + 4u * uint32_t((pyc + ky - ti.oy) * a.cfg.sw + (pxc + kx0 - ti.ox)),
             fmaf(kf, a00, fmaf(float(ky), m01sy, c00)), fmaf(kf, a10, fmaf(float(ky), m11sy, c10)),
@@ -825,6 +893,9 @@ __device__ __noinline__ void tail_forward(const TileArgs& a) {
 // groups; columns of a group outside the range add zero. All-zero groups are skipped.
 __device__ __forceinline__ void flush_rows(uint32_t* acc, int sw, const TileState& t, float* out) {
     const float unit = t.unit;
+    const auto value = [&](uint32_t v) {
+        return unit > 0.f ? float(v) * unit : __uint_as_float(v);
+    };
     const int x0 = t.x0, x1 = t.x1, y1 = t.y1;
     const int ox = t.ti.ox, oy = t.ti.oy, W = t.ti.W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -850,7 +921,7 @@ __device__ __forceinline__ void flush_rows(uint32_t* acc, int sw, const TileStat
                     const int c = gx + j;
                     v[j] = 0.f;
                     if (c >= x0 && c <= x1) {
-                        v[j] = float(arow[c]) * unit;
+                        v[j] = value(arow[c]);
                         arow[c] = 0u;
                     }
                 }
@@ -866,7 +937,7 @@ __device__ __forceinline__ void flush_rows(uint32_t* acc, int sw, const TileStat
             for (int gx = x0 + lane; gx <= x1; gx += 32) {
                 const uint32_t v = arow[gx];
                 if (v != 0u) {
-                    atomicAdd(grow + gx, float(v) * unit);
+                    atomicAdd(grow + gx, value(v));
                     arow[gx] = 0u;
                 }
             }
@@ -895,7 +966,7 @@ __device__ __noinline__ void redo_segment(const TileArgs& a, uint32_t* acc, Tile
     for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
         const float peak = count_peak(*t, a.srecs[i].e);
         if (!(rec_flags(a.srecs[i].packed) & kFlagFwdSkip) && peak > 0.f)
-            deposit_generic<true>(a, t, a.srecs + i, peak, acc_base);
+            deposit_slow<kCarry>(a, t, a.srecs + i, peak, acc_base);
     }
     __syncthreads();
 }
@@ -929,15 +1000,17 @@ __device__ __forceinline__ void forward_chunks(const TileArgs& a, uint32_t* acc,
         // every pass but the first covers at least one photon, so chunk + 1 passes suffice
         for (uint32_t pass = 0; pass <= chunk; ++pass) {
             const Segment sg = ts[cur].sg;
-            const uint32_t begin = max(sg.begin, p0), end = min(sg.end, p1);
-            const bool more = sg.end < p1;
+            const uint32_t stop = ts[cur].stop;
+            const bool more = stop < p1;
             walk_segment(
-                a, ts + cur, begin, end, [&](uint32_t i, bool valid) { walk(ts[cur], i, valid); },
+                a, ts + cur, sg.begin, stop,
+                [&](uint32_t i, bool valid) { walk(ts[cur], i, valid); },
                 [&] { if (!more && warp == 0) prepare(ts + pre, chunks + (par ^ 1)); });
             __syncthreads();
-            if (ts[cur].wrapped) redo_segment(a, acc, ts + cur, begin, end);
+            if (ts[cur].wrapped) redo_segment(a, acc, ts + cur, sg.begin, stop);
             if (more && threadIdx.x >= blockDim.x - 32)
-                start_segment(a, next_segment(a, sg), p1, ts + alt);
+                start_segment(a, stop < sg.end ? Segment{sg.tile, stop, sg.end} : next_segment(a, sg),
+                              p1, ts + alt);
             flush_rows(acc, sw, ts[cur], a.out);
             __syncthreads();
             if (!more) break;
@@ -961,13 +1034,13 @@ __global__ __launch_bounds__(NT, MINB) void fwd_tiles_kernel(const __grid_consta
         bool coop = false;
         if (valid) {
             const Rec r = load_rec(a.srecs + i);
-            coop = use_coop(r, a.cfg.coop_r);
             const float peak = count_peak(t, r.e);
+            coop = peak > 0.f && use_coop(r, a.cfg.coop_r);
             if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
                 if (!(peak > 0.f))
-                    deposit_direct(a, &t, a.srecs + i);
-                else if (!(a.cfg.band && deposit_band(r, t.ti, a.cfg.sw, peak, acc_base, &t.wrapped)))
-                    deposit_generic<false>(a, &t, a.srecs + i, peak, acc_base);
+                    deposit_uncounted(a, &t, a.srecs + i, r.e, acc_base);
+                else if (!(a.cfg.band && deposit_band<kMark>(a, t, r, peak, acc_base)))
+                    deposit_generic<kMark>(a, &t, a.srecs + i, peak, acc_base);
             }
         }
         if (a.cfg.coop_r > 0) {
@@ -1403,13 +1476,13 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
         bool generic = false, coop = false;
         if (valid) {
             const Rec r = load_rec(a.srecs + i);
-            coop = use_coop(r, a.cfg.coop_r);
+            peak = count_peak(t, r.e);
+            coop = peak > 0.f && use_coop(r, a.cfg.coop_r);
             if (!coop && !(rec_flags(r.packed) & kFlagFwdSkip)) {
                 int pxc, pyc, x0, x1, y0, y1;
                 rec_box(r, t.ti, pxc, pyc, x0, x1, y0, y1);
-                peak = count_peak(t, r.e);
                 if (!(peak > 0.f)) {
-                    deposit_direct(a, &t, a.srecs + i);
+                    deposit_uncounted(a, &t, a.srecs + i, r.e, acc_base);
                 } else {
                     generic = !prep_rows(r, t.ti, a.cfg.sw, pxc, pyc, x0, x1, y0, y1, g);
                     rows = generic ? 0 : g.rows;
@@ -1418,7 +1491,7 @@ __global__ __launch_bounds__(NT, MINB) void fwd_rows_kernel(const __grid_constan
         }
         __syncwarp();
         deposit_rows(a, t, g, rows, peak, acc_base);
-        if (generic) deposit_generic<false>(a, &t, a.srecs + i, peak, acc_base);
+        if (generic) deposit_generic<kMark>(a, &t, a.srecs + i, peak, acc_base);
         __syncwarp();
         for (uint32_t cm = __ballot_sync(0xFFFFFFFFu, coop); cm; cm &= cm - 1)
             deposit_coop(a, &t, a.srecs + __shfl_sync(0xFFFFFFFFu, i, __ffs(cm) - 1), acc_base);
