@@ -304,6 +304,7 @@ __device__ __forceinline__ int band_start(const Band& b, int ky) {
 // (the nearest integer to hw + 1/2, from the low mantissa bits of its sum with 1.5 * 2^23).
 constexpr float kRoundMagic = 12582912.f;
 constexpr uint32_t kRoundMagicBits = 0x4B400000u;
+constexpr float kMinHalf = 0.25f;  // half-width of the narrowest row walked
 
 __device__ __forceinline__ int band_pairs(float hw) {
     return __float_as_int((hw + 0.5f) + kRoundMagic) - int(kRoundMagicBits);
@@ -330,7 +331,7 @@ __device__ __forceinline__ int band_steps(float m00, float m01, float m10, float
     const float ey = A * hw * rcp_fast(fabsf(det));
     if (!(A > 0.f && A < 1e30f && hw <= float(rx) + 1.f && ey < 1e6f)) return (2 * rx + 1) * (ry + 1);
     const int rows = min(__float2int_rd(ey - dyp), ry) - max(__float2int_ru(-ey - dyp), -ry) + 1;
-    return min(band_pairs(hw), rx + 1) * max(rows, 1);
+    return min(band_pairs(fmaxf(hw, kMinHalf)), rx + 1) * max(rows, 1);
 }
 
 // The rows a photon's band walk visits inside its clipped box [kxb0, kxb1] x [kyb0, kyb1]

@@ -353,7 +353,8 @@ __device__ __noinline__ void deposit_direct(const TileArgs& a, const TileState* 
 // width the row is the whole box row, so no pixel needs an in-box test. When w is odd, the second
 // pixel of each row's last pair lies just outside the box and is masked: the remaining-pair count
 // is tail there. (A pixel that rounding puts just outside the window is at the support's edge to
-// within some 1e-6 of a pixel: it adds (1 - s)^2 ~ 1e-12 of the peak.)
+// within some 1e-6 of a pixel: it adds (1 - s)^2 ~ 1e-12 of the peak. Supports narrower than
+// 2 kMinHalf, whose centre that could be, are walked that wide: still one pair.)
 //
 // With rho = ky + dy0 / sy the photon's row offset in pixels, the support of a row is centred on
 // the column xc = beta rho - dx0 / sx, and with e = kx - xc
@@ -403,13 +404,14 @@ __device__ __forceinline__ bool pair_walk(const Rec& r, const TileInfo& ti, int 
     const int pxc = ti.ox + lx, pyc = ti.oy + ly;
     const int kxb0 = -min(rx, pxc), kxb1 = min(rx, ti.W - 1 - pxc);
     const int boxw = kxb1 - kxb0 + 1;
-    const int w = min(2 * band_pairs(hw), boxw);
+    const float wide = fmaxf(hw, kMinHalf);
+    const int w = min(2 * band_pairs(wide), boxw);
     const int ky0 = max(__float2int_ru(-ey - p.dyp), -min(ry, pyc));
     p.rows = min(__float2int_rd(ey - p.dyp), min(ry, ti.H - 1 - pyc)) - ky0 + 1;
     p.npairs = (w + 1) >> 1;
     p.tail = w & 1;
     p.ky0 = float(ky0);
-    p.hw5 = hw - 0.5f;
+    p.hw5 = wide - 0.5f;
     p.lo = float(kxb0);
     p.hi = float(kxb1 - w + 1);
     p.row = 4u * (uint32_t((ly + ky0) * sw + lx) - kRoundMagicBits);
