@@ -78,8 +78,10 @@ class _SplatPhotons(torch.autograd.Function):
             gE, gX, gM = plan.backward(grad.contiguous())
             E, M, _, _ = splat_inputs(Du, Dv, normal, flux, channel)
             wanted = [t for t, w in zip((Du, Dv, normal, flux), ctx.needs_input_grad) if w]
-            got = iter(torch.autograd.grad((E, M), wanted, (gE, gM), create_graph=True,
-                                           allow_unused=True) if wanted else ())
+            # (E does not depend on the normal, nor M on the flux)
+            outs = [(o, g) for o, g in ((E, gE), (M, gM)) if o.requires_grad]
+            got = iter(torch.autograd.grad([o for o, _ in outs], wanted, [g for _, g in outs],
+                                           create_graph=True, allow_unused=True) if wanted else ())
             grads = [next(got) if w else None for w in ctx.needs_input_grad[:4]]
             return (*grads, gX, None, None, None)
         plan.backward(grad.contiguous(), records=True)
