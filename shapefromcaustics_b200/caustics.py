@@ -76,8 +76,10 @@ class _SplatPhotons(torch.autograd.Function):
         plan = SplatPlan.planned((Ep, xy, Mp, cp, radius), ctx.shape, ctx.mpr, ctx.cfg, ws)
         if torch.is_grad_enabled():  # create_graph: the splat inputs' own torch operations
             gE, gX, gM = plan.backward(grad.contiguous())
-            E, M, _, _ = splat_inputs(Du, Dv, normal, flux, channel)
-            wanted = [t for t, w in zip((Du, Dv, normal, flux), ctx.needs_input_grad) if w]
+            # (views: the inputs' own hooks are run by the engine that asked for these gradients)
+            real = [t.view_as(t) for t in (Du, Dv, normal, flux)]
+            E, M, _, _ = splat_inputs(*real, channel)
+            wanted = [t for t, w in zip(real, ctx.needs_input_grad) if w]
             # (E does not depend on the normal, nor M on the flux)
             outs = [(o, g) for o, g in ((E, gE), (M, gM)) if o.requires_grad]
             got = iter(torch.autograd.grad([o for o, _ in outs], wanted, [g for _, g in outs],
