@@ -19,8 +19,8 @@ __all__ = ["DEFAULT", "CANDIDATES", "signature", "pick", "tune_batch", "cached"]
 
 # the library default first; then tile, class bits, walk, CTAs per SM and the cooperative
 # splat in all combinations, and the default with smaller and larger work chunks (sorted
-# photons a CTA takes at a time). min_blocks 0 is the library's choice (3 CTAs an SM in
-# both directions); 4 sets both.
+# photons a CTA takes at a time; 2048 is the default, which the library raises to 8192 for large
+# calls). min_blocks 0 is the library's choice (3 CTAs an SM in both directions); 4 sets both.
 DEFAULT = dict(tile=64, chunk=2048, class_bits=5, walk=3, min_blocks=0, coop_radius=-1)
 CANDIDATES = [dict(tile=t, chunk=2048, class_bits=b, walk=w, min_blocks=m, coop_radius=k)
               for t, b, w, m, k in itertools.product((64, 32), (5, 3), (3, 1), (0, 4), (-1, 8))]

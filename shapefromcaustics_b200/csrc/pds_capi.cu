@@ -43,7 +43,7 @@ struct Resolved {
 
 int resolve_cfg(const pds_config* in, pds_config& out) {
     out.tile = (in && in->tile) ? in->tile : 64;
-    out.chunk = (in && in->chunk) ? in->chunk : 2048;
+    out.chunk = (in && in->chunk) ? in->chunk : pds::kDefaultChunk;
     out.class_bits = (in && in->class_bits) ? in->class_bits : 5;
     if (out.class_bits == -1) out.class_bits = 0;
     out.apron_max = (in && in->apron_max) ? in->apron_max : 32;
@@ -71,21 +71,6 @@ int resolve_cfg(const pds_config* in, pds_config& out) {
     return PDS_OK;
 }
 
-// Photons per tile-kernel work chunk: the configured chunk (2048 by default), lowered for small
-// photon counts so that every resident CTA of the tile kernels (3 per SM) gets about four
-// chunks; at least 256 photons (one CTA-wide batch). Where none is configured it grows with the
-// photon count, up to 8192, while 48 chunks an SM are left: a chunk ends with its tile's pixels
-// added to the image or the next tile's staged, 6% of the forward at 2048 photons.
-int32_t effective_chunk(const pds_config* in, int32_t chunk, int64_t n) {
-    const int64_t sms = pds::num_sms();
-    const auto share = [&](int64_t per_sm) {
-        const int64_t target = (n + sms * per_sm - 1) / (sms * per_sm);
-        return (target + 255) / 256 * 256;
-    };
-    if (!(in && in->chunk)) chunk = int32_t(std::clamp<int64_t>(share(48), chunk, 8192));
-    return int32_t(std::clamp<int64_t>(share(12), 256, chunk));
-}
-
 int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resolved& r) {
     pds_config c;
     int rc = resolve_cfg(in, c);
@@ -96,7 +81,7 @@ int resolve(const pds_config* in, int32_t mpr, int64_t n_tiles, int64_t n, Resol
     if (inv >= (uint64_t(1) << 32))
         return fail(PDS_ERR_UNSUPPORTED, "sort key space exceeds 32 bits; lower class_bits");
     r.cfg.tile = c.tile;
-    r.cfg.chunk = effective_chunk(in, c.chunk, n);
+    r.cfg.chunk = pds::effective_chunk(c.chunk, n, pds::num_sms());
     r.cfg.class_bits = c.class_bits;
     r.cfg.apron = mpr < 0 ? 0 : (mpr < c.apron_max ? mpr : c.apron_max);
     // odd pitch: the rows of one column of the accumulator fall in different banks
