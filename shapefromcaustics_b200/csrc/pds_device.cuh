@@ -296,10 +296,6 @@ __device__ __forceinline__ Band make_band(float m00, float m01, float m10, float
     return b;
 }
 
-__device__ __forceinline__ int band_start(const Band& b, int ky) {
-    return __float2int_rd(fmaf(float(ky), b.beta, b.alpha - b.hw));
-}
-
 // The band walks take rows two pixels at a time: pairs of a row of half-width hw, floor(hw + 1)
 // (the nearest integer to hw + 1/2, from the low mantissa bits of its sum with 1.5 * 2^23).
 constexpr float kRoundMagic = 12582912.f;
@@ -353,10 +349,6 @@ __device__ __forceinline__ RowWalk row_walk(const Band& b, int kxb0, int kxb1, i
     r.kxb0 = kxb0;
     r.kxlast = kxb1 - r.w + 1;
     return r;
-}
-
-__device__ __forceinline__ int row_start(const Band& b, const RowWalk& r, int ky) {
-    return min(max(band_start(b, ky), r.kxb0), r.kxlast);
 }
 
 // Footprint class of the row walk: 3 bits for the row count and 3 for the row width, levels
