@@ -156,16 +156,16 @@ __device__ __forceinline__ void set_tile(const TileArgs& a, const Segment& sg, T
 // (set_scale): with c the photons' mean number of covers of a pixel if they were spread over the
 // tile, 2^32 counts hold at least 64 c typical peaks (or all of the segment's photons on one
 // pixel). Where the peak of the sample's dimmest photon would then be below 2^kMinCountBits counts,
-// a large segment is summed in pieces (kPiece), which need less room, and what is still missing is
-// taken from the room.
+// half the room is given up; then a large segment is summed in pieces (kPiece), which need less; and
+// what is still missing is taken from the room.
 //
 // An add is rounded to half a count (0.29 in the mean square): at most 2^-20 of its photon's peak,
 // mostly 2^-22 and less, as far as a photon evaluated in float32 is off anyway. Measured against 64
 // bits, and with sums in float instead:
 // - single photons of 0.5 to 4 px: 6.3e-8 of their peak in the mean square, 6.9e-8;
-// - a pixel of 2^24 photons on caustic curves, in chunks of 8192: 3.6e-9 of the peaks that cover
-//   it, 9.1e-9; the whole image 4.9e-8, 3.0e-7;
-// - of 2^22 uniform photons: 4.9e-9, 4.5e-9; the whole image 1.06e-7, 1.01e-7 (mostly the float
+// - a pixel of 2^24 photons on caustic curves, in chunks of 8192: 3.7e-9 of the peaks that cover
+//   it, 9.1e-9; the whole image 5.5e-8, 3.0e-7;
+// - of 2^22 uniform photons: 4.9e-9, 4.5e-9; the whole image 1.07e-7, 1.01e-7 (mostly the float
 //   sums of the segments in the image).
 //
 // - A pixel whose count wraps (photons gathered on few pixels) is seen by the lane that causes
@@ -186,8 +186,9 @@ constexpr int kMaxCountBits = 25;  // counts of a typical peak at most, leaving 
 constexpr int kMinCountBits = 21, kDimBits = 19;
 constexpr float kCountLimit = 2147483648.f;
 // Photons of a piece at least (each is added to the image by itself): 2^26 photons on caustic curves
-// in chunks of 8192 4.33 ms, 4.70 in pieces from 512 on, 4.58 to 4.77 from 2048 on (where some wrap),
-// 7.00 in whole segments; 4.31 with the typical peak at 18 bits.
+// in chunks of 8192 4.29 ms (4.36 with no room given up first, and then 4.70 in pieces from 512 on,
+// 4.58 to 4.77 from 2048 on, where some wrap); 7.00 in whole segments; 4.22 with the typical peak
+// at 18 bits.
 constexpr uint32_t kPiece = 1024;
 
 // Sets t's stop, and its scale, from at most 32 photons spread evenly over the sorted positions
@@ -220,7 +221,7 @@ __device__ __forceinline__ void set_scale(const TileArgs& a, uint32_t begin, uin
         const int mean = __float2int_rd(float(sum) / float(max(count, 1)));
         const int lift = kMinCountBits - least + mean;  // bits of a typical peak that this takes
         int halvings = 0;
-        while (lift > 30 - room + halvings && (n >> (halvings + 1)) >= kPiece) ++halvings;
+        while (lift > 31 - room + halvings && (n >> (halvings + 1)) >= kPiece) ++halvings;
         t->stop = begin + ((n + (1u << halvings) - 1u) >> halvings);
         const int k = max(min(kMaxCountBits, 30 - room + halvings), lift) - mean;
         const bool fits = count > 0 && most + k <= 30 && k <= 126;
