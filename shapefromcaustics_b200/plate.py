@@ -258,7 +258,9 @@ def _refract_point_backward_planned(height, light, params, direction, dtheta, dp
 class PointPlateSplat(torch.autograd.Function):
     """Caustic image of the plate lit by a point light (photons traced onto the height-field
     surface); differentiable in the height field. ``photons`` = ``(direction, dtheta, dphi,
-    flux)`` as from ``point_light_source``. ``keep_plan`` as in ``PlateSplat``."""
+    flux)`` as from ``point_light_source``. ``keep_plan`` as in ``PlateSplat``: 125 bytes a photon
+    are held for the backward; with ``keep_plan=False``, for many images whose backward comes later,
+    none are (the photons are refracted and planned again there)."""
 
     @staticmethod
     def forward(ctx, height, direction, dtheta, dphi, flux, light, params, output_size,
